@@ -278,6 +278,31 @@ MQV_HD uint64_t accept_cut_direct(int pref, double dE, double beta)
     return c < lo ? lo : c;
 }
 
+// ---- programmatic dependent launch -------------------------------------------
+// A kernel launched with launch_pdl may start while the kernel before it on
+// the stream still runs: what it does before grid_dep_wait must not touch
+// anything that kernel (or an earlier one) writes or reads.  Every kernel
+// launched this way waits, so completion stays in stream order.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+#ifdef __CUDACC__
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 // ---- Blackwell async copies (bulk copy engine) and mbarriers -----------------
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)

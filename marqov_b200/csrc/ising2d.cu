@@ -158,17 +158,26 @@ struct TieEntry {
     int32_t y, x;    // lattice coordinates of the word's first site
 };
 
-// Update the active-colour sites of one 32-site word: returns the word with
-// the decided flips applied; `tie` and `inA` receive the undecided sites.
-__device__ __forceinline__ uint32_t update_word(uint32_t A, uint32_t U, uint32_t D, uint32_t Lb, uint32_t Rb, int x,
-                                                int y, uint32_t tg_acc, const Ising2DArgs& a, const Thr& th,
-                                                uint32_t& tie, uint32_t& inA)
+// The eight random planes of the word whose first site is (x, y): the two
+// ACCEPT blocks of its 32-site group.
+struct Planes {
+    uint32_t b[8];
+};
+__device__ __forceinline__ Planes word_planes(int x, int y, uint32_t tg_acc, const Ising2DArgs& a)
 {
-    // the word's eight random planes: two Philox blocks of its 32-site group
     const uint32_t g = accept_group((uint32_t)y * (uint32_t)a.L + (uint32_t)x);
     const uint4 q0 = philox_rk(g, a.sweep, 0u, tg_acc, a);
     const uint4 q1 = philox_rk(g, a.sweep, 1u, tg_acc, a);
-    const uint32_t pl[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    return Planes{{q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w}};
+}
+
+// Update the active-colour sites of one 32-site word on its planes: returns
+// the word with the decided flips applied; `tie` and `inA` receive the
+// undecided sites.
+__device__ __forceinline__ uint32_t decide_word(uint32_t A, uint32_t U, uint32_t D, uint32_t Lb, uint32_t Rb,
+                                                const Planes& rnd, const Thr& th, uint32_t& tie, uint32_t& inA)
+{
+    const uint32_t* pl = rnd.b;
     // minus-neighbour count M = m0 + 2 m1 + 4 m2 (carry-save adder; M <= 4)
     const uint32_t s3 = U ^ D ^ Lb, c3 = (U & D) | (Lb & (U | D));  // full adder of three
     const uint32_t m0 = s3 ^ Rb, c4 = s3 & Rb;                        // plus the fourth
@@ -201,6 +210,12 @@ __device__ __forceinline__ uint32_t update_word(uint32_t A, uint32_t U, uint32_t
     tie = eq & test & ~zt;
     inA = tie & maskA;
     return A ^ (~test | borrow);
+}
+__device__ __forceinline__ uint32_t update_word(uint32_t A, uint32_t U, uint32_t D, uint32_t Lb, uint32_t Rb, int x,
+                                                int y, uint32_t tg_acc, const Ising2DArgs& a, const Thr& th,
+                                                uint32_t& tie, uint32_t& inA)
+{
+    return decide_word(A, U, D, Lb, Rb, word_planes(x, y, tg_acc, a), th, tie, inA);
 }
 
 // Bond sum s * sum(nbrs) = sum (1 - 2a)(4 - 2M) over the sites of a word
@@ -811,6 +826,138 @@ __global__ void __launch_bounds__(NT, MINB) ising2d_band(const __grid_constant__
     }
 }
 
+// ---- colour kernel: one launch per colour, in place ------------------------------
+//
+// For lattices that fit the L2 (L <= 8192): thread = T consecutive rows of one
+// word column.  A word of the colour needs its own 32 bytes and, from the rows
+// above, here and below, the other colour's words of the same column plus one
+// edge byte of the neighbouring column; a strip of T rows shares them, so a
+// word update packs 2 + 2 / T words.  Sites of one colour are independent and
+// only the active words are written, so the update is in place, without halo
+// re-computation, barriers or a tile queue: what bounds it is the latency of a
+// few dependent loads at small L and the instruction issue rate at large L
+// (per sweep, before with tiles and now: L = 1024 37.6 -> 7 us, L = 4096 50.8
+// -> 12.3 us; starting the draws before the previous launch has drained took
+// them from 8.5 and 16.8 us).
+// Top-byte ties are listed per warp and resolved after the strip, side by side
+// over the lanes; an accepted one is stored as a byte.  MEAS (launched for
+// colour 1): every bond joins a colour-1 site to a colour-0 site, so the
+// colour-1 words' bond sums after the update are the lattice's.
+template <int T>
+struct ColourGeom {
+    static constexpr int NT = 256;
+    static constexpr int TIECAP = 32 * T;  // every word of the warp's strips may hold ties
+};
+
+template <int T, bool MEAS>
+__global__ void __launch_bounds__(ColourGeom<T>::NT) ising2d_colour(const __grid_constant__ Ising2DArgs a, int colour)
+{
+    using G = ColourGeom<T>;
+    __shared__ uint4 ties[G::NT / 32][G::TIECAP];  // (row ncol + column, tie sites, class A, word)
+    __shared__ int red[2][G::NT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int L = a.L, Lh = L >> 1, ncol = L >> 6;
+    const uint32_t nstrip = (uint32_t)ncol * (uint32_t)(L / T);
+    const uint32_t id = blockIdx.x * G::NT + threadIdx.x;
+    const bool live = id < nstrip;
+    const uint32_t strip = live ? id : 0u, sy = strip / (uint32_t)ncol;
+    const int w = (int)(strip - sy * (uint32_t)ncol), y0 = (int)sy * T;
+    const uint32_t tg_acc = tag(kAccept, a.replica);
+    const Thr th = make_thr(a);
+    int8_t* s = a.dst;
+    // the draws need no lattice data: they run while the launch before this
+    // one drains (programmatic dependent launch), the state is touched after
+    Planes rnd[T];
+#pragma unroll
+    for (int k = 0; k < T; ++k) rnd[k] = word_planes(64 * w + ((y0 + k + colour) & 1), y0 + k, tg_acc, a);
+    grid_dep_launch();
+    grid_dep_wait();
+    // the other colour's words of rows y0 - 1 .. y0 + T (half 1 - p of a row
+    // whose active half is p), the active words, the edge sites
+    uint32_t g[T + 2], act[T], edge[T];
+#pragma unroll
+    for (int k = 0; k < T + 2; ++k) {
+        const int y = wrapi(y0 - 1 + k, L), p = (y0 - 1 + k + colour) & 1;
+        const int8_t* row = s + (size_t)y * L;
+        const uint4* q = reinterpret_cast<const uint4*>(row + (p ? 0 : Lh) + 32 * w);
+        g[k] = pack_word(q[0], q[1]);
+        if (k >= 1 && k <= T) {
+            const uint4* qa = reinterpret_cast<const uint4*>(row + (p ? Lh : 0) + 32 * w);
+            act[k - 1] = pack_word(qa[0], qa[1]);
+            // p = 1: site 0 of the even word to the right; p = 0: site 31 of the odd word to the left
+            const int8_t e = p ? row[32 * (w + 1 == ncol ? 0 : w + 1)] : row[Lh + 32 * (w == 0 ? ncol - 1 : w - 1) + 31];
+            edge[k - 1] = (uint32_t)e >> 31;
+        }
+    }
+    int ntie = 0, esum = 0, msum = 0;
+#pragma unroll
+    for (int k = 0; k < T; ++k) {
+        const int y = y0 + k, p = (y + colour) & 1;
+        const uint32_t G1 = g[k + 1];
+        const uint32_t Lb = p ? G1 : (G1 << 1) | edge[k];
+        const uint32_t Rb = p ? (G1 >> 1) | (edge[k] << 31) : G1;
+        uint32_t tie, inA;
+        const uint32_t An = decide_word(act[k], g[k], g[k + 2], Lb, Rb, rnd[k], th, tie, inA);
+        if (!live) tie = 0u;
+        const uint32_t has = __ballot_sync(0xffffffffu, tie != 0u);
+        if (tie)
+            ties[warp][ntie + __popc(has & ((1u << lane) - 1u))] =
+                make_uint4((uint32_t)y * (uint32_t)ncol + (uint32_t)w, tie, inA, An);
+        ntie += __popc(has);
+        if (live) {
+            uint4 lo, hi;
+            unpack_word(An, lo, hi);
+            uint4* q = reinterpret_cast<uint4*>(s + (size_t)y * L + (p ? Lh : 0) + 32 * w);
+            q[0] = lo;
+            q[1] = hi;
+            if (MEAS) {
+                esum += word_bonds(An, g[k], g[k + 2], Lb, Rb);
+                msum += 64 - 2 * __popc(An) - 2 * __popc(G1);
+            }
+        }
+    }
+    __syncwarp();
+    for (int e = lane; e < ntie; e += 32) {
+        const uint4 te = ties[warp][e];
+        const uint32_t y = te.x / (uint32_t)ncol, c = te.x - y * (uint32_t)ncol, p = (y + (uint32_t)colour) & 1u;
+        uint32_t m = te.y;
+        while (m) {
+            const int b = __ffs(m) - 1;
+            m &= m - 1;
+            const bool inA = (te.z >> b) & 1u;
+            const uint64_t u53 = ((uint64_t)(inA ? a.tA8 : a.tB8) << 45) |
+                                 (fine56_rk(y * (uint32_t)L + 64u * c + p + 2u * (uint32_t)b, a) >> 11);
+            if (u53 < (inA ? a.tA : a.tB)) {
+                const bool minus = (te.w >> b) & 1u;
+                s[(size_t)y * L + (p ? Lh : 0) + 32 * c + 4 * (b & 7) + (b >> 3)] = minus ? 1 : -1;
+                if (MEAS) {
+                    // the tested classes have s * sum(nbrs) = +-2 (A) or +-4 (B) before the flip
+                    esum += (inA ? 4 : 8) * (a.mode == 0 ? -1 : 1);
+                    msum += minus ? 2 : -2;
+                }
+            }
+        }
+    }
+    if (MEAS) {
+        esum = __reduce_add_sync(0xffffffffu, esum);
+        msum = __reduce_add_sync(0xffffffffu, msum);
+        if (lane == 0) {
+            red[0][warp] = esum;
+            red[1][warp] = msum;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            long long e = 0, m = 0;
+            for (int k = 0; k < G::NT / 32; ++k) {
+                e += red[0][k];
+                m += red[1][k];
+            }
+            atomicAdd(reinterpret_cast<unsigned long long*>(a.acc + kAccEne), (unsigned long long)(2 * e));
+            atomicAdd(reinterpret_cast<unsigned long long*>(a.acc + kAccMag), (unsigned long long)m);
+        }
+    }
+}
+
 // ---- layout conversion: row-major <-> split rows -----------------------------
 // One thread moves a group of 64 consecutive sites of a row (x = 64w .. 64w+63):
 // its even sites become word w of the even half, its odd sites word w of the
@@ -973,9 +1120,18 @@ static cudaError_t launch_band(const Ising2DArgs& a, int nsm, cudaStream_t strea
     return cudaGetLastError();
 }
 
+// Both colours of the colour kernel, in place on a.dst.
+template <int T, bool MEAS>
+static cudaError_t launch_colour(const Ising2DArgs& a, int, cudaStream_t stream)
+{
+    const unsigned nt = ColourGeom<T>::NT, grid = ((unsigned)(a.L >> 6) * (unsigned)(a.L / T) + nt - 1) / nt;
+    const cudaError_t e = launch_pdl(ising2d_colour<T, false>, grid, nt, stream, a, 0);
+    return e != cudaSuccess ? e : launch_pdl(ising2d_colour<T, MEAS>, grid, nt, stream, a, 1);
+}
+
 // Candidate kernels: tiles (tx x ty sites, nwarp independent warps per CTA)
 // or bands (band = NT threads spanning a lattice of side 64 NT, ties resolved
-// every S steps).  Every candidate computes the same result; the autotuner
+// every S steps) or the colour kernel (T rows per thread).  Every candidate computes the same result; the autotuner
 // keeps the fastest for a lattice size.
 struct SweepConfig {
     int tx, ty, nwarp;  // tile shape (band: tx = L, ty = S, nwarp = NT / 32)
@@ -984,6 +1140,7 @@ struct SweepConfig {
     SweepLauncher plain, meas;
     int w;              // band: word columns per thread
     int rs = 0;         // band: rows staged in registers, at most rs CTAs per SM (0: bulk-copy ring)
+    int strip = 0;      // colour kernel: rows per thread (updates the state in place)
 };
 
 #define MQV_CFG(TX, TY, NW) \
@@ -1000,7 +1157,11 @@ struct SweepConfig {
     SweepConfig{64 * NT * W, S, NT / 32, true, 0, launch_band<NT, S, 2, false, W, true, MINB>,             \
                 launch_band<NT, S, 2, true, W, true, MINB>, W, MINB}
 
+#define MQV_COLOUR(T) \
+    SweepConfig{64, T, 1, false, 0, launch_colour<T, false>, launch_colour<T, true>, 1, 0, T}
+
 static const SweepConfig kConfigs[] = {
+    MQV_COLOUR(1), MQV_COLOUR(2), MQV_COLOUR(4),
     MQV_CFG(512, 32, 4), MQV_CFG(256, 32, 4), MQV_CFG(512, 32, 2), MQV_CFG(256, 32, 8),
     MQV_CFG(1024, 32, 2), MQV_CFG(128, 32, 4), MQV_CFG(64, 32, 4),
     MQV_BAND(256, 4, 2), MQV_BAND(256, 2, 2), MQV_BAND(256, 4, 3), MQV_BAND(256, 4, 4),
@@ -1014,16 +1175,23 @@ static const SweepConfig kConfigs[] = {
 };
 constexpr int kNumConfigs = (int)(sizeof(kConfigs) / sizeof(kConfigs[0]));
 
+// Colour kernels up to here: at L = 8192 the 67 MB state still sits in the L2
+// and two passes over it cost what the band kernel's single pass does (38.8
+// against 41.4 us); at L = 16384 each pass goes to HBM (2 x 402 MB against 537).
+// Below L = 2048 one row per thread is taken without timing (L = 1024: 7 us a
+// sweep against 9 with four rows; tiles: 37.6 us).
+constexpr int kColourMaxLen = 8192;
 static bool config_fits(const SweepConfig& c, int L)
 {
     if (c.band) return L == c.tx;
+    if (c.strip) return L <= kColourMaxLen;
     return L % c.tx == 0 && L % c.ty == 0;
 }
 
 static void fill_args(Sim* s, const SweepConfig& c, long long* acc, Ising2DArgs& a)
 {
     a.src = (const int8_t*)s->state[s->cur];
-    a.dst = (int8_t*)s->state[s->cur ^ 1];
+    a.dst = (int8_t*)s->state[c.strip ? s->cur : s->cur ^ 1];
     a.L = s->len;
     a.ntx = c.band ? 1 : s->len / c.tx;
     a.ntiles = c.band ? 0 : a.ntx * (s->len / c.ty);
@@ -1066,7 +1234,8 @@ static void fill_args(Sim* s, const SweepConfig& c, long long* acc, Ising2DArgs&
 // lattices take the first fitting candidate.
 static void config_name(const SweepConfig& c, char* buf, int len)
 {
-    if (c.band && c.rs) snprintf(buf, len, "ising2d_band_rs<%d,%d,%d,%d>", c.nwarp * 32, c.ty, c.w, c.rs);
+    if (c.strip) snprintf(buf, len, "ising2d_colour<%d>", c.strip);
+    else if (c.band && c.rs) snprintf(buf, len, "ising2d_band_rs<%d,%d,%d,%d>", c.nwarp * 32, c.ty, c.w, c.rs);
     else if (c.band && c.w > 1) snprintf(buf, len, "ising2d_band<%d,%d,%d,%d>", c.nwarp * 32, c.ty, c.nsb, c.w);
     else if (c.band) snprintf(buf, len, "ising2d_band<%d,%d,%d>", c.nwarp * 32, c.ty, c.nsb);
     else snprintf(buf, len, "ising2d_sweep<%d,%d,%d>", c.tx, c.ty, c.nwarp);
@@ -1105,8 +1274,12 @@ static int pick_config(Sim* s)
     for (int round = 0; round < kRounds; ++round)
         for (int k = 0; k < kNumConfigs; ++k) {
             if (!config_fits(kConfigs[k], s->len)) continue;
+            // tiles are never the fastest where the colour kernels apply
+            // (L = 2048: 37 against 12 us, L = 4096: 51 against 12 us)
+            if (s->len <= kColourMaxLen && !kConfigs[k].band && !kConfigs[k].strip) continue;
             Ising2DArgs a{};
             fill_args(s, kConfigs[k], nullptr, a);
+            a.dst = (int8_t*)s->state[s->cur ^ 1];  // in-place kernels too: the state stays as it is
             cudaMemsetAsync(s->d_counter, 0, sizeof(int), s->stream);
             if (kConfigs[k].plain(a, s->num_sms, s->stream) != cudaSuccess) continue;  // warm-up
             cudaEventRecord(e0, s->stream);
@@ -1153,11 +1326,14 @@ cudaError_t launch_ising2d_sweep(Sim* s, long long* acc)
         a.wait_ns = s->inject_wait_ns;
         s->inject_row = -1;
     }
-    if (!c.band) {  // tiles are taken from a counter; bands are fixed per CTA
+    if (!c.band && !c.strip) {  // tiles are taken from a counter; bands are fixed per CTA
         const cudaError_t e = cudaMemsetAsync(s->d_counter, 0, sizeof(int), s->stream);
         if (e != cudaSuccess) return e;
     }
-    return acc ? c.meas(a, s->num_sms, s->stream) : c.plain(a, s->num_sms, s->stream);
+    const cudaError_t e = acc ? c.meas(a, s->num_sms, s->stream) : c.plain(a, s->num_sms, s->stream);
+    s->launches += c.strip ? 2 : 1;
+    if (!c.strip) s->cur ^= 1;
+    return e;
 }
 
 const char* ising2d_config_name(Sim* s, char* buf, int len)

@@ -203,9 +203,7 @@ cudaError_t launch_metropolis_int8(Sim* s, int slot)
     cudaError_t err = cudaSuccess;
     if (s->fused_ising2d) {
         long long* acc = slot >= 0 ? s->d_acc + (size_t)slot * kAccStride : nullptr;
-        err = launch_ising2d_sweep(s, acc);
-        s->launches++;
-        s->cur ^= 1;
+        err = launch_ising2d_sweep(s, acc);  // counts its launches, flips the state buffers unless in place
         s->sweep++;
         return err;
     }
