@@ -10,9 +10,9 @@
 //                    members on hypercubic lattices use the checkerboard,
 //                    CSR members their own colouring,
 //   batch_measure    CTAs (part, member) accumulate each member's observables,
-//   batch_tick       advances the EMCS counter.
+//   batch_tick       advances the EMCS counter by the EMCS of a graph.
 // Every per-step number (sweep and cluster serials, measurement slot) is
-// derived on the device from that counter, so the kernels of one EMCS form a
+// derived on the device from that counter and the EMCS's place in the graph, so the kernels of one EMCS form a
 // fixed sequence: it is captured once into a CUDA graph and replayed.  The
 // per-member arithmetic is that of the per-handle kernels, keyed by each
 // member's (seed, replica id, sweep, site), so a batched run equals running
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kBatchMetroThreads)
     batch_metro(const BatchRep* __restrict__ reps, const int64_t* __restrict__ prefix,
                 const int32_t* __restrict__ block_rep, const int32_t* __restrict__ cbegin,
                 const int32_t* __restrict__ ccount, int ncol, int64_t total, int colour,
-                const BatchCtr* __restrict__ ctr, int nmetro, int j)
+                const BatchCtr* __restrict__ ctr, uint32_t e_off, int nmetro, int j)
 {
     static_assert(kBatchMetroThreads == kAccSites, "one position per thread");
     __shared__ uint4 tab[kAccTab];
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kBatchMetroThreads)
     const BatchRep& R = reps[r];
     const int64_t t0 = g0 - prefix[r];
     const int64_t cnt = ccount[(size_t)r * ncol + colour];
-    const uint32_t sweep = R.sweep0 + ctr->e * (uint32_t)nmetro + (uint32_t)j;
+    const uint32_t sweep = R.sweep0 + (ctr->e + e_off) * (uint32_t)nmetro + (uint32_t)j;
     const int64_t t = t0 + threadIdx.x;
     const bool live = t < cnt;
     if (R.lat_kind == MQV_LATTICE_HYPERCUBIC) {
@@ -77,14 +77,13 @@ __global__ void __launch_bounds__(kBatchMetroThreads)
 
 template <bool F32>
 __global__ void __launch_bounds__(1024) batch_wolff(const BatchRep* __restrict__ reps,
-                                                    const BatchCtr* __restrict__ ctr, int ncluster, int c,
+                                                    const BatchCtr* __restrict__ ctr, ClusterStep step,
                                                     int32_t* __restrict__ csize, int nrep)
 {
     const BatchRep& R = reps[blockIdx.x];
     if (R.resident) return;  // its clusters are grown by batch_resident
-    const uint32_t e = ctr->e, slot = e - ctr->ebase;
-    const uint32_t serial = R.cluster0 + e * (uint32_t)ncluster + (uint32_t)c;
-    int32_t* out = csize + ((size_t)slot * ncluster + c) * nrep + blockIdx.x;
+    const uint32_t serial = cluster_serial(R, ctr, step);
+    int32_t* out = csize + cluster_slot(ctr, step, nrep, (int)blockIdx.x);
     const uint32_t tgs = tag(kWolffSeed, R.replica), tgb = tag(kWolffBond, R.replica);
     // frontier buffers: int8 ids, or float ids followed by their projections
     __shared__ __align__(16) unsigned char wbuf[kWolffSmem];
@@ -107,14 +106,14 @@ __global__ void __launch_bounds__(1024) batch_wolff(const BatchRep* __restrict__
 
 // One CTA per (member, part): member sizes set their number of parts.
 template <bool F32>
-__global__ void batch_measure(const BatchRep* __restrict__ reps, const BatchCtr* __restrict__ ctr,
+__global__ void batch_measure(const BatchRep* __restrict__ reps, const BatchCtr* __restrict__ ctr, uint32_t e_off,
                               long long* __restrict__ acc, int nrep, const int32_t* __restrict__ meas_prefix,
                               const int32_t* __restrict__ meas_rep)
 {
     const int r = meas_rep[blockIdx.x];
     const int part = (int)blockIdx.x - meas_prefix[r], nparts = meas_prefix[r + 1] - meas_prefix[r];
     const BatchRep& R = reps[r];
-    const uint32_t slot = ctr->e - ctr->ebase;
+    const uint32_t slot = ctr->e + e_off - ctr->ebase;
     long long* a = acc + ((size_t)slot * nrep + r) * kAccStride;
     if (F32) {
         if (R.lat_kind == MQV_LATTICE_HYPERCUBIC)
@@ -129,7 +128,7 @@ __global__ void batch_measure(const BatchRep* __restrict__ reps, const BatchCtr*
     }
 }
 
-__global__ void batch_tick(BatchCtr* ctr) { ctr->e += 1u; }
+__global__ void batch_tick(BatchCtr* ctr, uint32_t count) { ctr->e += count; }
 
 __global__ void batch_chunk_start(BatchCtr* ctr, uint32_t e)
 {
@@ -230,42 +229,97 @@ __global__ void batch_temper(BatchRep* __restrict__ reps, const BatchCtr* __rest
 
 // ---- launchers (stream-ordered; all capturable) ------------------------------------
 
+template <bool F32, int U, int LPU>
+static cudaError_t launch_tile_t(const BatchLaunch& b, cudaStream_t st, const ClusterStep& k)
+{
+    CclSeed* sd = (CclSeed*)b.ccl_seeds;
+    const unsigned g = (unsigned)b.tiles, nt = U * LPU;
+    cudaError_t e = launch_pdl(tile_label<F32, U, LPU>, g, nt, st, b.reps, b.tile_prefix, b.tile_rep, sd, b.ctr, k,
+                               b.csize, b.nrep);
+    if (e == cudaSuccess)
+        e = launch_pdl(tile_hook<F32, U, LPU>, g, nt, st, b.reps, b.tile_prefix, b.tile_rep, sd, b.ctr, k);
+    if (e == cudaSuccess)
+        e = launch_pdl(tile_flip<F32, U, LPU>, g, nt, st, b.reps, b.tile_prefix, b.tile_rep, sd, b.ctr, k, b.csize,
+                       b.nrep);
+    return e;
+}
+
+// Units per tile and lanes per unit by the units of all members, measured (us
+// per cluster with (64, 8) / (64, 4) / (128, 2)): 2 K units (2D L = 256) 28 /
+// 33 / 45, 16 K (32 x L = 128) 38 / 41 / 53, 49 K (24 x L = 256) 54 / 40 / 41,
+// 131 K (L = 2048) 122 / 89 / 89, 524 K (L = 4096) 435 / 284 / 248: more lanes
+// per unit shorten the serial steps while the chip is not full.
+constexpr int64_t kTileUnits8 = 24576, kTileUnits4 = 98304;
+int tile_units(int64_t total) { return total < kTileUnits4 ? 64 : 128; }
+
+cudaError_t launch_tile_cluster(const BatchLaunch& b, cudaStream_t st, const ClusterStep& k)
+{
+    if (b.tiles == 0) return cudaSuccess;
+    if (b.tile_units == 128) return b.f32 ? launch_tile_t<true, 128, 2>(b, st, k) : launch_tile_t<false, 128, 2>(b, st, k);
+    if ((int64_t)b.tiles * 64 >= kTileUnits8)
+        return b.f32 ? launch_tile_t<true, 64, 4>(b, st, k) : launch_tile_t<false, 64, 4>(b, st, k);
+    return b.f32 ? launch_tile_t<true, 64, 8>(b, st, k) : launch_tile_t<false, 64, 8>(b, st, k);
+}
+
+void tile_bind(BatchRep& r, const TileShape& t, int units, void* scratch)
+{
+    r.tl_nw = t.nw;
+    r.tl_ny = t.ny;
+    r.tl_nz = t.nz;
+    r.tl_tiles = t.n;
+    const size_t u = (size_t)t.n * units;
+    char* p = (char*)scratch;
+    r.tl_forest = (int*)p;
+    r.tl_lab = (unsigned short*)(p + u * 128);
+    r.tl_cand = (uint32_t*)(p + u * 192);
+    r.tl_xb = r.tl_cand + u;
+}
+
 template <bool F32>
-static void launch_emcs_t(const BatchLaunch& b, cudaStream_t st, int ncluster, int nmetro)
+static cudaError_t launch_emcs_t(const BatchLaunch& b, cudaStream_t st, int ncluster, int nmetro, uint32_t e_off)
 {
     for (int c = 0; c < ncluster; ++c) {
-        if (b.wolff_ccl) {
-            CclSeed* sd = (CclSeed*)b.ccl_seeds;
-            const unsigned gb = (unsigned)b.site_blocks;
-            if (b.site_blocks == 0) continue;  // every member is resident
-            ccl_seed<F32><<<(b.nrep + 127) / 128, 128, 0, st>>>(b.reps, b.ctr, ncluster, c, sd, b.csize, b.nrep);
-            ccl_local<F32><<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites,
-                                                              sd, b.ctr, ncluster, c);
-            ccl_hook<F32><<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites,
-                                                             sd, b.ctr, ncluster, c);
-            ccl_halve<<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites);
-            ccl_flip<F32><<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites,
-                                                             sd, b.ctr, ncluster, c, b.csize, b.nrep);
-        } else {
-            batch_wolff<F32><<<b.nrep, 1024, 0, st>>>(b.reps, b.ctr, ncluster, c, b.csize, b.nrep);
+        const ClusterStep k{e_off, 0u, ncluster, c};
+        if (!b.wolff_ccl) {
+            batch_wolff<F32><<<b.nrep, 1024, 0, st>>>(b.reps, b.ctr, k, b.csize, b.nrep);
+            continue;
         }
+        const cudaError_t e = launch_tile_cluster(b, st, k);
+        if (e != cudaSuccess) return e;
+        CclSeed* sd = (CclSeed*)b.ccl_seeds;
+        const unsigned gb = (unsigned)b.site_blocks;
+        if (b.site_blocks == 0) continue;  // every member is resident or tiled
+        ccl_seed<F32><<<(b.nrep + 127) / 128, 128, 0, st>>>(b.reps, b.ctr, k, sd, b.csize, b.nrep);
+        ccl_local<F32><<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites, sd,
+                                                          b.ctr, k);
+        ccl_hook<F32><<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites, sd,
+                                                         b.ctr, k);
+        ccl_halve<<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites);
+        ccl_flip<F32><<<gb, kBatchMetroThreads, 0, st>>>(b.reps, b.site_prefix, b.site_block_rep, b.total_sites, sd,
+                                                         b.ctr, k, b.csize, b.nrep);
     }
     for (int j = 0; j < nmetro; ++j)
         for (int colour = 0; colour < b.ncol; ++colour) {
             if (b.total[colour] == 0) continue;
             batch_metro<F32><<<b.blocks[colour], kBatchMetroThreads, 0, st>>>(
                 b.reps, b.prefix + (size_t)colour * (b.nrep + 1), b.block_rep + b.block_off[colour], b.cbegin,
-                b.ccount, b.ncol, b.total[colour], colour, b.ctr, nmetro, j);
+                b.ccount, b.ncol, b.total[colour], colour, b.ctr, e_off, nmetro, j);
         }
     if (b.meas_blocks > 0)
-        batch_measure<F32><<<b.meas_blocks, 256, 0, st>>>(b.reps, b.ctr, b.acc, b.nrep, b.meas_prefix, b.meas_rep);
-    batch_tick<<<1, 1, 0, st>>>(b.ctr);
+        batch_measure<F32><<<b.meas_blocks, 256, 0, st>>>(b.reps, b.ctr, e_off, b.acc, b.nrep, b.meas_prefix,
+                                                          b.meas_rep);
+    return cudaGetLastError();
 }
 
-cudaError_t batch_launch_emcs(const BatchLaunch& b, cudaStream_t st, int ncluster, int nmetro)
+cudaError_t batch_launch_emcs(const BatchLaunch& b, cudaStream_t st, int ncluster, int nmetro, uint32_t e_off)
 {
-    if (b.f32) launch_emcs_t<true>(b, st, ncluster, nmetro);
-    else launch_emcs_t<false>(b, st, ncluster, nmetro);
+    return b.f32 ? launch_emcs_t<true>(b, st, ncluster, nmetro, e_off)
+                 : launch_emcs_t<false>(b, st, ncluster, nmetro, e_off);
+}
+
+cudaError_t batch_launch_tick(const BatchLaunch& b, cudaStream_t st, uint32_t count)
+{
+    batch_tick<<<1, 1, 0, st>>>(b.ctr, count);
     return cudaGetLastError();
 }
 

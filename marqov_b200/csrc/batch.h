@@ -21,19 +21,49 @@ struct BatchRep {
     const unsigned long long* cuts;  // int8: the member's Metropolis cut table
     int D;                           // int8: its maximum degree
     int resident;                    // runs in one CTA's shared memory (batch_resident), not in the graphs
-    int tile;                        // labelling order (ccl_site): 0 site order, 2 16x16 tiles, 3 8x8x4 tiles
+    // labelling in bit tiles (wolff_tile.cuh): words per x-line, tiles in y and
+    // z, their number (0: the lattice is labelled site by site), scratch
+    int tl_nw, tl_ny, tl_nz, tl_tiles;
+    int* tl_forest;             // [tiles * units * 32] global parents of local roots
+    unsigned short* tl_lab;     // [tiles * units * 32] local root of every run
+    uint32_t *tl_cand, *tl_xb;  // [tiles * units] candidate and x-bond words
 };
 
-// Labelling order of a lattice: 2D stencils with len % 16 == 0 in 16 x 16
-// tiles, 3D stencils with len % 8 == 0 in 8 x 8 x 4 tiles (256 sites, one
-// CTA block of the labelling kernels each), others in site order.
-inline int ccl_tile_kind(int lat_kind, int dim, int len)
+// One cluster of a run: EMCS e_off after the device counter, cluster c of
+// ncluster, and what is added to its serial (single handles).
+struct ClusterStep {
+    uint32_t e_off, serial_add;
+    int ncluster, c;
+};
+
+// Units (32-site words of an x-line, one thread each) of a tile in y, in 3D
+constexpr __host__ __device__ int tile_ty3(int units) { return units >= 256 ? 16 : 8; }
+
+// Tiles of `units` units that cover a lattice (n = 0: not labelled in tiles:
+// CSR graphs, one- and four-dimensional lattices, ids beyond 31 bits).
+struct TileShape {
+    int nw = 0, ny = 0, nz = 0, n = 0;
+    size_t bytes(int units) const { return (size_t)n * units * (32 * 4 + 32 * 2 + 2 * 4); }
+};
+inline TileShape tile_shape(int lat_kind, int dim, int len, int units)
 {
-    if (lat_kind != MQV_LATTICE_HYPERCUBIC) return 0;
-    if (dim == 2 && len % 16 == 0) return 2;
-    if (dim == 3 && len % 8 == 0) return 3;
-    return 0;
+    TileShape t;
+    if (lat_kind != MQV_LATTICE_HYPERCUBIC || dim < 2 || dim > 3) return t;
+    const int ty = dim == 2 ? units : tile_ty3(units), tz = units / ty;
+    t.nw = (len + 31) / 32;
+    t.ny = (len + ty - 1) / ty;
+    t.nz = dim == 3 ? (len + tz - 1) / tz : 1;
+    const int64_t n = (int64_t)t.nw * t.ny * t.nz;
+    if (n * units * 32 >= (int64_t)1 << 31) return TileShape{};
+    t.n = (int)n;
+    return t;
 }
+inline int64_t tile_lattice_units(int dim, int len)
+{
+    return (int64_t)((len + 31) / 32) * len * (dim == 3 ? len : 1);
+}
+// Units per tile for so many units in all.
+int tile_units(int64_t total);
 
 // Sites of a member's lattice.
 __host__ __device__ __forceinline__ int64_t rep_sites(const BatchRep& R)
@@ -73,7 +103,12 @@ struct BatchLaunch {
     const int32_t* meas_prefix;  // [nrep + 1]
     const int32_t* meas_rep;     // [meas_blocks]
     int meas_blocks;
-    // site-level work (every site of every member) for the labelling Wolff
+    // labelling in bit tiles: tiles of member r from tile_prefix[r], tile_rep[t]
+    // the member of tile t
+    const int32_t* tile_prefix;  // [nrep + 1]
+    const int32_t* tile_rep;     // [tiles]
+    int tiles, tile_units;
+    // site-level work (every site of every other member) for the labelling Wolff
     const int64_t* site_prefix;  // [nrep + 1]
     const int32_t* site_block_rep;
     int64_t total_sites;
@@ -85,7 +120,12 @@ struct BatchLaunch {
     int32_t* csize;              // cluster sizes: (slot * ncluster + c) * nrep + r
 };
 
-cudaError_t batch_launch_emcs(const BatchLaunch& b, cudaStream_t st, int ncluster, int nmetro);
+// one EMCS, e_off after the device counter; batch_launch_tick advances it
+cudaError_t batch_launch_emcs(const BatchLaunch& b, cudaStream_t st, int ncluster, int nmetro, uint32_t e_off);
+cudaError_t batch_launch_tick(const BatchLaunch& b, cudaStream_t st, uint32_t count);
+void tile_bind(BatchRep& r, const TileShape& t, int units, void* scratch);
+// the three launches of one cluster labelled in bit tiles (every tiled member)
+cudaError_t launch_tile_cluster(const BatchLaunch& b, cudaStream_t st, const ClusterStep& k);
 // EMCS e0 .. e0 + count - 1 of the resident members order[0 .. nres) (the
 // largest with max_n sites), measurement slots from slot0 (smem_emcs.cu)
 cudaError_t batch_launch_resident(const BatchLaunch& b, cudaStream_t st, const int32_t* order, int nres, size_t smem,
@@ -104,14 +144,15 @@ cudaError_t batch_launch_samples(const BatchLaunch& b, cudaStream_t st, int nslo
 // the energies of the EMCS just done; perm/flags as batch_temper describes
 cudaError_t batch_launch_temper(const BatchLaunch& b, cudaStream_t st, const int32_t* pairs, int npairs, uint32_t step,
                                 uint64_t seed, double en_min, double en_max, int32_t* perm, int32_t* flags);
-// kernel launches of one EMCS
+// kernel launches of one EMCS (the counter tick of a graph apart)
 inline uint64_t batch_launches_per_emcs(const BatchLaunch& b, int ncluster, int nmetro)
 {
     int live = 0;
     for (int c = 0; c < b.ncol; ++c) live += b.total[c] > 0;
-    const uint64_t ccl = b.site_blocks > 0 ? 5ull : 0ull;  // seed, local, hook, halve, flip
+    // label, hook, flip of the tiled members; seed, local, hook, halve, flip of the others
+    const uint64_t ccl = (b.tiles > 0 ? 3ull : 0ull) + (b.site_blocks > 0 ? 5ull : 0ull);
     return (uint64_t)ncluster * (b.wolff_ccl ? ccl : 1ull) + (uint64_t)nmetro * (uint64_t)live +
-           (b.meas_blocks > 0 ? 2ull : 1ull);
+           (b.meas_blocks > 0 ? 1ull : 0ull);
 }
 
 }  // namespace mqv

@@ -39,6 +39,7 @@ int wolff_noalloc_max_clusters();
 cudaError_t wolff_noalloc_scratch(int device, uint32_t** out);
 cudaError_t launch_wolff_int8_noalloc(Sim* s, uint32_t* scratch, int slot);
 const int32_t* wolff_noalloc_sizes(const uint32_t* scratch);
+bool label_in_tiles(const Sim* s);
 bool resident_fits(const Sim* s);
 cudaError_t launch_emcs_cluster(Sim* s, int n_emcs, int ncluster, int nmetro, long long* acc, int32_t* csize);
 cudaError_t launch_emcs_resident(Sim* s, int n_emcs, int ncluster, int nmetro, bool measure, long long* acc,
@@ -110,7 +111,7 @@ static void free_sim(Sim* s)
     for (void* p : {s->state[0], s->state[1], (void*)s->d_rp, (void*)s->d_ci, (void*)s->d_bonds, (void*)s->d_order,
                     (void*)s->d_acc, (void*)s->d_obs, (void*)s->d_visited, (void*)s->d_queue, (void*)s->d_csize,
                     (void*)s->d_status, (void*)s->d_counter, (void*)s->d_cuts, (void*)s->d_rep1, (void*)s->d_ctr1,
-                    s->d_seed1, (void*)s->d_sprefix1, (void*)s->d_sbrep1})
+                    s->d_seed1, (void*)s->d_sprefix1, (void*)s->d_sbrep1, (void*)s->d_ttab1, s->d_tile})
         if (p) cudaFree(p);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -381,9 +382,12 @@ static bool cluster_by_label(const Sim* s)
 
 static mqv_status launch_cluster(Sim* s, int slot)
 {
-    mqv_status st = ensure_wolff(s);
-    if (st) return st;
-    if (cluster_by_label(s)) MQV_CK(launch_wolff_label(s, slot));
+    const bool label = cluster_by_label(s);
+    if (!label || !label_in_tiles(s)) {
+        const mqv_status st = ensure_wolff(s);
+        if (st) return st;
+    }
+    if (label) MQV_CK(launch_wolff_label(s, slot));
     else MQV_CK(s->is_f32 ? launch_wolff_f32(s, slot) : launch_wolff_int8(s, slot));
     return MQV_OK;
 }
@@ -1078,11 +1082,12 @@ MQV_API mqv_status mqv_selftest_philox(uint64_t seed, uint32_t c1, uint32_t c2, 
 
 namespace mqv {
 
-// host mirror of the labelling Wolff's per-member seed (wolff_ccl.cuh)
+// host mirror of the labelling Wolff's per-member seed (wolff_tile.cuh)
 struct CclSeedHost {
     int64_t rsite;
     int val, newq;
     float r[3];
+    double a;
 };
 
 struct Batch {
@@ -1113,6 +1118,13 @@ struct Batch {
     int32_t* d_meas_prefix = nullptr;
     int32_t* d_meas_rep = nullptr;
     void* d_ccl_seeds = nullptr;
+    // labelling in bit tiles: tables, scratch of every tiled member (at
+    // tile_off[r] bytes), allocated by the first run with clusters
+    int32_t* d_tile_prefix = nullptr;
+    int32_t* d_tile_rep = nullptr;
+    void* d_tile = nullptr;
+    size_t tile_bytes = 0;
+    std::vector<size_t> tile_off;
     int wolff_mode = MQV_WOLFF_AUTO;
     // MQV_WOLFF_AUTO: ms per EMCS of breadth first [0] and labelling [1] when
     // last timed (-1: never), the one in use, EMCS since the other was tried
@@ -1171,7 +1183,8 @@ static void free_batch(Batch* b)
     for (void* p : {(void*)b->d_reps, (void*)b->d_prefix, (void*)b->d_block_rep, (void*)b->d_cbegin,
                     (void*)b->d_ccount, (void*)b->d_res_order, (void*)b->d_ctr,
                     (void*)b->d_acc, (void*)b->d_obs, (void*)b->d_csize, (void*)b->d_site_prefix,
-                    (void*)b->d_site_block_rep, (void*)b->d_meas_prefix, (void*)b->d_meas_rep, b->d_ccl_seeds})
+                    (void*)b->d_site_block_rep, (void*)b->d_meas_prefix, (void*)b->d_meas_rep, b->d_ccl_seeds,
+                    (void*)b->d_tile_prefix, (void*)b->d_tile_rep, b->d_tile})
         if (p) cudaFree(p);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
@@ -1207,7 +1220,9 @@ static mqv_status batch_capture(Batch* b, int steps, int ncluster, int nmetro, c
     cudaGraph_t graph = nullptr;
     MQV_CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaSuccess;
-    for (int k = 0; k < steps && e == cudaSuccess; ++k) e = batch_launch_emcs(b->L, b->stream, ncluster, nmetro);
+    for (int k = 0; k < steps && e == cudaSuccess; ++k)
+        e = batch_launch_emcs(b->L, b->stream, ncluster, nmetro, (uint32_t)k);
+    if (e == cudaSuccess) e = batch_launch_tick(b->L, b->stream, (uint32_t)steps);
     const cudaError_t e2 = cudaStreamEndCapture(b->stream, &graph);
     MQV_CK(e);
     MQV_CK(e2);
@@ -1259,6 +1274,8 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
             if (st) return st;
         }
     }
+    if (ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile)
+        MQV_CK(cudaMalloc(&b->d_tile, b->tile_bytes));
     // member table at the start of the run
     b->reps.assign((size_t)b->nrep, BatchRep{});
     for (int i = 0; i < b->nrep; ++i) {
@@ -1280,7 +1297,10 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         r.cuts = s->d_cuts;
         r.D = s->max_degree;
         r.resident = b->resident[(size_t)i] ? 1 : 0;
-        r.tile = ccl_tile_kind(s->lat_kind, s->dim, s->len);
+        if (b->d_tile && !b->resident[(size_t)i]) {
+            const TileShape ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile_units);
+            if (ts.n) tile_bind(r, ts, b->L.tile_units, (char*)b->d_tile + b->tile_off[(size_t)i]);
+        }
     }
     MQV_CK(cudaMemcpyAsync(b->d_reps, b->reps.data(), sizeof(BatchRep) * b->reps.size(), cudaMemcpyHostToDevice,
                            b->stream));
@@ -1292,6 +1312,9 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     if (st) return st;
     if (b->d_acc != acc0 || b->d_csize != csize0) free_graphs(b);  // graphs hold the old pointers
     const int K = std::max(1, std::min(b->graph_steps, CH));
+    // the cost of breadth-first growth follows the clusters: while the choice
+    // is by timing, chunks are short enough to follow it too
+    const int max_chunk = b->wolff_mode == MQV_WOLFF_AUTO && ncluster > 0 ? 64 : CH;
     // Cluster algorithm: fixed, or (MQV_WOLFF_AUTO) chosen by measurement.
     // Both give the same clusters, so switching never changes the chain; the
     // cost of breadth-first growth follows the clusters (it rises as a farm
@@ -1383,7 +1406,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         if (K > 1)
             for (; j + K <= count; j += K) MQV_CK(cudaGraphLaunch(b->g_many[w], b->stream));
         for (; j < count; ++j) MQV_CK(cudaGraphLaunch(b->g_one[w], b->stream));
-        b->launches += per_emcs[w] * (uint64_t)count;
+        b->launches += per_emcs[w] * (uint64_t)count + (uint64_t)(count / K) + (uint64_t)(count % K);
         for (int i = 0; i < nside; ++i) MQV_CK(cudaStreamWaitEvent(b->stream, b->join_ev[i], 0));
         return MQV_OK;
     };
@@ -1400,7 +1423,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     std::vector<int32_t> csz;
     int done = 0;
     while (done < n_emcs) {
-        const int ch = std::min(n_emcs - done, CH);
+        const int ch = std::min(n_emcs - done, max_chunk);
         done_run = done;
         MQV_CK(cudaMemsetAsync(b->d_acc, 0, sizeof(long long) * kAccStride * (size_t)ch * b->nrep, b->stream));
         MQV_CK(batch_launch_chunk_start(b->L, b->stream, (uint32_t)done));
@@ -1410,7 +1433,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         if (adapt) {
             const double* est = b->wolff_est;
             const double r = est[w_try] > 0 && est[w_main] > 0 ? std::max(1.0, est[w_try] / est[w_main]) : 1.0;
-            if (est[w_try] < 0 || (double)b->wolff_since_try >= 256.0 * r) x = std::min(4, ch / 2);
+            if (est[w_try] < 0 || (double)b->wolff_since_try >= 256.0 * r) x = std::min(K, ch / 2);
         }
         int k = 0;
         // `count` EMCS from chunk position k, an exchange step where one ends
@@ -1648,9 +1671,30 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         }
     }
     if (brep.empty()) brep.push_back(0);
-    // site-level work of the labelling Wolff
+    // labelling Wolff: the tiles of the members labelled in bit tiles, the
+    // sites of the others
+    int64_t units = 0;
+    for (int r = 0; r < n; ++r) {
+        const Sim* s = b->sims[(size_t)r];
+        if (!b->resident[(size_t)r] && tile_shape(s->lat_kind, s->dim, s->len, 64).n) units += tile_lattice_units(s->dim, s->len);
+    }
+    b->L.tile_units = tile_units(units);
+    std::vector<int32_t> tprefix((size_t)n + 1, 0), trep;
     std::vector<int64_t> sprefix((size_t)n + 1, 0);
-    for (int r = 0; r < n; ++r) sprefix[r + 1] = sprefix[r] + (b->resident[(size_t)r] ? 0 : b->sims[(size_t)r]->n);
+    b->tile_off.assign((size_t)n, 0);
+    for (int r = 0; r < n; ++r) {
+        const Sim* s = b->sims[(size_t)r];
+        TileShape ts;
+        if (!b->resident[(size_t)r]) ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile_units);
+        if ((int64_t)tprefix[(size_t)r] + ts.n >= (int64_t)1 << 31) return bail(fail(MQV_ERR_INVALID_ARG, "batch too large"));
+        tprefix[(size_t)r + 1] = tprefix[(size_t)r] + ts.n;
+        trep.insert(trep.end(), (size_t)ts.n, (int32_t)r);
+        b->tile_off[(size_t)r] = b->tile_bytes;
+        b->tile_bytes += (ts.bytes(b->L.tile_units) + 255) / 256 * 256;
+        sprefix[r + 1] = sprefix[r] + (b->resident[(size_t)r] || ts.n ? 0 : s->n);
+    }
+    b->L.tiles = (int)trep.size();
+    if (trep.empty()) trep.push_back(0);
     const int64_t sblocks = (sprefix[n] + kBatchMetroThreads - 1) / kBatchMetroThreads;
     if (sblocks >= (int64_t)1 << 31) return bail(fail(MQV_ERR_INVALID_ARG, "batch too large"));
     std::vector<int32_t> sbrep((size_t)std::max<int64_t>(sblocks, 1), 0);
@@ -1683,6 +1727,8 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     if (!st) st = dcopy((void**)&b->d_block_rep, brep.data(), sizeof(int32_t) * brep.size());
     if (!st) st = dcopy((void**)&b->d_cbegin, cbegin.data(), sizeof(int32_t) * std::max<size_t>(cbegin.size(), 1));
     if (!st) st = dcopy((void**)&b->d_ccount, ccount.data(), sizeof(int32_t) * std::max<size_t>(ccount.size(), 1));
+    if (!st) st = dcopy((void**)&b->d_tile_prefix, tprefix.data(), sizeof(int32_t) * tprefix.size());
+    if (!st) st = dcopy((void**)&b->d_tile_rep, trep.data(), sizeof(int32_t) * trep.size());
     if (!st) st = dcopy((void**)&b->d_site_prefix, sprefix.data(), sizeof(int64_t) * sprefix.size());
     if (!st) st = dcopy((void**)&b->d_site_block_rep, sbrep.data(), sizeof(int32_t) * sbrep.size());
     if (st) return bail(st);
@@ -1711,6 +1757,8 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     b->L.meas_prefix = b->d_meas_prefix;
     b->L.meas_rep = b->d_meas_rep;
     b->L.meas_blocks = (int)mprefix[(size_t)n];
+    b->L.tile_prefix = b->d_tile_prefix;
+    b->L.tile_rep = b->d_tile_rep;
     b->L.site_prefix = b->d_site_prefix;
     b->L.site_block_rep = b->d_site_block_rep;
     b->L.total_sites = sprefix[n];

@@ -291,6 +291,11 @@ struct Sim {
     void* d_seed1 = nullptr;
     int64_t* d_sprefix1 = nullptr;
     int32_t* d_sbrep1 = nullptr;
+    std::vector<unsigned char> rep1_host;  // what d_rep1 holds
+    // labelling in bit tiles (wolff_tile.cuh): its tables, scratch, units per tile
+    int32_t* d_ttab1 = nullptr;
+    void* d_tile = nullptr;
+    int tile_units = 0;
     uint64_t launches = 0;
 };
 

@@ -17,6 +17,7 @@
 // the bitmap is zero again for the next cluster.
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <mutex>
 
 #include "wolff_ccl.cuh"
@@ -87,21 +88,23 @@ cudaError_t launch_wolff_int8(Sim* s, int slot)
 
 // ---------------------------------------------------------------------------
 // One cluster of one lattice by connected-component labelling (the batched
-// path's kernels, wolff_ccl.cuh, over a one-member table): a fixed number of
-// whole-lattice passes whatever the cluster's depth, where a breadth-first
-// growth pays a CTA barrier per level -- thousands of levels for a critical
-// cluster on a large lattice.  The labels are the handle's queue (n int32).
+// path's kernels over a one-member table: wolff_tile.cuh for 2D and 3D
+// lattices, wolff_ccl.cuh for the others): a fixed number of whole-lattice
+// passes whatever the cluster's depth, where a breadth-first growth pays a
+// CTA barrier per level -- thousands of levels for a critical cluster on a
+// large lattice.
 
-__global__ void single_rep_set(BatchRep* __restrict__ d, BatchRep r, BatchCtr* __restrict__ ctr, uint32_t serial)
+__global__ void single_rep_set(BatchRep* __restrict__ d, BatchRep r, BatchCtr* __restrict__ ctr)
 {
     *d = r;
-    ctr->e = serial;  // serial = cluster0 (0) + e * 1 + 0; slot = e - ebase = 0
-    ctr->ebase = serial;
+    ctr->e = 0;
+    ctr->ebase = 0;
 }
 
 static BatchRep single_rep(const Sim* s)
 {
-    BatchRep r{};
+    BatchRep r;
+    std::memset((void*)&r, 0, sizeof r);
     r.md = s->md;
     r.st = s->sten;
     r.csr = s->csr;
@@ -110,15 +113,24 @@ static BatchRep single_rep(const Sim* s)
     if (!s->is_f32) r.w = wolff_int8_params(s->md);
     r.key = make_key(s->seed);
     r.replica = s->replica;
-    r.sweep0 = (uint32_t)s->sweep;
+    r.sweep0 = 0;
     r.cluster0 = 0;
     r.s = s->state[s->cur];
     r.visited = s->d_visited;
     r.queue = s->d_queue;
     r.cuts = s->d_cuts;
     r.D = s->max_degree;
-    r.tile = ccl_tile_kind(s->lat_kind, s->dim, s->len);
+    if (s->d_tile) tile_bind(r, tile_shape(s->lat_kind, s->dim, s->len, s->tile_units), s->tile_units, s->d_tile);
     return r;
+}
+
+// The one-member table holds `r` (written only when something changed).
+static void set_single_rep(Sim* s, const BatchRep& r)
+{
+    if (s->rep1_host.size() == sizeof r && std::memcmp(s->rep1_host.data(), &r, sizeof r) == 0) return;
+    s->rep1_host.assign((const unsigned char*)&r, (const unsigned char*)&r + sizeof r);
+    single_rep_set<<<1, 1, 0, s->stream>>>(s->d_rep1, r, s->d_ctr1);
+    s->launches++;
 }
 
 template <bool F32>
@@ -127,30 +139,50 @@ static void launch_label_t(Sim* s, int32_t* csize)
     const int64_t n = s->n;
     const unsigned gb = (unsigned)((n + kBatchMetroThreads - 1) / kBatchMetroThreads);
     CclSeed* sd = (CclSeed*)s->d_seed1;
-    single_rep_set<<<1, 1, 0, s->stream>>>(s->d_rep1, single_rep(s), s->d_ctr1, (uint32_t)s->cluster);
-    ccl_seed<F32><<<1, 32, 0, s->stream>>>(s->d_rep1, s->d_ctr1, 1, 0, sd, csize, 1);
-    ccl_local<F32><<<gb, kBatchMetroThreads, 0, s->stream>>>(s->d_rep1, s->d_sprefix1, s->d_sbrep1, n, sd, s->d_ctr1,
-                                                             1, 0);
-    ccl_hook<F32><<<gb, kBatchMetroThreads, 0, s->stream>>>(s->d_rep1, s->d_sprefix1, s->d_sbrep1, n, sd, s->d_ctr1,
-                                                            1, 0);
+    const ClusterStep k{0u, (uint32_t)s->cluster, 1, 0};
+    ccl_seed<F32><<<1, 32, 0, s->stream>>>(s->d_rep1, s->d_ctr1, k, sd, csize, 1);
+    ccl_local<F32><<<gb, kBatchMetroThreads, 0, s->stream>>>(s->d_rep1, s->d_sprefix1, s->d_sbrep1, n, sd, s->d_ctr1, k);
+    ccl_hook<F32><<<gb, kBatchMetroThreads, 0, s->stream>>>(s->d_rep1, s->d_sprefix1, s->d_sbrep1, n, sd, s->d_ctr1, k);
     ccl_halve<<<gb, kBatchMetroThreads, 0, s->stream>>>(s->d_rep1, s->d_sprefix1, s->d_sbrep1, n);
-    ccl_flip<F32><<<gb, kBatchMetroThreads, 0, s->stream>>>(s->d_rep1, s->d_sprefix1, s->d_sbrep1, n, sd, s->d_ctr1, 1,
-                                                            0, csize, 1);
-    s->launches += 6;
+    ccl_flip<F32><<<gb, kBatchMetroThreads, 0, s->stream>>>(s->d_rep1, s->d_sprefix1, s->d_sbrep1, n, sd, s->d_ctr1, k,
+                                                            csize, 1);
+    s->launches += 5;
 }
 
-// The one-member tables of the labelling path, allocated on first use.
-cudaError_t ensure_label_tables(Sim* s)
+// The one-member tables of the labelling path and of the cluster-resident
+// kernel, allocated on first use; `label`: with the labelling's scratch.
+cudaError_t ensure_label_tables(Sim* s, bool label)
 {
-    if (s->d_sbrep1) return cudaSuccess;  // allocated last: all tables present
     const int64_t n = s->n;
-    const int64_t gb = (n + kBatchMetroThreads - 1) / kBatchMetroThreads;
-    const int64_t pre[2] = {0, n};
     cudaError_t e = cudaSuccess;
     if (!s->d_rep1) e = cudaMalloc(&s->d_rep1, sizeof(BatchRep));
     if (e == cudaSuccess && !s->d_ctr1) e = cudaMalloc(&s->d_ctr1, sizeof(BatchCtr));
     if (e == cudaSuccess && !s->d_seed1) e = cudaMalloc(&s->d_seed1, sizeof(CclSeed));
-    if (e == cudaSuccess && !s->d_sprefix1) e = cudaMalloc(&s->d_sprefix1, sizeof(pre));
+    const int units = tile_units(s->lat_kind == MQV_LATTICE_HYPERCUBIC ? tile_lattice_units(s->dim, s->len) : 0);
+    const TileShape ts = tile_shape(s->lat_kind, s->dim, s->len, units);
+    if (label && ts.n && e == cudaSuccess && !s->d_tile) {
+        // tables: the tiles' prefix {0, n}, every tile's member 0
+        const int32_t pre[2] = {0, ts.n};
+        int32_t* tab = nullptr;
+        const size_t words = (size_t)ts.n + 2;
+        e = cudaMalloc(&tab, sizeof(int32_t) * words);
+        if (e == cudaSuccess) e = cudaMemsetAsync(tab, 0, sizeof(int32_t) * words, s->stream);
+        if (e == cudaSuccess) e = upload_sync(s->stream, tab, pre, sizeof(pre));
+        void* scratch = nullptr;
+        if (e == cudaSuccess) e = cudaMalloc(&scratch, ts.bytes(units));
+        if (e == cudaSuccess) {
+            s->d_ttab1 = tab;
+            s->d_tile = scratch;
+            s->tile_units = units;
+        } else if (tab) {
+            cudaFree(tab);
+        }
+    }
+    if (e != cudaSuccess || s->d_sbrep1 || (label && ts.n)) return e;
+    // site-by-site labelling (and the member list of the cluster-resident kernel)
+    const int64_t gb = (n + kBatchMetroThreads - 1) / kBatchMetroThreads;
+    const int64_t pre[2] = {0, n};
+    if (!s->d_sprefix1) e = cudaMalloc(&s->d_sprefix1, sizeof(pre));
     // on the handle's stream, before the kernels that read them
     if (e == cudaSuccess) e = upload_sync(s->stream, s->d_sprefix1, pre, sizeof(pre));
     int32_t* brep = nullptr;
@@ -165,31 +197,57 @@ cudaError_t ensure_label_tables(Sim* s)
 // (cluster_emcs.cu) through the one-member table; acc NULL: no measurement.
 cudaError_t launch_emcs_cluster(Sim* s, int n_emcs, int ncluster, int nmetro, long long* acc, int32_t* csize)
 {
-    cudaError_t e = ensure_label_tables(s);
+    cudaError_t e = ensure_label_tables(s, false);
     if (e != cudaSuccess) return e;
     BatchRep r = single_rep(s);
     r.cluster0 = (uint32_t)s->cluster;
-    single_rep_set<<<1, 1, 0, s->stream>>>(s->d_rep1, r, s->d_ctr1, 0u);
+    r.sweep0 = (uint32_t)s->sweep;
+    set_single_rep(s, r);
     BatchLaunch b{};
     b.reps = s->d_rep1;
     b.nrep = 1;
     b.acc = acc;
     b.csize = csize;
     e = batch_launch_cluster(b, s->stream, s->d_sbrep1, 1, cluster_ctas(s->n), 0u, 0, n_emcs, ncluster, nmetro);
-    s->launches += 2;
+    s->launches++;
     s->sweep += (uint64_t)n_emcs * (uint64_t)nmetro;
     s->cluster += (uint64_t)n_emcs * (uint64_t)ncluster;
     return e;
 }
 
+// whether the lattice is labelled in bit tiles (which need no cluster queue)
+bool label_in_tiles(const Sim* s)
+{
+    return s->lat_kind == MQV_LATTICE_HYPERCUBIC &&
+           tile_shape(s->lat_kind, s->dim, s->len, tile_units(tile_lattice_units(s->dim, s->len))).n > 0;
+}
+
 cudaError_t launch_wolff_label(Sim* s, int slot)
 {
-    const cudaError_t e = ensure_label_tables(s);
+    cudaError_t e = ensure_label_tables(s, true);
     if (e != cudaSuccess) return e;
-    if (s->is_f32) launch_label_t<true>(s, s->d_csize + slot);
-    else launch_label_t<false>(s, s->d_csize + slot);
+    set_single_rep(s, single_rep(s));
+    if (s->d_tile) {
+        BatchLaunch b{};
+        b.reps = s->d_rep1;
+        b.nrep = 1;
+        b.f32 = s->is_f32 ? 1 : 0;
+        b.tile_prefix = s->d_ttab1;
+        b.tile_rep = s->d_ttab1 + 2;
+        b.tiles = tile_shape(s->lat_kind, s->dim, s->len, s->tile_units).n;
+        b.tile_units = s->tile_units;
+        b.ccl_seeds = s->d_seed1;
+        b.ctr = s->d_ctr1;
+        b.csize = s->d_csize + slot;
+        e = launch_tile_cluster(b, s->stream, ClusterStep{0u, (uint32_t)s->cluster, 1, 0});
+        s->launches += 3;
+    } else {
+        if (s->is_f32) launch_label_t<true>(s, s->d_csize + slot);
+        else launch_label_t<false>(s, s->d_csize + slot);
+        e = cudaGetLastError();
+    }
     s->cluster++;
-    return cudaGetLastError();
+    return e;
 }
 
 // ---------------------------------------------------------------------------
