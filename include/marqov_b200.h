@@ -130,8 +130,10 @@ enum {
                                  keeps the state in shared memory for a whole chunk of EMCS; launch
                                  per cluster, colour and measurement instead (same results) */
     MQV_FLAG_RESIDENT = 4     /* take the resident path wherever the lattice fits it.  Default (neither
-                                 flag): a single handle is resident up to 16384 sites; batch members
-                                 run on the batch's graph path */
+                                 flag): a single handle is resident up to 16384 sites, Ising-type 2D and
+                                 3D lattices (held as bit planes; bonds +-1) up to 32768 sites; these
+                                 are resident in a batch too (spin glasses up to 65536 sites), the
+                                 batch's other members run on its graph path */
 };
 
 typedef struct mqv_run_params {
@@ -203,8 +205,8 @@ MQV_API mqv_status mqv_metropolis(mqv_sim* sim, int32_t nsweeps);
  * activated-bond components in a fixed number of whole-lattice passes. */
 enum { MQV_WOLFF_AUTO = 0, MQV_WOLFF_BFS = 1, MQV_WOLFF_LABEL = 2 };
 /* No counterpart in the reference.  The cluster algorithm of a handle:
- * MQV_WOLFF_AUTO (default) labels int8 lattices of at least 2^18 sites and
- * grows the others breadth first; lattices on the resident path
+ * MQV_WOLFF_AUTO (default) labels int8 lattices of at least 2^18 sites (2D and
+ * 3D hypercubic ones from 2^15) and grows the others breadth first; lattices on the resident path
  * (MQV_FLAG_NO_RESIDENT unset, int8 stencils of <= 262144 sites) label in
  * (distributed) shared memory. */
 MQV_API mqv_status mqv_set_wolff(mqv_sim* sim, int32_t algorithm);

@@ -43,8 +43,9 @@ class Config:
     per_colour: bool = False
     # int8 stencil lattices of <= 65536 sites (one CTA) or <= 262144 sites (a
     # thread-block cluster) can run whole chunks of EMCS in shared memory.
-    # None: the engine decides (single handles up to 16384 sites; batch
-    # members take the batch's graph path); True: wherever the lattice fits;
+    # None: the engine decides (single handles up to 16384 sites, Ising-type
+    # lattices, which are held as bit planes, up to 32768 sites, also in a
+    # batch, whose other members take its graph path); True: wherever the lattice fits;
     # False: never (launch per step).  The results are the same.
     resident: bool | None = None
 
@@ -238,7 +239,8 @@ class Core:
 
     def set_wolff(self, algorithm: str):
         """Cluster algorithm of this lattice: "auto" (labelling for int8 lattices
-        of >= 2^18 sites), "bfs" or "label"; the clusters are the same."""
+        of >= 2^18 sites, 2D and 3D ones from 2^15), "bfs" or "label"; the
+        clusters are the same."""
         code = {"auto": L.WOLFF_AUTO, "bfs": L.WOLFF_BFS, "label": L.WOLFF_LABEL}[algorithm]
         L.check(self._lib.mqv_set_wolff(self._h, code))
 

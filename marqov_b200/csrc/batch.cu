@@ -182,11 +182,12 @@ __global__ void batch_samples(const long long* __restrict__ acc, int nslots, int
 // swaps the members' state pointers in the member table (the graphs read
 // them there) and in the permutation the host applies to its handles.
 template <bool F32>
-__global__ void batch_temper(BatchRep* __restrict__ reps, const BatchCtr* __restrict__ ctr,
-                             const long long* __restrict__ acc, int nrep, const int32_t* __restrict__ pairs,
-                             int npairs, uint32_t step, Key key, double en_min, double en_max,
+__global__ void batch_temper(BatchRep* __restrict__ reps, int slot, const long long* __restrict__ acc, int nrep,
+                             const int32_t* __restrict__ pairs, int npairs, uint32_t step, Key key, double en_min, double en_max,
                              int32_t* __restrict__ perm, int32_t* __restrict__ flags)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npairs) return;
     const int a = pairs[2 * p], b = pairs[2 * p + 1];
@@ -194,7 +195,6 @@ __global__ void batch_temper(BatchRep* __restrict__ reps, const BatchCtr* __rest
         flags[p] = -1;
         return;
     }
-    const uint32_t slot = ctr->e - 1u - ctr->ebase;
     double oa[4], ob[4];
     BatchRep& Ra = reps[a];
     BatchRep& Rb = reps[b];
@@ -245,20 +245,26 @@ static cudaError_t launch_tile_t(const BatchLaunch& b, cudaStream_t st, const Cl
 }
 
 // Units per tile and lanes per unit by the units of all members, measured (us
-// per cluster with (64, 8) / (64, 4) / (128, 2)): 2 K units (2D L = 256) 28 /
-// 33 / 45, 16 K (32 x L = 128) 38 / 41 / 53, 49 K (24 x L = 256) 54 / 40 / 41,
-// 131 K (L = 2048) 122 / 89 / 89, 524 K (L = 4096) 435 / 284 / 248: more lanes
-// per unit shorten the serial steps while the chip is not full.
-constexpr int64_t kTileUnits8 = 24576, kTileUnits4 = 98304;
-int tile_units(int64_t total) { return total < kTileUnits4 ? 64 : 128; }
+// per cluster with (64, 8) / (128, 4) / (64, 2) / (128, 1)): 2 K units (2D L =
+// 256) 27 / 29 / 36 / 50, 33 K (L = 1024) 48 / 36 / 44 / 58, 49 K (24 x L = 256)
+// 55 / 42 / 36 / 46, 131 K (L = 2048) 128 / 95 / 77 / 77, 262 K (32 phi^4
+// chains of 64^3) 380 / 284 / 221 / 215, 524 K (L = 4096) 451 / 311 / 212 /
+// 200: more lanes per unit shorten the steps while the chip is not full.
+TileConfig tile_config(int64_t units)
+{
+    return units < 24576 ? TileConfig{64, 8} : units < 40960 ? TileConfig{128, 4}
+         : units < 196608 ? TileConfig{64, 2} : TileConfig{128, 1};
+}
 
 cudaError_t launch_tile_cluster(const BatchLaunch& b, cudaStream_t st, const ClusterStep& k)
 {
     if (b.tiles == 0) return cudaSuccess;
-    if (b.tile_units == 128) return b.f32 ? launch_tile_t<true, 128, 2>(b, st, k) : launch_tile_t<false, 128, 2>(b, st, k);
-    if ((int64_t)b.tiles * 64 >= kTileUnits8)
-        return b.f32 ? launch_tile_t<true, 64, 4>(b, st, k) : launch_tile_t<false, 64, 4>(b, st, k);
-    return b.f32 ? launch_tile_t<true, 64, 8>(b, st, k) : launch_tile_t<false, 64, 8>(b, st, k);
+    switch (b.tile.lanes) {
+        case 8: return b.f32 ? launch_tile_t<true, 64, 8>(b, st, k) : launch_tile_t<false, 64, 8>(b, st, k);
+        case 4: return b.f32 ? launch_tile_t<true, 128, 4>(b, st, k) : launch_tile_t<false, 128, 4>(b, st, k);
+        case 2: return b.f32 ? launch_tile_t<true, 64, 2>(b, st, k) : launch_tile_t<false, 64, 2>(b, st, k);
+        default: return b.f32 ? launch_tile_t<true, 128, 1>(b, st, k) : launch_tile_t<false, 128, 1>(b, st, k);
+    }
 }
 
 void tile_bind(BatchRep& r, const TileShape& t, int units, void* scratch)
@@ -273,6 +279,7 @@ void tile_bind(BatchRep& r, const TileShape& t, int units, void* scratch)
     r.tl_lab = (unsigned short*)(p + u * 128);
     r.tl_cand = (uint32_t*)(p + u * 192);
     r.tl_xb = r.tl_cand + u;
+    r.tl_base = r.tl_xb + u;
 }
 
 template <bool F32>
@@ -336,18 +343,14 @@ cudaError_t batch_launch_finalize(const BatchLaunch& b, cudaStream_t st, int nsl
     return cudaGetLastError();
 }
 
-cudaError_t batch_launch_temper(const BatchLaunch& b, cudaStream_t st, const int32_t* pairs, int npairs, uint32_t step,
-                                uint64_t seed, double en_min, double en_max, int32_t* perm, int32_t* flags)
+cudaError_t batch_launch_temper(const BatchLaunch& b, cudaStream_t st, int slot, const int32_t* pairs, int npairs,
+                                uint32_t step, uint64_t seed, double en_min, double en_max, int32_t* perm, int32_t* flags)
 {
     if (npairs <= 0) return cudaSuccess;
     const unsigned g = (unsigned)((npairs + 127) / 128);
-    if (b.f32)
-        batch_temper<true><<<g, 128, 0, st>>>(const_cast<BatchRep*>(b.reps), b.ctr, b.acc, b.nrep, pairs, npairs, step,
-                                               make_key(seed), en_min, en_max, perm, flags);
-    else
-        batch_temper<false><<<g, 128, 0, st>>>(const_cast<BatchRep*>(b.reps), b.ctr, b.acc, b.nrep, pairs, npairs,
-                                                step, make_key(seed), en_min, en_max, perm, flags);
-    return cudaGetLastError();
+    auto* kernel = b.f32 ? batch_temper<true> : batch_temper<false>;
+    return launch_pdl(kernel, g, 128, st, const_cast<BatchRep*>(b.reps), slot, b.acc, b.nrep, pairs, npairs, step,
+                      make_key(seed), en_min, en_max, perm, flags);
 }
 
 cudaError_t batch_launch_samples(const BatchLaunch& b, cudaStream_t st, int nslots, int e0, int n_total,

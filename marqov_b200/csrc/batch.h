@@ -26,7 +26,8 @@ struct BatchRep {
     int tl_nw, tl_ny, tl_nz, tl_tiles;
     int* tl_forest;             // [tiles * units * 32] global parents of local roots
     unsigned short* tl_lab;     // [tiles * units * 32] local root of every run
-    uint32_t *tl_cand, *tl_xb;  // [tiles * units] candidate and x-bond words
+    // [tiles * units] candidate and x-bond words, first run of every unit
+    uint32_t *tl_cand, *tl_xb, *tl_base;
 };
 
 // One cluster of a run: EMCS e_off after the device counter, cluster c of
@@ -43,7 +44,7 @@ constexpr __host__ __device__ int tile_ty3(int units) { return units >= 256 ? 16
 // CSR graphs, one- and four-dimensional lattices, ids beyond 31 bits).
 struct TileShape {
     int nw = 0, ny = 0, nz = 0, n = 0;
-    size_t bytes(int units) const { return (size_t)n * units * (32 * 4 + 32 * 2 + 2 * 4); }
+    size_t bytes(int units) const { return (size_t)n * units * (32 * 4 + 32 * 2 + 3 * 4); }
 };
 inline TileShape tile_shape(int lat_kind, int dim, int len, int units)
 {
@@ -62,8 +63,11 @@ inline int64_t tile_lattice_units(int dim, int len)
 {
     return (int64_t)((len + 31) / 32) * len * (dim == 3 ? len : 1);
 }
-// Units per tile for so many units in all.
-int tile_units(int64_t total);
+// Units per tile and lanes per unit for so many units in all.
+struct TileConfig {
+    int units, lanes;
+};
+TileConfig tile_config(int64_t units);
 
 // Sites of a member's lattice.
 __host__ __device__ __forceinline__ int64_t rep_sites(const BatchRep& R)
@@ -107,7 +111,8 @@ struct BatchLaunch {
     // the member of tile t
     const int32_t* tile_prefix;  // [nrep + 1]
     const int32_t* tile_rep;     // [tiles]
-    int tiles, tile_units;
+    int tiles;
+    TileConfig tile;
     // site-level work (every site of every other member) for the labelling Wolff
     const int64_t* site_prefix;  // [nrep + 1]
     const int32_t* site_block_rep;
@@ -130,6 +135,9 @@ cudaError_t launch_tile_cluster(const BatchLaunch& b, cudaStream_t st, const Clu
 // largest with max_n sites), measurement slots from slot0 (smem_emcs.cu)
 cudaError_t batch_launch_resident(const BatchLaunch& b, cudaStream_t st, const int32_t* order, int nres, size_t smem,
                                   uint32_t e0, int slot0, int count, int ncluster, int nmetro, int device);
+// the same for Ising-type members held as bit planes (bits_emcs.cu)
+cudaError_t batch_launch_bits(const BatchLaunch& b, cudaStream_t st, const int32_t* order, int nmem, size_t smem,
+                              uint32_t e0, int slot0, int count, int ncluster, int nmetro, int device);
 // the same for members held by clusters of `ctas` CTAs (cluster_emcs.cu)
 cudaError_t batch_launch_cluster(const BatchLaunch& b, cudaStream_t st, const int32_t* order, int nmem, int ctas,
                                  uint32_t e0, int slot0, int count, int ncluster, int nmetro);
@@ -141,8 +149,8 @@ cudaError_t batch_launch_finalize(const BatchLaunch& b, cudaStream_t st, int nsl
 cudaError_t batch_launch_samples(const BatchLaunch& b, cudaStream_t st, int nslots, int e0, int n_total,
                                  double* samples);
 // replica exchange of the step's disjoint pairs ([npairs][2] member ids) from
-// the energies of the EMCS just done; perm/flags as batch_temper describes
-cudaError_t batch_launch_temper(const BatchLaunch& b, cudaStream_t st, const int32_t* pairs, int npairs, uint32_t step,
+// the energies in measurement slot `slot`; perm/flags as batch_temper describes
+cudaError_t batch_launch_temper(const BatchLaunch& b, cudaStream_t st, int slot, const int32_t* pairs, int npairs, uint32_t step,
                                 uint64_t seed, double en_min, double en_max, int32_t* perm, int32_t* flags);
 // kernel launches of one EMCS (the counter tick of a graph apart)
 inline uint64_t batch_launches_per_emcs(const BatchLaunch& b, int ncluster, int nmetro)

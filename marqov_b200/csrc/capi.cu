@@ -15,6 +15,7 @@
 
 #include "batch.h"
 #include "engine.h"
+#include "resident.h"
 
 namespace mqv {
 
@@ -303,6 +304,7 @@ static mqv_status lower_stencil_bonds(Sim* s, const int8_t* bonds)
 {
     const int64_t n = s->n;
     const int dim = s->dim, deg = 2 * dim;
+    s->bonds_unit = true;
     std::vector<int8_t> fb((size_t)dim * (size_t)n);
     for (int64_t i = 0; i < n; ++i)
         for (int d = 0; d < dim; ++d) {
@@ -311,6 +313,7 @@ static mqv_status lower_stencil_bonds(Sim* s, const int8_t* bonds)
             if (bonds[(size_t)j * deg + 2 * d + 1] != w)
                 return fail(MQV_ERR_BAD_DESCRIPTOR, "hypercubic bonds are not symmetric at site " + std::to_string(i));
             fb[(size_t)d * n + i] = w;
+            s->bonds_unit &= w == 1 || w == -1;
         }
     MQV_CK(cudaMalloc(&s->d_bonds, fb.size()));
     MQV_CK(upload_sync(s->stream, s->d_bonds, fb.data(), fb.size()));
@@ -370,14 +373,16 @@ static mqv_status launch_sweep(Sim* s, int slot)
 }
 // Clusters by labelling (a fixed number of whole-lattice passes) or by one
 // CTA's breadth-first growth (one barrier per level of the cluster's depth):
-// MQV_WOLFF_AUTO labels int8 lattices of at least kLabelMinSites sites, where
+// MQV_WOLFF_AUTO labels int8 lattices of at least kLabelMinSites sites (2D and
+// 3D ones, labelled in bit tiles, from kLabelMinTiled: 27 against 600 us for a
+// critical cluster at 2D L = 256, 35 against 55 at 3D L = 32), where
 // critical clusters are thousands of levels deep; both give the same cluster.
-constexpr int64_t kLabelMinSites = (int64_t)1 << 18;
+constexpr int64_t kLabelMinSites = (int64_t)1 << 18, kLabelMinTiled = 32768;
 static bool cluster_by_label(const Sim* s)
 {
     if (s->wolff_algo == MQV_WOLFF_LABEL) return true;
     if (s->wolff_algo == MQV_WOLFF_BFS) return false;
-    return !s->is_f32 && s->n >= kLabelMinSites;
+    return !s->is_f32 && s->n >= (label_in_tiles(s) ? kLabelMinTiled : kLabelMinSites);
 }
 
 static mqv_status launch_cluster(Sim* s, int slot)
@@ -410,11 +415,20 @@ static mqv_status check_wolff_supported(Sim* s)
 // at L = 128: 176 against 335 us per EMCS); above it the launches, which
 // spread a sweep over every SM, win (L = 256: 678 against 646 us).
 constexpr int64_t kResidentAutoSites = 16384;
-// EMCS of this handle run on the resident path (smem_emcs.cu)?
-static bool use_resident(const Sim* s)
+// Ising-type lattices are held as bit planes (bits_emcs.cu) up to this many
+// sites.  Per EMCS of one cluster and one sweep, beside the launches (us): 2D
+// L = 64 13 against 127 (the per-site resident kernel: 24.6), L = 128 31
+// against 310, L = 160 52 against 50 by labelling; 3D L = 32 62 against 45;
+// sweep and measurement alone at 3D L = 32: 6.8 against 12.5.  In a batch the
+// launches of members without clusters (spin glasses) lose up to the size that
+// fits (32 x L = 32: 9 against 42 us per EMCS).
+constexpr int64_t kBitsAutoSites = 32768;
+// EMCS of this handle run on the resident path (smem_emcs.cu, bits_emcs.cu)?
+static bool use_resident(const Sim* s, int ncluster)
 {
-    if ((s->flags & MQV_FLAG_NO_RESIDENT) || !resident_fits(s)) return false;
-    return (s->flags & MQV_FLAG_RESIDENT) || s->n <= kResidentAutoSites;
+    if ((s->flags & MQV_FLAG_NO_RESIDENT) || s->n > kResidentMaxSites) return false;
+    if (s->n <= kBitsAutoSites && bits_fits(s, ncluster > 0)) return true;
+    return resident_fits(s) && ((s->flags & MQV_FLAG_RESIDENT) || s->n <= kResidentAutoSites);
 }
 // ... or on a thread-block cluster (cluster_emcs.cu), for int8 stencils of
 // 65,537 .. 262,144 sites the device can co-schedule (when asked for)
@@ -764,7 +778,7 @@ MQV_API mqv_status mqv_wolff(mqv_sim* h, int32_t nclusters, int32_t* sizes)
         const int chunk = std::min(nclusters - done, 65536);
         st = ensure_cslots(s, chunk);
         if (st) return st;
-        if (use_resident(s)) {
+        if (use_resident(s, 1)) {
             MQV_CK(launch_emcs_resident(s, chunk, 1, 0, false, nullptr, s->d_csize));
         } else if (use_cluster(s)) {
             MQV_CK(launch_emcs_cluster(s, chunk, 1, 0, nullptr, s->d_csize));
@@ -844,7 +858,7 @@ MQV_API mqv_status mqv_emcs(mqv_sim* h, int32_t n_emcs, int32_t ncluster, int32_
             if (st) return st;
         }
         MQV_CK(cudaMemsetAsync(s->d_acc, 0, sizeof(long long) * kAccStride * (size_t)ch, s->stream));
-        if (use_resident(s)) {
+        if (use_resident(s, ncluster)) {
             MQV_CK(ensure_cuts(s));
             MQV_CK(launch_emcs_resident(s, ch, ncluster, nmetro, true, s->d_acc, s->d_csize));
         } else if (use_cluster(s)) {
@@ -914,7 +928,7 @@ MQV_API mqv_status mqv_emcs_samples(mqv_sim* h, int32_t n_emcs, int32_t ncluster
             if (st) return st;
         }
         MQV_CK(cudaMemsetAsync(s->d_acc, 0, sizeof(long long) * kAccStride * (size_t)ch, s->stream));
-        if (use_resident(s)) {
+        if (use_resident(s, ncluster)) {
             MQV_CK(ensure_cuts(s));
             MQV_CK(launch_emcs_resident(s, ch, ncluster, nmetro, true, s->d_acc, s->d_csize));
         } else if (use_cluster(s)) {
@@ -992,8 +1006,8 @@ MQV_API mqv_status mqv_describe(mqv_sim* h, char* buf, size_t len)
     // the sweep kernel's name, when there is one, ends the line
     std::snprintf(buf, len, "model=%d lattice=%s n=%lld clusters=%s path=%s%s%s", s->md.kind,
                   s->lat_kind == MQV_LATTICE_HYPERCUBIC ? (s->termsel ? "bipartite" : "hypercubic") : "csr", (long long)s->n,
-                  use_resident(s) ? "label-smem" : use_cluster(s) ? "label-dsmem" : (cluster_by_label(s) ? "label" : "bfs"),
-                  use_resident(s) ? "resident-smem"
+                  use_resident(s, 0) ? "label-smem" : use_cluster(s) ? "label-dsmem" : (cluster_by_label(s) ? "label" : "bfs"),
+                  use_resident(s, 0) ? "resident-smem"
                   : use_cluster(s) ? "resident-cluster"
                                    : (s->fused_ising2d ? "fused-2d-bitsliced" : (s->is_f32 ? "per-colour-f32" : "per-colour-int8")),
                   cfg[0] ? " kernel=" : "", cfg);
@@ -1109,6 +1123,10 @@ struct Batch {
     int32_t* d_res_order = nullptr;
     int nres[2] = {0, 0};
     size_t res_smem[2] = {0, 0};  // dynamic shared memory of each class (its largest layout)
+    // Ising-type members held as bit planes (batch_bits): nbits of them at
+    // d_res_order + bits_off, shared memory without and with clusters
+    int nbits = 0, bits_off = 0;
+    size_t bits_smem[2] = {0, 0};
     // members held by thread-block clusters of c CTAs (c = 2 .. 8): ncl[c]
     // of them at d_res_order + cl_off[c]
     int ncl[9] = {};
@@ -1150,7 +1168,7 @@ struct Batch {
     // run on side streams beside the graph members on `stream`: forked from
     // it by fork_ev, joined back by join_ev[i] before anything that reads
     // every member (exchanges, the chunk's reductions and copies).
-    static constexpr int kSide = 9;  // 2 resident classes + cluster sizes 2 .. 8
+    static constexpr int kSide = 10;  // bit planes, 2 resident classes, cluster sizes 2 .. 8
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[kSide] = {};
 };
@@ -1268,13 +1286,17 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         if (s->failed) return check_runnable(s);
         if (!b->f32) MQV_CK(ensure_cuts(s));
         if (ncluster > 0) {
-            mqv_status st = check_wolff_supported(s);
-            if (st) return st;
-            st = ensure_wolff(s);
+            const mqv_status st = check_wolff_supported(s);
             if (st) return st;
         }
     }
-    if (ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile)
+    if (ncluster > 0)
+        for (int i = 0; i < b->nrep; ++i) {
+            if (b->resident[(size_t)i]) continue;
+            const mqv_status st = ensure_wolff(b->sims[(size_t)i]);
+            if (st) return st;
+        }
+    if (ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile)  // graph members
         MQV_CK(cudaMalloc(&b->d_tile, b->tile_bytes));
     // member table at the start of the run
     b->reps.assign((size_t)b->nrep, BatchRep{});
@@ -1298,8 +1320,8 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         r.D = s->max_degree;
         r.resident = b->resident[(size_t)i] ? 1 : 0;
         if (b->d_tile && !b->resident[(size_t)i]) {
-            const TileShape ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile_units);
-            if (ts.n) tile_bind(r, ts, b->L.tile_units, (char*)b->d_tile + b->tile_off[(size_t)i]);
+            const TileShape ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile.units);
+            if (ts.n) tile_bind(r, ts, b->L.tile.units, (char*)b->d_tile + b->tile_off[(size_t)i]);
         }
     }
     MQV_CK(cudaMemcpyAsync(b->d_reps, b->reps.data(), sizeof(BatchRep) * b->reps.size(), cudaMemcpyHostToDevice,
@@ -1312,18 +1334,21 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     if (st) return st;
     if (b->d_acc != acc0 || b->d_csize != csize0) free_graphs(b);  // graphs hold the old pointers
     const int K = std::max(1, std::min(b->graph_steps, CH));
-    // the cost of breadth-first growth follows the clusters: while the choice
-    // is by timing, chunks are short enough to follow it too
-    const int max_chunk = b->wolff_mode == MQV_WOLFF_AUTO && ncluster > 0 ? 64 : CH;
-    // Cluster algorithm: fixed, or (MQV_WOLFF_AUTO) chosen by measurement.
+    // Cluster algorithm of the graph members: fixed, or (MQV_WOLFF_AUTO) chosen
+    // by measurement.
     // Both give the same clusters, so switching never changes the chain; the
     // cost of breadth-first growth follows the clusters (it rises as a farm
     // orders), labelling costs the same every EMCS.  Each chunk is timed; the
     // algorithm not in use is tried on a few EMCS at the start of a chunk when
     // it has no estimate or its estimate is old (256 EMCS, scaled by how
-    // much slower it was), and the faster estimate is used after that.
-    const bool adapt = b->wolff_mode == MQV_WOLFF_AUTO && ncluster > 0;
+    // much slower it was), and the faster estimate is used after that.  Chunks
+    // are short while the choice is by timing: a hot start's clusters, and with
+    // them the cost of growing them, change within a few dozen EMCS.
+    bool graph = false;  // members on the graph path
+    for (char r : b->resident) graph |= r == 0;
+    const bool adapt = b->wolff_mode == MQV_WOLFF_AUTO && ncluster > 0 && graph;
     const int fixed = b->wolff_mode == MQV_WOLFF_LABEL ? 1 : 0;
+    const int max_chunk = adapt ? 64 : CH;
     if (b->g_ncluster != ncluster || b->g_nmetro != nmetro || b->g_steps != K) {
         free_graphs(b);
         b->g_ncluster = ncluster;
@@ -1331,7 +1356,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         b->g_steps = K;
     }
     for (int w = 0; w < 2; ++w) {
-        if (!adapt && w != fixed) continue;
+        if (!graph || (!adapt && w != fixed)) continue;
         if (b->g_one[w] && (K == 1 || b->g_many[w])) continue;
         MQV_CK(cudaStreamSynchronize(b->stream));
         b->L.wolff_ccl = w;
@@ -1358,9 +1383,10 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         per_emcs[w] = batch_launches_per_emcs(l, ncluster, nmetro);
     }
     // side streams of the resident classes and cluster sizes (created once)
-    int nside_needed = (b->nres[0] ? 1 : 0) + (b->nres[1] ? 1 : 0);
+    int nside_needed = (b->nres[0] ? 1 : 0) + (b->nres[1] ? 1 : 0) + (b->nbits ? 1 : 0);
     for (int c = 2; c <= 8; ++c) nside_needed += b->ncl[c] ? 1 : 0;
-    if (nside_needed && !b->fork_ev) {
+    const bool inline_bits = b->nbits == b->nrep;  // nothing to run beside them
+    if (nside_needed && !inline_bits && !b->fork_ev) {
         MQV_CK(cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming));
         for (int i = 0; i < Batch::kSide; ++i) {
             MQV_CK(cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking));
@@ -1372,6 +1398,12 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     // members (algorithm w) on the batch stream, joined at the end
     auto launch_emcs = [&](int w, int count, int k0) -> mqv_status {
         int nside = 0;
+        if (inline_bits) {
+            MQV_CK(batch_launch_bits(b->L, b->stream, b->d_res_order + b->bits_off, b->nbits, b->bits_smem[ncluster > 0],
+                                     (uint32_t)(done_run + k0), k0, count, ncluster, nmetro, b->device));
+            b->launches++;
+            return MQV_OK;
+        }
         if (nside_needed) MQV_CK(cudaEventRecord(b->fork_ev, b->stream));
         // the next side stream, ordered after the fork
         auto side_stream = [&](cudaStream_t& st2) -> cudaError_t {
@@ -1393,6 +1425,14 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
             MQV_CK(side_done(st2));
             b->launches++;
         }
+        if (b->nbits) {
+            cudaStream_t st2 = nullptr;
+            MQV_CK(side_stream(st2));
+            MQV_CK(batch_launch_bits(b->L, st2, b->d_res_order + b->bits_off, b->nbits, b->bits_smem[ncluster > 0],
+                                     (uint32_t)(done_run + k0), k0, count, ncluster, nmetro, b->device));
+            MQV_CK(side_done(st2));
+            b->launches++;
+        }
         for (int c = 2; c <= 8; ++c) {
             if (!b->ncl[c]) continue;
             cudaStream_t st2 = nullptr;
@@ -1402,11 +1442,13 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
             MQV_CK(side_done(st2));
             b->launches++;
         }
-        int j = 0;
-        if (K > 1)
-            for (; j + K <= count; j += K) MQV_CK(cudaGraphLaunch(b->g_many[w], b->stream));
-        for (; j < count; ++j) MQV_CK(cudaGraphLaunch(b->g_one[w], b->stream));
-        b->launches += per_emcs[w] * (uint64_t)count + (uint64_t)(count / K) + (uint64_t)(count % K);
+        if (graph) {
+            int j = 0;
+            if (K > 1)
+                for (; j + K <= count; j += K) MQV_CK(cudaGraphLaunch(b->g_many[w], b->stream));
+            for (; j < count; ++j) MQV_CK(cudaGraphLaunch(b->g_one[w], b->stream));
+            b->launches += per_emcs[w] * (uint64_t)count + (uint64_t)(count / K) + (uint64_t)(count % K);
+        }
         for (int i = 0; i < nside; ++i) MQV_CK(cudaStreamWaitEvent(b->stream, b->join_ev[i], 0));
         return MQV_OK;
     };
@@ -1414,7 +1456,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     auto exchange_after = [&](int e) -> mqv_status {
         if (!pt || e % pt->interval != 0) return MQV_OK;
         const int t = e / pt->interval - 1;
-        MQV_CK(batch_launch_temper(b->L, b->stream, pt->d_plan + (size_t)2 * pt->npairs * t, pt->npairs,
+        MQV_CK(batch_launch_temper(b->L, b->stream, e - 1 - done_run, pt->d_plan + (size_t)2 * pt->npairs * t, pt->npairs,
                                    pt->step0 + (uint32_t)t, pt->seed, kTemperEnMin, kTemperEnMax, pt->d_perm,
                                    pt->d_flags + (size_t)pt->npairs * t));
         b->launches++;
@@ -1597,11 +1639,19 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     // resident members: int8 stencil lattices that fit one CTA's shared
     // memory (or a thread-block cluster's) and whose spec asks for it
     b->resident.assign((size_t)n, 0);
-    std::vector<int32_t> res_order[2], cl_order[9];
-    bool cl_ok[9] = {};
-    for (int c = 2; c <= 8; ++c) cl_ok[c] = cluster_launchable(c);
+    std::vector<int32_t> res_order[2], cl_order[9], bits_order;
+    bool cl_ok[9] = {}, cl_asked = false;
     for (int r = 0; r < n; ++r) {
         const Sim* s = b->sims[(size_t)r];
+        // Ising-type members as bit planes: one SM then advances a lattice
+        // faster than its share of the launches of the graph path
+        if (!(specs[r].params.flags & MQV_FLAG_NO_RESIDENT) &&
+            s->n <= (s->md.kind == MQV_MODEL_EA ? kResidentMaxSites : kBitsAutoSites) && bits_fits(s, s->md.kind != MQV_MODEL_EA)) {
+            b->resident[(size_t)r] = 3;
+            bits_order.push_back(r);
+            for (int c = 0; c < 2; ++c) b->bits_smem[c] = std::max(b->bits_smem[c], bits_smem(s, c && s->md.kind != MQV_MODEL_EA));
+            continue;
+        }
         // A resident member runs on one CTA (or one cluster) for a whole chunk
         // of EMCS, which leaves it at the speed of one SM (or a few): the
         // graph path, whose launches spread every member over all SMs, is the
@@ -1613,6 +1663,9 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
             res_order[s->n > kResSmall ? 1 : 0].push_back(r);
         } else if (!s->is_f32 && s->lat_kind == MQV_LATTICE_HYPERCUBIC) {
             const int c = cluster_ctas(s->n);
+            if (!cl_asked)
+                for (int k = 2; k <= 8; ++k) cl_ok[k] = cluster_launchable(k);
+            cl_asked = true;
             if (c >= 2 && cl_ok[c]) {
                 b->resident[(size_t)r] = 2;
                 cl_order[c].push_back(r);
@@ -1634,6 +1687,11 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         b->ncl[c] = (int)cl_order[c].size();
         res_all.insert(res_all.end(), cl_order[c].begin(), cl_order[c].end());
     }
+    std::stable_sort(bits_order.begin(), bits_order.end(),
+                     [&](int32_t x, int32_t y) { return b->sims[(size_t)x]->n > b->sims[(size_t)y]->n; });
+    b->nbits = (int)bits_order.size();
+    b->bits_off = (int)res_all.size();
+    res_all.insert(res_all.end(), bits_order.begin(), bits_order.end());
     // per-colour work: colour c concatenates every graph member's colour-c
     // sites (resident members contribute none), each member's count padded
     // to whole blocks of kAccSites, so that a CTA's block lies in one member
@@ -1678,19 +1736,19 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         const Sim* s = b->sims[(size_t)r];
         if (!b->resident[(size_t)r] && tile_shape(s->lat_kind, s->dim, s->len, 64).n) units += tile_lattice_units(s->dim, s->len);
     }
-    b->L.tile_units = tile_units(units);
+    b->L.tile = tile_config(units);
     std::vector<int32_t> tprefix((size_t)n + 1, 0), trep;
     std::vector<int64_t> sprefix((size_t)n + 1, 0);
     b->tile_off.assign((size_t)n, 0);
     for (int r = 0; r < n; ++r) {
         const Sim* s = b->sims[(size_t)r];
         TileShape ts;
-        if (!b->resident[(size_t)r]) ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile_units);
+        if (!b->resident[(size_t)r]) ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile.units);
         if ((int64_t)tprefix[(size_t)r] + ts.n >= (int64_t)1 << 31) return bail(fail(MQV_ERR_INVALID_ARG, "batch too large"));
         tprefix[(size_t)r + 1] = tprefix[(size_t)r] + ts.n;
         trep.insert(trep.end(), (size_t)ts.n, (int32_t)r);
         b->tile_off[(size_t)r] = b->tile_bytes;
-        b->tile_bytes += (ts.bytes(b->L.tile_units) + 255) / 256 * 256;
+        b->tile_bytes += (ts.bytes(b->L.tile.units) + 255) / 256 * 256;
         sprefix[r + 1] = sprefix[r] + (b->resident[(size_t)r] || ts.n ? 0 : s->n);
     }
     b->L.tiles = (int)trep.size();

@@ -57,6 +57,39 @@ MQV_HD uint4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, Key k)
     return make_uint4(c0, c1, c2, c3);
 }
 
+#ifdef __CUDACC__
+// The round keys of a Philox key, held in registers: a loop that draws many
+// blocks with one key then pays two multiplications and two three-way
+// exclusive ors per round and nothing for the key schedule.
+struct RoundKeys {
+    uint32_t a[10], b[10];
+    __device__ __forceinline__ explicit RoundKeys(Key k)
+    {
+#pragma unroll
+        for (int r = 0; r < 10; ++r) {
+            a[r] = k.k0 + (uint32_t)r * 0x9E3779B9u;
+            b[r] = k.k1 + (uint32_t)r * 0xBB67AE85u;
+            asm volatile("" : "+r"(a[r]), "+r"(b[r]));  // not recomputed where they are used
+        }
+    }
+};
+__device__ __forceinline__ uint4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, const RoundKeys& k)
+{
+#pragma unroll
+    for (int r = 0; r < 10; ++r) {
+        uint32_t hi0, lo0, hi1, lo1;
+        mulhilo(0xD2511F53u, c0, hi0, lo0);
+        mulhilo(0xCD9E8D57u, c2, hi1, lo1);
+        const uint32_t n0 = hi1 ^ c1 ^ k.a[r], n2 = hi0 ^ c3 ^ k.b[r];
+        c0 = n0;
+        c1 = lo1;
+        c2 = n2;
+        c3 = lo0;
+    }
+    return make_uint4(c0, c1, c2, c3);
+}
+#endif
+
 MQV_HD uint64_t lo64(uint4 v) { return (uint64_t)v.x | ((uint64_t)v.y << 32); }
 MQV_HD uint64_t hi64(uint4 v) { return (uint64_t)v.z | ((uint64_t)v.w << 32); }
 
@@ -288,7 +321,8 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 
 #ifdef __CUDACC__
 template <class... P, class... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A&&... args)
+inline cudaError_t launch_pdl_smem(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                                   cudaStream_t stream, A&&... args)
 {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -296,10 +330,16 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned thre
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A&&... args)
+{
+    return launch_pdl_smem(kernel, grid, threads, 0, stream, static_cast<A&&>(args)...);
 }
 #endif
 

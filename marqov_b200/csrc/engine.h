@@ -246,6 +246,7 @@ struct Sim {
     int32_t* d_rp = nullptr;
     int32_t* d_ci = nullptr;
     int8_t* d_bonds = nullptr;
+    bool bonds_unit = false;  // stencil bonds are all +-1
     int max_degree = 0;
     uint64_t lat_hash = 0;            // CSR: FNV-1a of row_ptr, col_idx and bonds
     std::vector<int32_t> colour_ptr;  // host

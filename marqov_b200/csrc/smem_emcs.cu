@@ -32,6 +32,7 @@
 
 #include "batch.h"
 #include "int8_site.cuh"
+#include "resident.h"
 #include "wolff_int8.cuh"
 
 namespace mqv {
@@ -39,22 +40,6 @@ namespace mqv {
 constexpr int kResThreads = 512;
 constexpr int kResWarps = kResThreads / 32;
 constexpr int kResBatch = 4;  // plane words a warp handles side by side
-
-struct ResidentRun {
-    ModelDev m;
-    StencilDev st;  // the lattice in its global layout (split rows or not)
-    WolffDev w;
-    Key key;
-    uint32_t replica, sweep0, cluster0;  // counters of the chunk's first EMCS
-    int n_emcs, ncluster, nmetro, D, runs;
-    const unsigned long long* cuts;
-    int8_t* state;      // global state, read at the start and written at the end
-    long long* acc;     // measurement accumulators of the first EMCS (zeroed), or NULL
-    int64_t acc_e;      // stride between EMCS (long longs)
-    int32_t* csize;     // cluster size of the first cluster
-    int64_t csize_e;    // stride between EMCS
-    int64_t csize_c;    // stride between the clusters of one EMCS
-};
 
 // Bit planes of the flood-fill cluster: rows are the x-lines of the lattice
 // (n / len of them), each padded to kRowWords(len) 32-site words.
@@ -663,27 +648,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int r = order[blockIdx.x];
-    const BatchRep& B = reps[r];
     ResidentRun R;
-    R.m = B.md;
-    R.st = B.st;
-    R.w = B.w;
-    R.key = B.key;
-    R.replica = B.replica;
-    R.sweep0 = B.sweep0 + e0 * (uint32_t)nmetro;
-    R.cluster0 = B.cluster0 + e0 * (uint32_t)ncluster;
-    R.n_emcs = count;
-    R.ncluster = ncluster;
-    R.nmetro = nmetro;
-    R.D = B.D;
-    R.runs = resident_runs(B.st.n);
-    R.cuts = B.cuts;
-    R.state = (int8_t*)B.s;
-    R.acc = acc + ((size_t)slot0 * nrep + r) * kAccStride;
-    R.acc_e = (int64_t)nrep * kAccStride;
-    R.csize = csize + (size_t)slot0 * ncluster * nrep + r;
-    R.csize_e = (int64_t)ncluster * nrep;
-    R.csize_c = nrep;
+    resident_member(R, reps[r], r, nrep, e0, slot0, count, ncluster, nmetro, acc, csize);
+    R.runs = resident_runs(R.st.n);
     resident_run(R, smem);
 }
 
@@ -712,7 +679,8 @@ static cudaError_t resident_attr(int device)
 cudaError_t launch_emcs_resident(Sim* s, int n_emcs, int ncluster, int nmetro, bool measure, long long* acc,
                                  int32_t* csize)
 {
-    cudaError_t e = resident_attr(s->device);
+    const bool bits = bits_fits(s, ncluster > 0);
+    cudaError_t e = bits ? cudaSuccess : resident_attr(s->device);
     if (e != cudaSuccess) return e;
     ResidentRun R{};
     R.m = s->md;
@@ -734,7 +702,12 @@ cudaError_t launch_emcs_resident(Sim* s, int n_emcs, int ncluster, int nmetro, b
     R.csize = csize;
     R.csize_e = ncluster;
     R.csize_c = 1;
-    emcs_resident<<<1, kResThreads, resident_smem_for(s->sten), s->stream>>>(R);
+    if (bits) {
+        e = launch_bits_emcs(R, s->d_bonds != nullptr, s->stream, s->device);
+        if (e != cudaSuccess) return e;
+    } else {
+        emcs_resident<<<1, kResThreads, resident_smem_for(s->sten), s->stream>>>(R);
+    }
     s->launches++;
     s->sweep += (uint64_t)n_emcs * (uint64_t)nmetro;
     s->cluster += (uint64_t)n_emcs * (uint64_t)ncluster;

@@ -149,6 +149,11 @@ static void launch_label_t(Sim* s, int32_t* csize)
     s->launches += 5;
 }
 
+static TileConfig single_tile_config(const Sim* s)
+{
+    return tile_config(s->lat_kind == MQV_LATTICE_HYPERCUBIC ? tile_lattice_units(s->dim, s->len) : 0);
+}
+
 // The one-member tables of the labelling path and of the cluster-resident
 // kernel, allocated on first use; `label`: with the labelling's scratch.
 cudaError_t ensure_label_tables(Sim* s, bool label)
@@ -158,7 +163,7 @@ cudaError_t ensure_label_tables(Sim* s, bool label)
     if (!s->d_rep1) e = cudaMalloc(&s->d_rep1, sizeof(BatchRep));
     if (e == cudaSuccess && !s->d_ctr1) e = cudaMalloc(&s->d_ctr1, sizeof(BatchCtr));
     if (e == cudaSuccess && !s->d_seed1) e = cudaMalloc(&s->d_seed1, sizeof(CclSeed));
-    const int units = tile_units(s->lat_kind == MQV_LATTICE_HYPERCUBIC ? tile_lattice_units(s->dim, s->len) : 0);
+    const int units = single_tile_config(s).units;
     const TileShape ts = tile_shape(s->lat_kind, s->dim, s->len, units);
     if (label && ts.n && e == cudaSuccess && !s->d_tile) {
         // tables: the tiles' prefix {0, n}, every tile's member 0
@@ -219,7 +224,7 @@ cudaError_t launch_emcs_cluster(Sim* s, int n_emcs, int ncluster, int nmetro, lo
 bool label_in_tiles(const Sim* s)
 {
     return s->lat_kind == MQV_LATTICE_HYPERCUBIC &&
-           tile_shape(s->lat_kind, s->dim, s->len, tile_units(tile_lattice_units(s->dim, s->len))).n > 0;
+           tile_shape(s->lat_kind, s->dim, s->len, single_tile_config(s).units).n > 0;
 }
 
 cudaError_t launch_wolff_label(Sim* s, int slot)
@@ -235,7 +240,7 @@ cudaError_t launch_wolff_label(Sim* s, int slot)
         b.tile_prefix = s->d_ttab1;
         b.tile_rep = s->d_ttab1 + 2;
         b.tiles = tile_shape(s->lat_kind, s->dim, s->len, s->tile_units).n;
-        b.tile_units = s->tile_units;
+        b.tile = single_tile_config(s);
         b.ccl_seeds = s->d_seed1;
         b.ctr = s->d_ctr1;
         b.csize = s->d_csize + slot;

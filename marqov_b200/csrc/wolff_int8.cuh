@@ -39,8 +39,9 @@ __device__ __forceinline__ uint32_t uf_prio(uint32_t i) { return i * 0x9E3779B1u
 __device__ __forceinline__ uint32_t uf_prio16(uint32_t i) { return (i * 0x9E37u) & 0xFFFFu; }
 
 // Bond activation of the int8 rules on the bond's keyed word
+template <class K>  // Key or RoundKeys
 __device__ __forceinline__ bool wolff_int8_active(const WolffDev& w, uint32_t a, uint32_t b, uint32_t serial,
-                                                  uint32_t tg_bond, Key key)
+                                                  uint32_t tg_bond, const K& key)
 {
     const uint32_t lo = a < b ? a : b, hi = a < b ? b : a;
     const unsigned long long u53 = lo64(philox(lo, serial, hi, tg_bond, key)) >> 11;

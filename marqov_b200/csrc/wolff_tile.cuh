@@ -12,8 +12,9 @@
 //               idles on a bond that needs no draw; bonds active along x
 //               join the sites of a word into runs without any union, and
 //               the active bonds between units (one per pair of runs where
-//               they are adjacent) are united by union-find on 16-bit
-//               parents in shared memory.  The tile's candidate and x-bond
+//               they are adjacent) join the runs' trees in shared memory:
+//               the first of a run by a plain store, the others in rounds of
+//               hooking and flattening.  The tile's candidate and x-bond
 //               words and its run labels go to global memory, its local
 //               roots enter the global forest;
 //   tile_hook   one thread per bond that leaves its tile, united in the
@@ -27,6 +28,7 @@
 #pragma once
 #include "batch.h"
 #include "f32_site.cuh"
+#include "runs.cuh"
 #include "wolff_int8.cuh"
 
 namespace mqv {
@@ -74,34 +76,6 @@ struct TileAt {
     }
 };
 
-// first site of the run that holds bit b (S: first sites of the runs)
-__device__ __forceinline__ int run_start(uint32_t S, int b) { return 31 - __clz(S & (0xFFFFFFFFu >> (31 - b))); }
-
-// union-find on the tile's parents: of two roots the larger id hangs below the
-// smaller by an atomic minimum, and a lost race goes on from the parent it
-// found instead of from the start
-__device__ __forceinline__ int tile_find(volatile int* p, int x)
-{
-    int px;
-    while ((px = p[x]) != x) {
-        const int gp = p[px];
-        if (gp == px) return px;
-        p[x] = gp;
-        x = gp;
-    }
-    return x;
-}
-__device__ __forceinline__ void tile_unite(int* p, int a, int b)
-{
-    a = tile_find(p, a);
-    b = tile_find(p, b);
-    while (a != b) {
-        const int lo = min(a, b), hi = max(a, b), old = atomicMin(p + hi, lo);
-        if (old == hi) return;
-        a = tile_find(p, lo);
-        b = tile_find(p, old);
-    }
-}
 // union-find on the global forest of local roots
 __device__ __forceinline__ int forest_find(int* __restrict__ p, int x)
 {
@@ -128,26 +102,18 @@ __device__ __forceinline__ void forest_unite(int* __restrict__ p, int a, int b)
     }
 }
 
-// activation of the bond (lo, hi) of a float member given both ends'
-// projections on the reflection vector
-__device__ __forceinline__ bool ccl_active_f32(const BatchRep& R, uint32_t serial, int64_t lo, int64_t hi, double alo,
-                                               double ahi)
-{
-    const double cpl = embed_cpl(R.md.J, alo, ahi);
-    return cpl > 0 && !update_accepted(2, cpl, R.md.beta,
-                                       lo64(philox((uint32_t)lo, serial, (uint32_t)hi, tag(kWolffBond, R.replica), R.key)));
-}
 // activation of the bond between candidates i and j
-template <bool F32>
-__device__ __forceinline__ bool tile_active(const BatchRep& R, const WolffDev& w, Key key, uint32_t tgb,
+template <bool F32, class K>
+__device__ __forceinline__ bool tile_active(const BatchRep& R, const WolffDev& w, const K& key, uint32_t tgb,
                                             const float r[3], uint32_t serial, uint32_t i, uint32_t j)
 {
     if (F32) {
         const float* s = (const float*)R.s;
         const int64_t n = R.st.n;
         const uint32_t lo = i < j ? i : j, hi = i < j ? j : i;
-        return ccl_active_f32(R, serial, lo, hi, embed_proj(R.md.symd, s, n, lo, r[0], r[1], r[2]),
-                              embed_proj(R.md.symd, s, n, hi, r[0], r[1], r[2]));
+        const double cpl = embed_cpl(R.md.J, embed_proj(R.md.symd, s, n, lo, r[0], r[1], r[2]),
+                                     embed_proj(R.md.symd, s, n, hi, r[0], r[1], r[2]));
+        return cpl > 0 && !update_accepted(2, cpl, R.md.beta, lo64(philox(lo, serial, hi, tgb, key)));
     }
     return wolff_int8_active(w, i, j, serial, tgb, key);
 }
@@ -175,47 +141,30 @@ __device__ __forceinline__ size_t cluster_slot(const BatchCtr* ctr, const Cluste
     return ((size_t)slot * k.ncluster + k.c) * nrep + r;
 }
 
-// (L = 4096, 16.8 M sites at the critical point: 176 us, against 415 for the
-// site-by-site kernel in 16 x 16 tiles; L = 1024: 25 against 31 us, with 10
-// against 24 us in each of the two launches after it.)
 // LPU lanes share a unit: lane l of a warp works on bits [32 / LPU * (l % LPU),
-// ...) of unit l / LPU of the warp's 32 / LPU units, so that a lane's serial
-// steps over bonds and runs shrink with LPU (latency, on lattices that leave
-// the chip half empty) where LPU = 1 keeps the lanes evenest (throughput).
+// ...) of unit l / LPU of the warp's 32 / LPU units, so that the steps over the
+// bits of a unit shrink with LPU (latency, on lattices that leave the chip
+// half empty) where LPU = 1 pays the per-warp steps once per 32 units
+// (throughput).
 template <bool F32, int U, int LPU>
 __global__ void __launch_bounds__(U * LPU, 1280 / (U * LPU))
     tile_label(const BatchRep* __restrict__ reps, const int32_t* __restrict__ tile_prefix,
                const int32_t* __restrict__ tile_rep, CclSeed* __restrict__ seeds, const BatchCtr* __restrict__ ctr,
                ClusterStep step, int32_t* __restrict__ csize, int nrep)
 {
-    constexpr int NT = U * LPU, UW = 32 / LPU, BITS = 32 / LPU;
-    __shared__ __align__(16) int P[U * 32];
-    __shared__ unsigned short lists[U * 32];  // a list of bonds per warp
+    constexpr int NT = U * LPU, UW = 32 / LPU, BITS = 32 / LPU, NW = NT / 32;
+    constexpr int DIRS = U == 64 ? 3 : 1;          // directions in one bond list
+    constexpr int LIST = UW * 32 * DIRS;           // bond list entries of a warp
+    constexpr int EDGES = U * 16;                  // edges between runs (the rest is found again in the planes)
+    constexpr int RES = LIST / 32 + 3;             // outcome words of a warp's list
+    constexpr int PN = U * 32 > NW * RES ? U * 32 : NW * RES;
+    __shared__ __align__(16) int P[PN];            // parents of the runs (before: the outcomes)
+    __shared__ uint32_t edge[NW * LIST / 2 > EDGES ? NW * LIST / 2 : EDGES];  // edges (before: the bond lists)
     __shared__ uint32_t sC[U], sB[3][U], sS[U];
+    __shared__ int sR[U], s_warp[NW], s_nedge;
     __shared__ CclSeed s_seed;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int u = tid / LPU;  // this lane's unit
-    unsigned short* list = lists + warp * (UW * 32);
-    // the bonds Q of the warp's units (this lane's part of its unit), listed
-    auto list_bonds = [&](uint32_t Q) -> int {
-        const int cnt = __popc(Q);
-        int pos = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, pos, o);
-            if (lane >= o) pos += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, pos, 31);
-        pos -= cnt;
-        __syncwarp();  // the list's last readers are done
-        while (Q) {
-            const int b = __ffs(Q) - 1;
-            Q &= Q - 1;
-            list[pos++] = (unsigned short)(((lane / LPU) << 5) | b);
-        }
-        __syncwarp();
-        return total;
-    };
     const uint32_t part = (LPU == 1 ? 0xFFFFFFFFu : (1u << (BITS & 31)) - 1u) << (BITS * (tid % LPU));
     grid_dep_launch();
     grid_dep_wait();
@@ -224,22 +173,21 @@ __global__ void __launch_bounds__(U * LPU, 1280 / (U * LPU))
     const uint32_t serial = cluster_serial(R, ctr, step);
     const TileAt<U> at(R, t);
     const int dim = R.st.dim, L = at.L;
-    const int row = at.row(u), xb = at.tx * 32;
-    int* forest = R.tl_forest;
-    uint32_t *gcand = R.tl_cand + (int64_t)t * U, *gxb = R.tl_xb + (int64_t)t * U;
-    uint4* lab = reinterpret_cast<uint4*>(R.tl_lab + (int64_t)t * (U * 32));
+    const int row = at.row(u), xb = at.tx * 32, base = t * (U * 32);
+    int* forest = R.tl_forest + base;
+    unsigned short* lab = R.tl_lab + base;
+    uint32_t *gcand = R.tl_cand + (int64_t)t * U, *gxb = R.tl_xb + (int64_t)t * U, *gbase = R.tl_base + (int64_t)t * U;
     if (tid == 0) {
         CclSeed sd{};
         tile_seed<F32>(R, serial, sd);
         s_seed = sd;
+        s_nedge = 0;
         if (t == 0) {
             seeds[r] = sd;
             csize[cluster_slot(ctr, step, nrep, r)] = 0;
         }
     }
     if (tid < U) sB[0][tid] = sB[1][tid] = sB[2][tid] = 0u;
-#pragma unroll
-    for (int k = 0; k < 32 / LPU; ++k) P[k * NT + tid] = k * NT + tid;
     __syncthreads();
     const float rv[3] = {s_seed.r[0], s_seed.r[1], s_seed.r[2]};
     // candidates: the warp's lanes read the 32 sites of one unit after the other
@@ -279,87 +227,147 @@ __global__ void __launch_bounds__(U * LPU, 1280 / (U * LPU))
     }
     __syncthreads();
     const uint32_t C = sC[u];
-    // the active bonds inside the tile, drawn from the warp's list of bonds
-    // between two candidates
+    const int uy = at.uy(u), uz = at.uz(u);
+    // The active bonds inside the tile: the bonds between two candidates are
+    // listed per warp and drawn side by side over the lanes; the outcomes come
+    // back as a bit string in the list's order.
     {
         const WolffDev w = R.w;
-        const Key key = R.key;
+        const RoundKeys key(R.key);
         const uint32_t tgb = tag(kWolffBond, R.replica);
-        for (int d = 0; d < dim; ++d) {
-            uint32_t Q, step_j;
-            if (d == 0) {
-                Q = C & (C >> 1);
-                step_j = 1u;
-            } else if (d == 1) {
-                Q = at.uy(u) < at.TY - 1 ? C & sC[u + 1] : 0u;
-                step_j = (uint32_t)L;
-            } else {
-                Q = at.uz(u) < at.TZ - 1 ? C & sC[u + at.TY] : 0u;
-                step_j = (uint32_t)L * (uint32_t)L;
+        unsigned short* list = reinterpret_cast<unsigned short*>(edge) + warp * LIST;
+        uint32_t* res = reinterpret_cast<uint32_t*>(P) + warp * RES;
+        const int first_site = row * L + xb;
+        for (int d0 = 0; d0 < dim; d0 += DIRS) {
+            uint32_t Q[3] = {0u, 0u, 0u};
+            if (d0 == 0) Q[0] = C & (C >> 1) & part;
+            if (DIRS == 3 || d0 == 1) Q[1] = uy < at.TY - 1 ? C & sC[u + 1] & part : 0u;
+            if ((DIRS == 3 || d0 == 2) && dim == 3) Q[2] = uz < at.TZ - 1 ? C & sC[u + at.TY] & part : 0u;
+            const int cnt = __popc(Q[0]) + __popc(Q[1]) + __popc(Q[2]);
+            int pos = warp_prefix(cnt, lane);
+            const int total = __shfl_sync(0xffffffffu, pos, 31), from = pos -= cnt;
+            __syncwarp();  // the list's last readers are done
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                for (uint32_t m = Q[d]; m; m &= m - 1)
+                    list[pos++] = (unsigned short)((d << 10) | ((lane / LPU) << 5) | (__ffs(m) - 1));
+            __syncwarp();
+            for (int k0 = 0; k0 < total; k0 += 64) {
+                uint32_t i[2], j[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = k0 + 32 * h + lane;
+                    const uint32_t id = list[k < total ? k : 0];
+                    i[h] = (uint32_t)__shfl_sync(0xffffffffu, first_site, ((id >> 5) & 31u) * LPU) + (id & 31u);
+                    const uint32_t d = id >> 10;
+                    j[h] = i[h] + (d == 0 ? 1u : d == 1 ? (uint32_t)L : (uint32_t)L * (uint32_t)L);
+                }
+                const bool a0 = tile_active<F32>(R, w, key, tgb, rv, serial, i[0], j[0]);
+                const bool a1 = tile_active<F32>(R, w, key, tgb, rv, serial, i[1], j[1]);
+                const uint32_t r0 = __ballot_sync(0xffffffffu, a0), r1 = __ballot_sync(0xffffffffu, a1);
+                if (lane == 0) {
+                    res[k0 >> 5] = r0;
+                    res[(k0 >> 5) + 1] = r1;
+                }
             }
-            const int total = list_bonds(Q & part);
-            for (int k0 = 0; k0 < total; k0 += 32) {
-                const int k = k0 + lane;
-                const uint32_t id = list[k < total ? k : 0];
-                const int rk = __shfl_sync(0xffffffffu, row, (id >> 5) * LPU);
-                const uint32_t i = (uint32_t)rk * (uint32_t)L + (uint32_t)xb + (id & 31u);
-                if (k < total && tile_active<F32>(R, w, key, tgb, rv, serial, i, i + step_j))
-                    atomicOr(&sB[d][warp * UW + (id >> 5)], 1u << (id & 31u));
+            __syncwarp();
+            int at_bit = from;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if (DIRS == 1 && d != d0) continue;
+                const uint32_t B = Q[d] ? bit_deposit(bit_string(res, at_bit), Q[d]) : 0u;
+                at_bit += __popc(Q[d]);
+                const uint32_t all = group_or(B, LPU);
+                if (tid % LPU == 0) sB[d][u] = all;
             }
         }
     }
+    // Runs: the bonds along x join the sites of a unit.  They are numbered
+    // through the tile (sR: first run of every unit), so that the steps below
+    // take one run or edge per thread.
     __syncthreads();
-    // runs, and one union per pair of adjacent runs that active bonds join
     const uint32_t X = sB[0][u], S = C & ~(X << 1);
     if (tid % LPU == 0) {
         sS[u] = S;
         gxb[u] = X;
     }
     __syncthreads();
-    // Along y every run first takes the run below its lowest active bond as
-    // its parent, by a plain store (parents point to smaller units, so no
-    // cycle); only its further bonds, to other runs below, need a union.
-    uint32_t more = 0u;
-    if (at.uy(u) > 0) {
-        const uint32_t Y = sB[1][u - 1], A = X << 1, E = (Y << 1) & A;
-        const uint32_t above = E | (((A + E) ^ A) & A);  // sites joined along x to a lower active bond
-        for (uint32_t m = Y & ~above & part; m; m &= m - 1) {
-            const int b = __ffs(m) - 1;
-            P[u * 32 + run_start(S, b)] = (u - 1) * 32 + run_start(sS[u - 1], b);
-        }
-        // the bond to the left joins the same two runs
-        more = Y & above & ~((Y & X & sB[0][u - 1]) << 1) & part;
-    }
-    __syncthreads();
-    for (int d = 1; d < dim; ++d) {
-        const int du = d == 1 ? -1 : at.TY;
-        if (d == 2) {
-            more = sB[2][u];
-            if (more) more &= ~((more & X & sB[0][u + du]) << 1) & part;
-        }
-        const int total = list_bonds(more);
-        for (int k = lane; k < total; k += 32) {
-            const int id = list[k], ua = warp * UW + (id >> 5), ub = ua + du, b = id & 31;
-            tile_unite(P, ua * 32 + run_start(sS[ua], b), ub * 32 + run_start(sS[ub], b));
-        }
-    }
-    __syncthreads();
-    const int base = t * (U * 32);
-    for (uint32_t m = S & part; m; m &= m - 1) {
-        // read-only walks: a parent halved here could overwrite a root written by the run's own thread
-        const int x = u * 32 + __ffs(m) - 1;
-        int root = x, px;
-        while ((px = ((volatile int*)P)[root]) != root) root = px;
-        if (root == x) forest[base + x] = base + x;
-        else P[x] = root;
-    }
-    __syncthreads();
+    {
+        const int cnt = tid < U ? __popc(sS[tid]) : 0, pos = warp_prefix(cnt, lane);
+        if (lane == 31) s_warp[warp] = pos;
+        __syncthreads();
+        int before = 0;
 #pragma unroll
-    for (int k = tid; k < U * 4; k += NT) {
-        const int4 p = reinterpret_cast<const int4*>(P)[2 * k], q = reinterpret_cast<const int4*>(P)[2 * k + 1];
-        lab[k] = make_uint4((uint32_t)(p.x | (p.y << 16)), (uint32_t)(p.z | (p.w << 16)),
-                            (uint32_t)(q.x | (q.y << 16)), (uint32_t)(q.z | (q.w << 16)));
+        for (int k = 0; k < U / 32; ++k) before += k < warp ? s_warp[k] : 0;
+        if (tid < U) {
+            sR[tid] = before + pos - cnt;
+            gbase[tid] = (uint32_t)sR[tid];
+        }
     }
+    __syncthreads();
+    const int nrun = sR[U - 1] + __popc(sS[U - 1]);
+    for (int k = tid; k < nrun; k += NT) P[k] = k;
+    __syncthreads();
+    auto run_of = [&](int v, int b) { return sR[v] + __popc(sS[v] & (0xFFFFFFFFu >> (31 - b))) - 1; };
+    // Along y every run first takes the run below its lowest active bond as
+    // its parent, by a plain store; the further bonds between runs, one per
+    // pair where they are adjacent, are the edges left, listed.
+    auto edges_z = [&](int v, uint32_t Xv) -> uint32_t {
+        const uint32_t Z = sB[2][v];
+        return Z ? Z & ~((Z & Xv & sB[0][v + at.TY]) << 1) : 0u;
+    };
+    {
+        uint32_t ey = 0u, ez = 0u;
+        if (uy > 0) {
+            const uint32_t Y = sB[1][u - 1], above = run_above(Y, X);
+            for (uint32_t m = Y & ~above & part; m; m &= m - 1) {
+                const int b = __ffs(m) - 1;
+                P[run_of(u, b)] = run_of(u - 1, b);
+            }
+            ey = Y & above & ~((Y & X & sB[0][u - 1]) << 1) & part;
+        }
+        if (dim == 3) ez = edges_z(u, X) & part;
+        const int cnt = __popc(ey) + __popc(ez), pos = warp_prefix(cnt, lane);
+        int slot = 0;
+        if (lane == 31 && pos) slot = atomicAdd(&s_nedge, pos);
+        slot = __shfl_sync(0xffffffffu, slot, 31) + pos - cnt;
+        for (; ey; ey &= ey - 1, ++slot)
+            if (slot < EDGES) edge[slot] = (uint32_t)run_of(u, __ffs(ey) - 1) | ((uint32_t)run_of(u - 1, __ffs(ey) - 1) << 16);
+        for (; ez; ez &= ez - 1, ++slot)
+            if (slot < EDGES)
+                edge[slot] = (uint32_t)run_of(u, __ffs(ez) - 1) | ((uint32_t)run_of(u + at.TY, __ffs(ez) - 1) << 16);
+    }
+    __syncthreads();
+    const int nedge = min(s_nedge, EDGES);
+    forest_jump(P, nrun, tid, NT);
+    __syncthreads();
+    for (int k = tid; k < nedge; k += NT) forest_join(P, (int)(edge[k] & 0xFFFFu), (int)(edge[k] >> 16));
+    if (s_nedge > EDGES && tid < U) {  // more than the list holds: once more from the planes
+        if (at.uy(tid) < at.TY - 1)
+            for (uint32_t m = sB[1][tid]; m; m &= m - 1)
+                forest_join(P, run_of(tid, __ffs(m) - 1), run_of(tid + 1, __ffs(m) - 1));
+        if (dim == 3)
+            for (uint32_t m = sB[2][tid]; m; m &= m - 1)
+                forest_join(P, run_of(tid, __ffs(m) - 1), run_of(tid + at.TY, __ffs(m) - 1));
+    }
+    __syncthreads();
+    forest_jump(P, nrun, tid, NT);
+    __syncthreads();
+    for (int k = tid; k < nrun; k += NT) {
+        const int p = P[k];
+        lab[k] = (unsigned short)p;
+        if (p == k) forest[k] = base + k;
+    }
+}
+
+// global id of the local root of candidate bit b of unit (t, u), whose words
+// are C and X
+template <int U>
+__device__ __forceinline__ int tile_root_of(const BatchRep& R, int t, int u, uint32_t C, uint32_t X, int b)
+{
+    const uint32_t S = C & ~(X << 1);
+    const int run = (int)R.tl_base[(int64_t)t * U + u] + __popc(S & (0xFFFFFFFFu >> (31 - b))) - 1;
+    return t * (U * 32) + (int)R.tl_lab[(int64_t)t * (U * 32) + run];
 }
 
 template <bool F32, int U, int LPU>
@@ -425,8 +433,8 @@ __global__ void __launch_bounds__(U * LPU)
         }
         int ra = 0, rb = 0;
         if (live) {
-            ra = t * (U * 32) + R.tl_lab[(int64_t)t * (U * 32) + u * 32 + run_start(C & ~(X << 1), b)];
-            rb = t2 * (U * 32) + R.tl_lab[(int64_t)t2 * (U * 32) + u2 * 32 + run_start(C2 & ~(X2 << 1), b2)];
+            ra = tile_root_of<U>(R, t, u, C, X, b);
+            rb = tile_root_of<U>(R, t2, u2, C2, X2, b2);
         }
         // lanes that join the same two local roots unite them once
         const unsigned long long pair =
@@ -436,15 +444,6 @@ __global__ void __launch_bounds__(U * LPU)
     }
 }
 
-// global id of the local root of candidate bit b of unit (t, u)
-template <int U>
-__device__ __forceinline__ int tile_root_of(const BatchRep& R, int t, int u, uint32_t C, int b)
-{
-    const uint32_t X = R.tl_xb[(int64_t)t * U + u];
-    const int start = run_start(C & ~(X << 1), b);
-    return t * (U * 32) + (int)R.tl_lab[(int64_t)t * (U * 32) + u * 32 + start];
-}
-
 template <bool F32, int U, int LPU>
 __global__ void __launch_bounds__(U * LPU)
     tile_flip(const BatchRep* __restrict__ reps, const int32_t* __restrict__ tile_prefix,
@@ -452,9 +451,9 @@ __global__ void __launch_bounds__(U * LPU)
               const BatchCtr* __restrict__ ctr, ClusterStep step, int32_t* __restrict__ csize, int nrep)
 {
     constexpr int NT = U * LPU, UW = 32 / LPU, BITS = 32 / LPU;
-    __shared__ __align__(16) unsigned short P[U * 32];
-    __shared__ uint32_t in[U], hit[U];
-    __shared__ int s_root, s_cnt;
+    __shared__ unsigned short lab[U * 32];
+    __shared__ uint32_t in[U + 1], hit[U + 1];  // a bit per run, in order
+    __shared__ int s_root, s_cnt, s_nrun;
     const int tid = threadIdx.x, lane = tid & 31, u = tid / LPU;
     const uint32_t part = (LPU == 1 ? 0xFFFFFFFFu : (1u << (BITS & 31)) - 1u) << (BITS * (tid % LPU));
     grid_dep_launch();
@@ -465,64 +464,50 @@ __global__ void __launch_bounds__(U * LPU)
     const TileAt<U> at(R, t);
     const int L = at.L, base = t * (U * 32);
     const uint32_t C = R.tl_cand[(int64_t)t * U + u], X = R.tl_xb[(int64_t)t * U + u], S = C & ~(X << 1);
-    const uint4* lab = reinterpret_cast<const uint4*>(R.tl_lab + base);
-#pragma unroll
-    for (int k = tid; k < U * 4; k += NT) reinterpret_cast<uint4*>(P)[k] = lab[k];
-    if (tid < U) in[tid] = hit[tid] = 0u;
+    const int run0 = (int)R.tl_base[(int64_t)t * U + u];
     const int* forest = R.tl_forest;
     auto walk = [&](int x) {
         int p;
         while ((p = __ldcg(forest + x)) != x) x = p;
         return x;
     };
-    if (tid == NT - 1) {
+    if (tid == NT - 1) {  // a lane of the tile's last unit
+        s_nrun = run0 + __popc(S);
+        s_cnt = 0;
+    }
+    __syncthreads();
+    const int nrun = s_nrun;
+    for (int k = tid; k < nrun; k += NT) lab[k] = R.tl_lab[base + k];
+    if (tid == 0) {
         // the seed's root
         const uint32_t i = (uint32_t)sd.rsite, rw = R.st.lg >= 0 ? i >> R.st.lg : R.st.divlen(i);
         const int x = (int)(i - rw * (uint32_t)L);
         const int z = at.Lz > 1 ? (int)(R.st.lg >= 0 ? rw >> R.st.lg : R.st.divlen(rw)) : 0, y = (int)rw - z * L;
         const int st = (x >> 5) + R.tl_nw * ((y >> at.lty) + R.tl_ny * (z / at.TZ)),
                   su = at.uy(y) + at.TY * (z % at.TZ);
-        s_root = walk(tile_root_of<U>(R, st, su, R.tl_cand[(int64_t)st * U + su], x & 31));
-        s_cnt = 0;
+        s_root = walk(tile_root_of<U>(R, st, su, R.tl_cand[(int64_t)st * U + su], R.tl_xb[(int64_t)st * U + su], x & 31));
     }
     __syncthreads();
     const int root = s_root;
-    // the forest above each local root of this lane's part of its unit
-    // (four first steps in flight: most local roots are roots of the forest)
-    uint32_t f = 0u, mine = 0u;
-    for (uint32_t m = S & part; m; m &= m - 1) {
-        const int b = __ffs(m) - 1;
-        if (P[u * 32 + b] == u * 32 + b) mine |= 1u << b;
+    // the forest above each local root
+    for (int k0 = tid - lane; k0 < nrun; k0 += NT) {
+        const int k = k0 + lane;
+        const uint32_t m = __ballot_sync(0xffffffffu, k < nrun && lab[k] == k && walk(base + k) == root);
+        if (lane == 0) in[k0 >> 5] = m;
     }
-    while (mine) {
-        int b[4], p[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            b[k] = __ffs(mine) - 1;
-            mine &= mine - 1;
-            p[k] = b[k] >= 0 ? __ldcg(forest + base + u * 32 + b[k]) : -1;
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (b[k] >= 0 && (p[k] == base + u * 32 + b[k] ? p[k] : walk(p[k])) == root) f |= 1u << b[k];
-    }
-    if (f) atomicOr(&in[u], f);
     __syncthreads();
-    for (uint32_t m = S & part & ~f; m; m &= m - 1) {
-        const int b = __ffs(m) - 1, l = P[u * 32 + b];
-        if ((in[l >> 5] >> (l & 31)) & 1u) f |= 1u << b;
+    // every run follows its local root
+    for (int k0 = tid - lane; k0 < nrun; k0 += NT) {
+        const int k = k0 + lane, l = k < nrun ? lab[k] : 0;
+        const uint32_t m = __ballot_sync(0xffffffffu, k < nrun && ((in[l >> 5] >> (l & 31)) & 1u));
+        if (lane == 0) hit[k0 >> 5] = m;
     }
-    if (LPU > 1) {
-        if (f) atomicOr(&hit[u], f);
-        __syncwarp();
-        f = hit[u];
-    }
-    // the runs of the marked first sites: a carry ripples up each run's bonds
-    {
-        const uint32_t A = X << 1, E = (f << 1) & A;
-        f |= E | (((A + E) ^ A) & A);
-        f &= C;
-    }
+    __syncthreads();
+    // ... and the words' sites their runs
+    const uint32_t mine = S & part;
+    uint32_t f = mine ? bit_deposit(bit_string(hit, run0 + __popc(S & (part - 1u) & ~part)), mine) : 0u;
+    f = group_or(f, LPU);
+    if (f) f = run_fill(f, X);
     const int cnt = __reduce_add_sync(0xffffffffu, tid % LPU == 0 ? __popc(f) : 0);
     if (lane == 0 && cnt) atomicAdd(&s_cnt, cnt);
     const int row = at.row(u), x = at.tx * 32 + lane;

@@ -1,6 +1,6 @@
 """Clusters labelled in bit tiles against breadth-first growth, on the GPU:
 single handles and batches, sizes below, at and beyond the tiles' edges
-(words of 32 sites, 64 and 128 rows, 8 x 8 and 8 x 16 units in 3D), the three
+(words of 32 sites, 64 and 128 rows, 8 x 8 and 8 x 16 units in 3D), the four
 launch shapes (by the number of units), int8 and float models."""
 import numpy as np
 import pytest
@@ -39,7 +39,7 @@ def test_single_handle(model, dim, L):
 
 
 @pytest.mark.parametrize("model,dim,sizes", [("ising", 2, (32, 34, 64, 128)), ("potts", 2, (64, 256, 512, 512, 512, 512)),
-                                             ("ising", 2, (1024,) * 4), ("phi4", 3, (6, 16, 20)), ("heis", 3, (40, 40, 64))])
+                                             ("ising", 2, (1024,)), ("ising", 2, (1024,) * 4), ("ising", 2, (2048, 2048)), ("phi4", 3, (6, 16, 20)), ("heis", 3, (40, 40, 64))])
 def test_batch(model, dim, sizes):
     import marqov_b200 as M
     ham, beta = models()[model]
