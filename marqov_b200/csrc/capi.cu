@@ -41,6 +41,9 @@ cudaError_t wolff_noalloc_scratch(int device, uint32_t** out);
 cudaError_t launch_wolff_int8_noalloc(Sim* s, uint32_t* scratch, int slot);
 const int32_t* wolff_noalloc_sizes(const uint32_t* scratch);
 bool label_in_tiles(const Sim* s);
+cudaError_t build_ell(Sim* s, int64_t n, const int32_t* rp, const int32_t* ci, const int8_t* bonds,
+                      const std::vector<int32_t>& col);
+cudaError_t launch_ell_emcs(Sim* s, int n_emcs, int nmetro, long long* acc);
 bool resident_fits(const Sim* s);
 cudaError_t launch_emcs_cluster(Sim* s, int n_emcs, int ncluster, int nmetro, long long* acc, int32_t* csize);
 cudaError_t launch_emcs_resident(Sim* s, int n_emcs, int ncluster, int nmetro, bool measure, long long* acc,
@@ -112,7 +115,8 @@ static void free_sim(Sim* s)
     for (void* p : {s->state[0], s->state[1], (void*)s->d_rp, (void*)s->d_ci, (void*)s->d_bonds, (void*)s->d_order,
                     (void*)s->d_acc, (void*)s->d_obs, (void*)s->d_visited, (void*)s->d_queue, (void*)s->d_csize,
                     (void*)s->d_status, (void*)s->d_counter, (void*)s->d_cuts, (void*)s->d_rep1, (void*)s->d_ctr1,
-                    s->d_seed1, (void*)s->d_sprefix1, (void*)s->d_sbrep1, (void*)s->d_ttab1, s->d_tile})
+                    s->d_seed1, (void*)s->d_sprefix1, (void*)s->d_sbrep1, (void*)s->d_ttab1, s->d_tile,
+                    s->d_ell})
         if (p) cudaFree(p);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -178,6 +182,10 @@ static mqv_status check_runnable(const Sim* s)
     if (!s->initialised) return fail(MQV_ERR_STATE, "state not initialised");
     return MQV_OK;
 }
+
+// Graphs swept by one cluster (csr_sweep.cu) up to here: above, the launches,
+// which spread a colour over every SM, win (400,000 sites: 112 against 123 us).
+constexpr int64_t kEllMaxSites = 262144;
 
 // ---- lattice lowering -----------------------------------------------------------
 
@@ -273,6 +281,9 @@ static mqv_status lower_csr(Sim* s, const mqv_lattice_desc* L)
         MQV_CK(cudaMalloc(&s->d_bonds, (size_t)std::max<int64_t>(nnz, 1)));
         MQV_CK(upload_sync(s->stream, s->d_bonds, L->bonds, (size_t)nnz));
     }
+    if (!(s->flags & MQV_FLAG_PER_COLOUR) && !s->is_f32 && s->md.kind != MQV_MODEL_POTTS &&
+        s->md.kind != MQV_MODEL_BLUME_CAPEL && n <= kEllMaxSites)
+        MQV_CK(build_ell(s, n, rp, ci, L->bonds, col));
     s->n = n;
     s->max_degree = maxdeg;
     s->csr = CSRDev{n, s->d_rp, s->d_ci, s->d_bonds};
@@ -369,6 +380,19 @@ static mqv_status launch_finalize(Sim* s, int nslots)
 static mqv_status launch_sweep(Sim* s, int slot)
 {
     MQV_CK(s->is_f32 ? launch_metropolis_f32(s, slot) : launch_metropolis_int8(s, slot));
+    return MQV_OK;
+}
+// count sweeps, the last one measured into `slot` (-1: none)
+static mqv_status launch_sweeps(Sim* s, int count, int slot)
+{
+    if (s->d_ell && count > 0) {
+        MQV_CK(launch_ell_emcs(s, 1, count, slot < 0 ? nullptr : s->d_acc + (size_t)slot * kAccStride));
+        return MQV_OK;
+    }
+    for (int j = 0; j < count; ++j) {
+        const mqv_status st = launch_sweep(s, j == count - 1 ? slot : -1);
+        if (st) return st;
+    }
     return MQV_OK;
 }
 // Clusters by labelling (a fixed number of whole-lattice passes) or by one
@@ -755,11 +779,7 @@ MQV_API mqv_status mqv_metropolis(mqv_sim* h, int32_t nsweeps)
         const mqv_status rs = check_runnable(s);
         if (rs) return rs;
     }
-    for (int t = 0; t < nsweeps; ++t) {
-        mqv_status st = launch_sweep(s, -1);
-        if (st) return st;
-    }
-    return MQV_OK;
+    return launch_sweeps(s, nsweeps, -1);
 }
 
 MQV_API mqv_status mqv_wolff(mqv_sim* h, int32_t nclusters, int32_t* sizes)
@@ -864,16 +884,16 @@ MQV_API mqv_status mqv_emcs(mqv_sim* h, int32_t n_emcs, int32_t ncluster, int32_
         } else if (use_cluster(s)) {
             MQV_CK(ensure_cuts(s));
             MQV_CK(launch_emcs_cluster(s, ch, ncluster, nmetro, s->d_acc, s->d_csize));
+        } else if (s->d_ell && ncluster == 0) {
+            MQV_CK(launch_ell_emcs(s, ch, nmetro, s->d_acc));
         } else {
             for (int e = 0; e < ch; ++e) {
                 for (int c = 0; c < ncluster; ++c) {
                     st = launch_cluster(s, e * ncluster + c);
                     if (st) return st;
                 }
-                for (int j = 0; j < nmetro; ++j) {
-                    st = launch_sweep(s, j == nmetro - 1 ? e : -1);
-                    if (st) return st;
-                }
+                st = launch_sweeps(s, nmetro, e);
+                if (st) return st;
                 if (nmetro == 0) {
                     st = launch_measure(s, e);
                     if (st) return st;
@@ -934,16 +954,16 @@ MQV_API mqv_status mqv_emcs_samples(mqv_sim* h, int32_t n_emcs, int32_t ncluster
         } else if (use_cluster(s)) {
             MQV_CK(ensure_cuts(s));
             MQV_CK(launch_emcs_cluster(s, ch, ncluster, nmetro, s->d_acc, s->d_csize));
+        } else if (s->d_ell && ncluster == 0) {
+            MQV_CK(launch_ell_emcs(s, ch, nmetro, s->d_acc));
         } else {
             for (int e = 0; e < ch; ++e) {
                 for (int c = 0; c < ncluster; ++c) {
                     st = launch_cluster(s, e * ncluster + c);
                     if (st) return st;
                 }
-                for (int j = 0; j < nmetro; ++j) {
-                    st = launch_sweep(s, j == nmetro - 1 ? e : -1);
-                    if (st) return st;
-                }
+                st = launch_sweeps(s, nmetro, e);
+                if (st) return st;
                 if (nmetro == 0) {
                     st = launch_measure(s, e);
                     if (st) return st;

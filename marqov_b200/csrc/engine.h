@@ -176,6 +176,23 @@ struct CSRDev {
     MQV_HD int bond(int64_t i, int slot) const { return bonds ? bonds[rp[i] + slot] : 1; }
 };
 
+// A coloured graph with sliced neighbour lists for the kernel of csr_sweep.cu:
+// CTA r of `ctas` owns sites [r range, (r + 1) range); its sites of colour c lie
+// at positions [cptr[r ncol + c], cptr[r ncol + c + 1]), a multiple of 32; the
+// positions of the neighbours of the site at position p are
+// nb[slice[p / 32] + p % 32 + 32 t].
+struct EllDev {
+    const int64_t* slice;
+    const int32_t* cptr;
+    const int32_t* cwords;  // 32-position words of every colour, all CTAs
+    const int32_t* site;    // -1: padding
+    const int32_t* deg;
+    const int32_t* nb;
+    const int8_t* bonds;
+    int ncol, ctas, range, npos;
+    int rounds;  // room for the rounds of a sweep
+};
+
 // Wolff activation rule of the int8 models.
 struct WolffDev {
     int mode;               // 0 Ising exact, 1 embedded (threshold rule), 2 Potts
@@ -248,6 +265,8 @@ struct Sim {
     int8_t* d_bonds = nullptr;
     bool bonds_unit = false;  // stencil bonds are all +-1
     int max_degree = 0;
+    EllDev ell{};                     // CSR, Ising-type: for chunks of EMCS in one launch
+    void* d_ell = nullptr;
     uint64_t lat_hash = 0;            // CSR: FNV-1a of row_ptr, col_idx and bonds
     std::vector<int32_t> colour_ptr;  // host
     int32_t* d_order = nullptr;       // sites grouped by colour
