@@ -73,6 +73,9 @@ static bool is_f32_kind(int k) { return k == MQV_MODEL_HEISENBERG || k == MQV_MO
 bool ising2d_supported(int L);
 int ising2d_band_config(const Sim* s);
 const char* ising2d_config_name(Sim* s, char* buf, int len);
+bool ising2d_use_bits(Sim* s, int64_t sweeps);
+cudaError_t ising2d_bits_begin(Sim* s);
+cudaError_t ising2d_bits_end(Sim* s);
 cudaError_t launch_split_rows(Sim* s, const void* rowmajor, void* split);
 cudaError_t launch_merge_rows(Sim* s, const void* split, void* rowmajor);
 cudaError_t launch_validate_int8(Sim* s, const void* rowmajor, int* flag);
@@ -382,6 +385,31 @@ static mqv_status launch_sweep(Sim* s, int slot)
     MQV_CK(s->is_f32 ? launch_metropolis_f32(s, slot) : launch_metropolis_int8(s, slot));
     return MQV_OK;
 }
+// A run of sweeps with nothing between them but measurements, on bit planes
+// where that pays (ising2d.cu).  A run inside another one does nothing.
+class BitRun {
+public:
+    cudaError_t begin(Sim* s, int64_t sweeps)
+    {
+        if (s->bits_on || !ising2d_use_bits(s, sweeps)) return cudaSuccess;
+        s_ = s;
+        return ising2d_bits_begin(s);
+    }
+    cudaError_t end()
+    {
+        Sim* s = s_;
+        s_ = nullptr;
+        return s ? ising2d_bits_end(s) : cudaSuccess;
+    }
+    ~BitRun()
+    {
+        if (s_) s_->bits_on = false;  // a launch failed: the state stays as it was
+    }
+
+private:
+    Sim* s_ = nullptr;
+};
+
 // count sweeps, the last one measured into `slot` (-1: none)
 static mqv_status launch_sweeps(Sim* s, int count, int slot)
 {
@@ -389,10 +417,13 @@ static mqv_status launch_sweeps(Sim* s, int count, int slot)
         MQV_CK(launch_ell_emcs(s, 1, count, slot < 0 ? nullptr : s->d_acc + (size_t)slot * kAccStride));
         return MQV_OK;
     }
+    BitRun bits;
+    MQV_CK(bits.begin(s, count));
     for (int j = 0; j < count; ++j) {
         const mqv_status st = launch_sweep(s, j == count - 1 ? slot : -1);
         if (st) return st;
     }
+    MQV_CK(bits.end());
     return MQV_OK;
 }
 // Clusters by labelling (a fixed number of whole-lattice passes) or by one
@@ -464,6 +495,38 @@ static bool use_cluster(Sim* s)
     if (c < 2) return false;
     if (s->cluster_ok < 0) s->cluster_ok = cluster_launchable(c) ? 1 : 0;
     return s->cluster_ok == 1;
+}
+
+// One chunk of EMCS: ncluster clusters, nmetro sweeps and a measurement each,
+// into the accumulator and cluster-size slots from 0 on.
+static mqv_status launch_chunk(Sim* s, int ch, int ncluster, int nmetro)
+{
+    if (use_resident(s, ncluster)) {
+        MQV_CK(ensure_cuts(s));
+        MQV_CK(launch_emcs_resident(s, ch, ncluster, nmetro, true, s->d_acc, s->d_csize));
+        return MQV_OK;
+    }
+    if (use_cluster(s)) {
+        MQV_CK(ensure_cuts(s));
+        MQV_CK(launch_emcs_cluster(s, ch, ncluster, nmetro, s->d_acc, s->d_csize));
+        return MQV_OK;
+    }
+    if (s->d_ell && ncluster == 0) {
+        MQV_CK(launch_ell_emcs(s, ch, nmetro, s->d_acc));
+        return MQV_OK;
+    }
+    BitRun bits;
+    if (ncluster == 0) MQV_CK(bits.begin(s, (int64_t)ch * nmetro));
+    for (int e = 0; e < ch; ++e) {
+        for (int c = 0; c < ncluster; ++c) {
+            const mqv_status st = launch_cluster(s, e * ncluster + c);
+            if (st) return st;
+        }
+        const mqv_status st = nmetro > 0 ? launch_sweeps(s, nmetro, e) : launch_measure(s, e);
+        if (st) return st;
+    }
+    MQV_CK(bits.end());
+    return MQV_OK;
 }
 
 }  // namespace mqv
@@ -878,28 +941,8 @@ MQV_API mqv_status mqv_emcs(mqv_sim* h, int32_t n_emcs, int32_t ncluster, int32_
             if (st) return st;
         }
         MQV_CK(cudaMemsetAsync(s->d_acc, 0, sizeof(long long) * kAccStride * (size_t)ch, s->stream));
-        if (use_resident(s, ncluster)) {
-            MQV_CK(ensure_cuts(s));
-            MQV_CK(launch_emcs_resident(s, ch, ncluster, nmetro, true, s->d_acc, s->d_csize));
-        } else if (use_cluster(s)) {
-            MQV_CK(ensure_cuts(s));
-            MQV_CK(launch_emcs_cluster(s, ch, ncluster, nmetro, s->d_acc, s->d_csize));
-        } else if (s->d_ell && ncluster == 0) {
-            MQV_CK(launch_ell_emcs(s, ch, nmetro, s->d_acc));
-        } else {
-            for (int e = 0; e < ch; ++e) {
-                for (int c = 0; c < ncluster; ++c) {
-                    st = launch_cluster(s, e * ncluster + c);
-                    if (st) return st;
-                }
-                st = launch_sweeps(s, nmetro, e);
-                if (st) return st;
-                if (nmetro == 0) {
-                    st = launch_measure(s, e);
-                    if (st) return st;
-                }
-            }
-        }
+        st = launch_chunk(s, ch, ncluster, nmetro);
+        if (st) return st;
         st = launch_finalize(s, ch);
         if (st) return st;
         if (obs) MQV_CK(cudaMemcpyAsync(obs + done, s->d_obs, sizeof(double) * 4 * ch, cudaMemcpyDeviceToHost, s->stream));
@@ -948,28 +991,8 @@ MQV_API mqv_status mqv_emcs_samples(mqv_sim* h, int32_t n_emcs, int32_t ncluster
             if (st) return st;
         }
         MQV_CK(cudaMemsetAsync(s->d_acc, 0, sizeof(long long) * kAccStride * (size_t)ch, s->stream));
-        if (use_resident(s, ncluster)) {
-            MQV_CK(ensure_cuts(s));
-            MQV_CK(launch_emcs_resident(s, ch, ncluster, nmetro, true, s->d_acc, s->d_csize));
-        } else if (use_cluster(s)) {
-            MQV_CK(ensure_cuts(s));
-            MQV_CK(launch_emcs_cluster(s, ch, ncluster, nmetro, s->d_acc, s->d_csize));
-        } else if (s->d_ell && ncluster == 0) {
-            MQV_CK(launch_ell_emcs(s, ch, nmetro, s->d_acc));
-        } else {
-            for (int e = 0; e < ch; ++e) {
-                for (int c = 0; c < ncluster; ++c) {
-                    st = launch_cluster(s, e * ncluster + c);
-                    if (st) return st;
-                }
-                st = launch_sweeps(s, nmetro, e);
-                if (st) return st;
-                if (nmetro == 0) {
-                    st = launch_measure(s, e);
-                    if (st) return st;
-                }
-            }
-        }
+        st = launch_chunk(s, ch, ncluster, nmetro);
+        if (st) return st;
         MQV_CK(launch_acc_to_samples(s->d_acc, s->is_f32 ? 1 : 0, ch, d_samples + 4 * (size_t)done, s->stream));
         s->launches++;
         done += ch;

@@ -283,6 +283,11 @@ struct Sim {
     double thr_J = 0, thr_beta = -1;  // (J, beta) the cached 2D thresholds belong to
     unsigned long long thr_cut[5] = {};
     int sweep_cfg = -1;  // autotuned fused-sweep configuration (-1: not chosen yet)
+    // sweeps on bit planes: rows per thread and the fewest sweeps in a row (-1:
+    // not asked yet; 0: never), whether the state is there now, whether the last
+    // sweep ran there
+    int bits_rows = -1, bits_min = 0;
+    bool bits_on = false, bits_last = false;
     uint32_t flags = 0;  // MQV_FLAG_* of the run parameters
     // a device wait gave up: compute is refused until the state is set again
     bool failed = false;

@@ -59,7 +59,6 @@ struct Ising2DArgs {
     int mode;
     uint32_t useA, useB;        // 1 when the class needs a test (cut below 2^53)
     uint32_t tA8, tB8;          // threshold top bytes
-    uint32_t ztA, ztB;          // 1 when a top-byte tie rejects without the fine bits
     unsigned long long tA, tB;  // full u53 thresholds
     long long* acc;
     int* status;
@@ -128,8 +127,8 @@ __device__ __forceinline__ int wrapi(int v, int L)
 // Per-launch constants of the decision, as all-ones / all-zeros lane masks.
 struct Thr {
     uint32_t tA[8], tB[8];  // bit b of the class thresholds' top bytes
-    uint32_t useA, useB, ztA, ztB;
-    int mode;
+    uint32_t useA, useB;
+    uint32_t anti;  // J > 0
 };
 
 __device__ __forceinline__ Thr make_thr(const Ising2DArgs& a)
@@ -140,11 +139,9 @@ __device__ __forceinline__ Thr make_thr(const Ising2DArgs& a)
         t.tA[b] = 0u - ((a.tA8 >> b) & 1u);
         t.tB[b] = 0u - ((a.tB8 >> b) & 1u);
     }
-    t.useA = 0u - a.useA;
-    t.useB = 0u - a.useB;
-    t.ztA = 0u - a.ztA;
-    t.ztB = 0u - a.ztB;
-    t.mode = a.mode;
+    t.useA = a.mode == 2 ? 0u : 0u - a.useA;
+    t.useB = a.mode == 2 ? 0u : 0u - a.useB;
+    t.anti = a.mode == 1 ? ~0u : 0u;
     return t;
 }
 
@@ -178,26 +175,17 @@ __device__ __forceinline__ uint32_t decide_word(uint32_t A, uint32_t U, uint32_t
                                                 const Planes& rnd, const Thr& th, uint32_t& tie, uint32_t& inA)
 {
     const uint32_t* pl = rnd.b;
-    // minus-neighbour count M = m0 + 2 m1 + 4 m2 (carry-save adder; M <= 4)
-    const uint32_t s3 = U ^ D ^ Lb, c3 = (U & D) | (Lb & (U | D));  // full adder of three
-    const uint32_t m0 = s3 ^ Rb, c4 = s3 & Rb;                        // plus the fourth
-    const uint32_t m1 = c3 ^ c4, m2 = c3 & c4;
-    // the two tested classes (aligned count a = M for a -1 site, 4 - M for +1)
-    uint32_t maskA, maskB;
-    if (th.mode == 0) {
-        maskA = m0 & ~(A ^ m1);                    // a = 3
-        maskB = (A & m2) | (~A & ~(m0 | m1 | m2));  // a = 4
-    } else if (th.mode == 1) {
-        maskA = m0 & (A ^ m1);                     // a = 1
-        maskB = (~A & m2) | (A & ~(m0 | m1 | m2));  // a = 0
-    } else {
-        maskA = 0u;
-        maskB = 0u;
-    }
-    maskA &= th.useA;
-    maskB &= th.useB;
+    // The tested classes count unlike neighbours: none (class B) and one (class
+    // A) for J < 0, four and three for J > 0, which is the same of the flipped
+    // site.  Carry-save adder of three neighbours plus the fourth; a majority
+    // is self-dual, so comparing with the site comes after adding.
+    const uint32_t S = A ^ th.anti;
+    const uint32_t s3 = U ^ D ^ Lb, c3 = (U & D) | (Lb & (U | D));
+    const uint32_t maskA = (s3 ^ Rb) & ~(c3 ^ S);
+    const uint32_t maskB = ~((s3 ^ S) | (c3 ^ S)) & ~(Rb ^ S);
+    const uint32_t test = (maskA & th.useA) | (maskB & th.useB);
     // X < T and X == T for the per-site threshold byte T (class A or B)
-    uint32_t borrow = 0u, eq = ~0u;
+    uint32_t borrow = 0u, eq = test;
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
         const uint32_t tb = (maskA & th.tA[b]) | (~maskA & th.tB[b]);
@@ -205,10 +193,8 @@ __device__ __forceinline__ uint32_t decide_word(uint32_t A, uint32_t U, uint32_t
         borrow = (nx & (tb | borrow)) | (tb & borrow);
         eq &= ~(pl[b] ^ tb);
     }
-    const uint32_t test = maskA | maskB;
-    const uint32_t zt = (maskA & th.ztA) | (~maskA & th.ztB);
-    tie = eq & test & ~zt;
-    inA = tie & maskA;
+    tie = eq;
+    inA = eq & maskA;
     return A ^ (~test | borrow);
 }
 __device__ __forceinline__ uint32_t update_word(uint32_t A, uint32_t U, uint32_t D, uint32_t Lb, uint32_t Rb, int x,
@@ -958,6 +944,183 @@ __global__ void __launch_bounds__(ColourGeom<T>::NT) ising2d_colour(const __grid
     }
 }
 
+// ---- bit planes: several sweeps between two visits to the int8 state -------------
+//
+// A run of sweeps with nothing between them but measurements packs the state
+// once into a bit per site (in the spare state buffer: row y holds the L/64
+// words of its even half, then those of its odd half), sweeps the bits in
+// place, a launch per colour, and unpacks at the end.  A word update then
+// costs its draws and its logic and nothing else: no packing (30 of about 240
+// instructions), 5 words of L2 traffic instead of 4 x 32 bytes of HBM (L =
+// 16384: 34 MB of bits).  Bound by the ALU pipe (two Philox blocks, a
+// carry-save adder and an 8-step comparison per 32 sites).  Thread = T rows of
+// one word column, as in the colour kernel; the draws of its first rows come
+// before the launch waits for its predecessor.
+// Per sweep, int8 kernels before and this one (us): L = 1024 5.5 -> 4.0, L = 4096
+// 12.1 -> 7.7, L = 8192 38.5 -> 21.2, L = 16384 114 -> 71; packing and unpacking
+// together take what 1.4 sweeps take at L = 16384.  At L = 16384 186 instructions
+// per word, half of them for the Philox blocks, the ALU pipe busy 63 % of the time.
+template <int T>
+struct BitsGeom {
+    static constexpr int NT = T <= 2 ? 128 : 256;
+    static constexpr int TIECAP = 32 * T;       // every word of the warp's strips may hold ties
+    static constexpr int EARLY = T < 2 ? T : T <= 4 ? 2 : 0;  // rows whose draws come before the launch waits
+};
+
+__global__ void __launch_bounds__(256) ising2d_pack(const int8_t* __restrict__ s, uint32_t* __restrict__ bits,
+                                                    int64_t words)
+{
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k >= words) return;
+    const uint4* q = reinterpret_cast<const uint4*>(s) + 2 * k;
+    const uint4 lo = __ldcs(q), hi = __ldcs(q + 1);
+    bits[k] = pack_word(lo, hi);
+}
+__global__ void __launch_bounds__(256) ising2d_unpack(const uint32_t* __restrict__ bits, int8_t* __restrict__ s,
+                                                      int64_t words)
+{
+    grid_dep_wait();
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k >= words) return;
+    uint4 lo, hi;
+    unpack_word(bits[k], lo, hi);
+    uint4* q = reinterpret_cast<uint4*>(s) + 2 * k;
+    __stcs(q, lo);
+    __stcs(q + 1, hi);
+}
+
+// sum over the sites of a word of s * sum(nbrs): 4 per site less 2 per unlike
+// neighbour, the unlike neighbours added up by the carry-save adder
+__device__ __forceinline__ int word_bonds_unlike(uint32_t An, uint32_t U, uint32_t D, uint32_t Lb, uint32_t Rb)
+{
+    U ^= An;
+    D ^= An;
+    Lb ^= An;
+    Rb ^= An;
+    const uint32_t s3 = U ^ D ^ Lb, c3 = (U & D) | (Lb & (U | D));
+    const uint32_t m0 = s3 ^ Rb, c4 = s3 & Rb;
+    return 128 - 2 * __popc(m0) - 4 * __popc(c3 ^ c4) - 8 * __popc(c3 & c4);
+}
+
+template <int T, int COLOUR, bool MEAS>
+__global__ void __launch_bounds__(BitsGeom<T>::NT) ising2d_bits(const __grid_constant__ Ising2DArgs a)
+{
+    using G = BitsGeom<T>;
+    __shared__ uint4 ties[G::NT / 32][G::TIECAP];         // (byte offset, tie sites, class A, word)
+    __shared__ uint32_t tie_site[G::NT / 32][G::TIECAP];  // the word's first site
+    __shared__ int red[2][G::NT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t L = (uint32_t)a.L, ncol = L >> 6, half = 4 * ncol, pitch = 8 * ncol;  // bytes of a half-row and row
+    const uint32_t nstrip = ncol * (L / T);
+    const uint32_t id = blockIdx.x * G::NT + threadIdx.x;
+    const bool live = id < nstrip;
+    const uint32_t strip = live ? id : 0u, sy = strip / ncol, w = strip - sy * ncol, y0 = sy * T;
+    const uint32_t tg_acc = tag(kAccept, a.replica);
+    Thr th = make_thr(a);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) asm volatile("" : "+r"(th.tA[b]), "+r"(th.tB[b]));  // held, not derived again per word
+    // parity of the active half of row y0 + k; a strip of an even number of
+    // rows starts on an even one
+    const uint32_t odd = T % 2 ? y0 & 1u : 0u;
+    auto par = [&](int k) -> uint32_t { return ((uint32_t)(k + COLOUR) + odd) & 1u; };
+    // the word's 32-site group (accept_group of its first site)
+    const uint32_t g0 = 2u * (y0 * ncol + w);
+    auto planes = [&](int k) -> Planes {
+        const uint32_t g = g0 + 2u * (uint32_t)k * ncol + par(k);
+        const uint4 q0 = philox_rk(g, a.sweep, 0u, tg_acc, a);
+        const uint4 q1 = philox_rk(g, a.sweep, 1u, tg_acc, a);
+        return Planes{{q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w}};
+    };
+    char* bits = reinterpret_cast<char*>(a.dst);
+    auto at = [&](uint32_t off) -> uint32_t& { return *reinterpret_cast<uint32_t*>(bits + off); };
+    Planes rnd[G::EARLY > 0 ? G::EARLY : 1];
+#pragma unroll
+    for (int k = 0; k < G::EARLY; ++k) rnd[k] = planes(k);
+    grid_dep_launch();
+    grid_dep_wait();
+    // rows y0 - 1 .. y0 + T: the other colour's words (half 1 - p of a row
+    // whose active half is p), and of rows y0 .. the active words and the edge
+    // words: the even word to the right (p = 1), the odd word to the left (p = 0)
+    const uint32_t c0 = y0 * pitch + 4 * w;  // the even word of row y0
+    const uint32_t e1 = y0 * pitch + (w + 1 == ncol ? 0u : 4 * w + 4), e0 = y0 * pitch + half + (w == 0 ? half - 4 : 4 * w - 4);
+    uint32_t g[T + 2], act[T], edge[T];
+    g[0] = at((y0 == 0 ? c0 + (L - 1) * pitch : c0 - pitch) + (par(1) ? 0u : half));  // row y0 - 1 has row y0 + 1's parity
+    g[T + 1] = at((y0 + T == L ? c0 - y0 * pitch : c0 + T * pitch) + (par(T) ? 0u : half));
+#pragma unroll
+    for (int k = 0; k < T; ++k) {
+        const uint32_t p = par(k), rk = (uint32_t)k * pitch;
+        g[k + 1] = at(c0 + rk + (p ? 0u : half));
+        act[k] = at(c0 + rk + (p ? half : 0u));
+        edge[k] = at((p ? e1 : e0) + rk);
+    }
+    int ntie = 0, esum = 0, msum = 0;
+#pragma unroll
+    for (int k = 0; k < T; ++k) {
+        const uint32_t p = par(k);
+        const uint32_t G1 = g[k + 1];
+        const uint32_t Lb = p ? G1 : __funnelshift_l(edge[k], G1, 1);
+        const uint32_t Rb = p ? __funnelshift_r(G1, edge[k], 1) : G1;
+        uint32_t tie, inA;
+        const Planes r = k < G::EARLY ? rnd[k < G::EARLY ? k : 0] : planes(k);
+        const uint32_t An = decide_word(act[k], g[k], g[k + 2], Lb, Rb, r, th, tie, inA);
+        const uint32_t off = c0 + (uint32_t)k * pitch + (p ? half : 0u);
+        if (!live) tie = 0u;
+        const uint32_t has = __ballot_sync(0xffffffffu, tie != 0u);
+        if (tie) {
+            const int e = ntie + __popc(has & ((1u << lane) - 1u));
+            ties[warp][e] = make_uint4(off, tie, inA, An);
+            tie_site[warp][e] = (y0 + (uint32_t)k) * L + 64u * w + p;
+        }
+        ntie += __popc(has);
+        if (live) {
+            at(off) = An;
+            if (MEAS) {
+                esum += word_bonds_unlike(An, g[k], g[k + 2], Lb, Rb);
+                msum += 64 - 2 * __popc(An) - 2 * __popc(G1);
+            }
+        }
+    }
+    __syncwarp();
+    for (int e = lane; e < ntie; e += 32) {
+        const uint4 te = ties[warp][e];
+        const uint32_t site = tie_site[warp][e];
+        uint32_t flip = 0u;
+        for (uint32_t m = te.y; m; m &= m - 1) {
+            const int b = __ffs(m) - 1;
+            const bool inA = (te.z >> b) & 1u;
+            const uint64_t u53 = ((uint64_t)(inA ? a.tA8 : a.tB8) << 45) | (fine56_rk(site + 2u * (uint32_t)b, a) >> 11);
+            if (u53 < (inA ? a.tA : a.tB)) {
+                flip |= 1u << b;
+                if (MEAS) {
+                    // the tested classes have s * sum(nbrs) = +-2 (A) or +-4 (B) before the flip
+                    esum += (inA ? 4 : 8) * (a.mode == 0 ? -1 : 1);
+                    msum += (te.w >> b) & 1u ? 2 : -2;
+                }
+            }
+        }
+        // the word's only other writer in this launch stored it before the warp barrier
+        if (flip) at(te.x) = te.w ^ flip;
+    }
+    if (MEAS) {
+        esum = __reduce_add_sync(0xffffffffu, esum);
+        msum = __reduce_add_sync(0xffffffffu, msum);
+        if (lane == 0) {
+            red[0][warp] = esum;
+            red[1][warp] = msum;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            long long e = 0, m = 0;
+            for (int k = 0; k < G::NT / 32; ++k) {
+                e += red[0][k];
+                m += red[1][k];
+            }
+            atomicAdd(reinterpret_cast<unsigned long long*>(a.acc + kAccEne), (unsigned long long)(2 * e));
+            atomicAdd(reinterpret_cast<unsigned long long*>(a.acc + kAccMag), (unsigned long long)m);
+        }
+    }
+}
+
 // ---- layout conversion: row-major <-> split rows -----------------------------
 // One thread moves a group of 64 consecutive sites of a row (x = 64w .. 64w+63):
 // its even sites become word w of the even half, its odd sites word w of the
@@ -1220,8 +1383,6 @@ static void fill_args(Sim* s, const SweepConfig& c, long long* acc, Ising2DArgs&
     a.tB = TB;
     a.tA8 = (uint32_t)(TA >> 45) & 0xFFu;
     a.tB8 = (uint32_t)(TB >> 45) & 0xFFu;
-    a.ztA = (TA & ((1ull << 45) - 1)) == 0;
-    a.ztB = (TB & ((1ull << 45) - 1)) == 0;
     a.acc = acc;
     a.status = s->d_status;
     a.counter = s->d_counter;
@@ -1311,8 +1472,89 @@ int ising2d_band_config(const Sim* s)
     return -1;
 }
 
+// ---- host side of the bit planes ---------------------------------------------------
+
+template <int T>
+static cudaError_t launch_bits_t(const Ising2DArgs& a, cudaStream_t stream)
+{
+    const unsigned nt = BitsGeom<T>::NT, grid = ((unsigned)(a.L >> 6) * (unsigned)(a.L / T) + nt - 1) / nt;
+    const cudaError_t e = launch_pdl(ising2d_bits<T, 0, false>, grid, nt, stream, a);
+    if (e != cudaSuccess) return e;
+    return a.acc ? launch_pdl(ising2d_bits<T, 1, true>, grid, nt, stream, a)
+                 : launch_pdl(ising2d_bits<T, 1, false>, grid, nt, stream, a);
+}
+
+// Rows per thread: one shortens a launch, more share the neighbour rows and the
+// set-up (us per sweep with 1 / 2 / 4 / 8 rows: L = 1024 4.3 / 4.4 / 5.9 / 7.8, L =
+// 4096 9.3 / 7.7 / 9.8 / 12, L = 8192 31 / 24.5 / 21.2 / 22.3, L = 16384 118 / 92 / 77
+// / 71).
+static int bits_rows(int L) { return L < 3072 ? 1 : L < 6144 ? 2 : L < 12288 ? 4 : 8; }
+// Sweeps in a row from which packing and unpacking pay (us, int8 and bits: 3
+// sweeps at L = 16384 340 and 318, at L = 4096 38 and 36; 2 at L = 16384 227 and
+// 247, at L = 4096 26 and 28; at L = 1024 3 sweeps 17 and 18, 20 sweeps 115 and 87).
+static int bits_min_sweeps(int L) { return L < 2048 ? 5 : 3; }
+
+static void bits_name(const Sim* s, char* buf, int len) { snprintf(buf, len, "ising2d_bits<%d>", s->bits_rows); }
+
+// whether `sweeps` sweeps in a row run on bit planes
+bool ising2d_use_bits(Sim* s, int64_t sweeps)
+{
+    if (!s->fused_ising2d || s->inject_row >= 0) return false;
+    if (s->bits_rows < 0) {
+        // MARQOV_B200_SWEEP_CONFIG: ising2d_bits<T> takes the bit planes for any
+        // number of sweeps, another kernel's name never
+        s->bits_rows = bits_rows(s->len);
+        s->bits_min = bits_min_sweeps(s->len);
+        if (const char* want = getenv("MARQOV_B200_SWEEP_CONFIG")) {
+            int t = 0;
+            const bool named = sscanf(want, "ising2d_bits<%d>", &t) == 1 && (t == 1 || t == 2 || t == 4 || t == 8);
+            if (named) s->bits_rows = t;
+            s->bits_min = named ? 1 : 0;
+        }
+    }
+    return s->bits_min > 0 && sweeps >= s->bits_min;
+}
+
+// The state to bit planes in the spare buffer; until ising2d_bits_end the
+// sweeps (launch_ising2d_sweep) run there.
+cudaError_t ising2d_bits_begin(Sim* s)
+{
+    const int64_t words = s->n / 32;
+    ising2d_pack<<<(unsigned)((words + 255) / 256), 256, 0, s->stream>>>((const int8_t*)s->state[s->cur],
+                                                                        (uint32_t*)s->state[s->cur ^ 1], words);
+    s->launches++;
+    s->bits_on = true;
+    return cudaGetLastError();
+}
+
+cudaError_t ising2d_bits_end(Sim* s)
+{
+    const int64_t words = s->n / 32;
+    s->launches++;
+    s->bits_on = false;
+    s->bits_last = true;
+    return launch_pdl(ising2d_unpack, (unsigned)((words + 255) / 256), 256, s->stream,
+                      (const uint32_t*)s->state[s->cur ^ 1], (int8_t*)s->state[s->cur], words);
+}
+
+static cudaError_t launch_bits_sweep(Sim* s, long long* acc)
+{
+    Ising2DArgs a{};
+    fill_args(s, kConfigs[0], acc, a);
+    a.dst = (int8_t*)s->state[s->cur ^ 1];
+    s->launches += 2;
+    switch (s->bits_rows) {
+        case 1: return launch_bits_t<1>(a, s->stream);
+        case 2: return launch_bits_t<2>(a, s->stream);
+        case 4: return launch_bits_t<4>(a, s->stream);
+        default: return launch_bits_t<8>(a, s->stream);
+    }
+}
+
 cudaError_t launch_ising2d_sweep(Sim* s, long long* acc)
 {
+    if (s->bits_on) return launch_bits_sweep(s, acc);
+    s->bits_last = false;
     if (s->inject_row >= 0) s->sweep_cfg = ising2d_band_config(s);
     if (s->sweep_cfg < 0) {
         s->sweep_cfg = pick_config(s);
@@ -1338,6 +1580,10 @@ cudaError_t launch_ising2d_sweep(Sim* s, long long* acc)
 
 const char* ising2d_config_name(Sim* s, char* buf, int len)
 {
+    if (s->bits_last) {
+        bits_name(s, buf, len);
+        return buf;
+    }
     if (s->sweep_cfg < 0) return "";
     config_name(kConfigs[s->sweep_cfg], buf, len);
     return buf;
