@@ -75,6 +75,30 @@ __global__ void __launch_bounds__(kBatchMetroThreads)
     }
 }
 
+// The same over float members that all lie on hypercubic lattices and have SYMD
+// components: blocks and tables as batch_metro, NS sites per thread.
+template <int SYMD, int NS>
+__global__ void __launch_bounds__(kAccSites / NS)
+    batch_metro_f32(const BatchRep* __restrict__ reps, const int64_t* __restrict__ prefix,
+                    const int32_t* __restrict__ block_rep, const int32_t* __restrict__ ccount, int ncol, int colour,
+                    const BatchCtr* __restrict__ ctr, uint32_t e_off, int nmetro, int j)
+{
+    __shared__ uint4 tab[kAccTab];
+    const int r = block_rep[blockIdx.x];
+    const BatchRep& R = reps[r];
+    const int64_t t0 = (int64_t)blockIdx.x * kAccSites - prefix[r];
+    const uint32_t sweep = R.sweep0 + (ctr->e + e_off) * (uint32_t)nmetro + (uint32_t)j;
+    const uint32_t run0 = (uint32_t)(t0 / 32);
+    const Key key = R.key;
+    const uint32_t replica = R.replica;
+    if (threadIdx.x < 32) accept_tab_fill(tab, run0, key, sweep, replica);
+    __syncthreads();
+    with_dim(R.st, [&](const auto& lt) {
+        f32_block<SYMD, NS>(R.md, lt, (float*)R.s, t0, ccount[(size_t)r * ncol + colour], colour, key, sweep,
+                                   replica, tab, run0);
+    });
+}
+
 template <bool F32>
 __global__ void __launch_bounds__(1024) batch_wolff(const BatchRep* __restrict__ reps,
                                                     const BatchCtr* __restrict__ ctr, ClusterStep step,
@@ -308,6 +332,14 @@ static cudaError_t launch_emcs_t(const BatchLaunch& b, cudaStream_t st, int nclu
     for (int j = 0; j < nmetro; ++j)
         for (int colour = 0; colour < b.ncol; ++colour) {
             if (b.total[colour] == 0) continue;
+            if (F32 && b.stencil_symd) {
+                const int ns = f32_sites(b.stencil_symd, b.blocks[colour]);
+                auto* kernel = b.stencil_symd != 1 ? batch_metro_f32<3, 1> : ns == 1 ? batch_metro_f32<1, 1> : batch_metro_f32<1, 2>;
+                kernel<<<b.blocks[colour], kAccSites / ns, 0, st>>>(
+                    b.reps, b.prefix + (size_t)colour * (b.nrep + 1), b.block_rep + b.block_off[colour], b.ccount,
+                    b.ncol, colour, b.ctr, e_off, nmetro, j);
+                continue;
+            }
             batch_metro<F32><<<b.blocks[colour], kBatchMetroThreads, 0, st>>>(
                 b.reps, b.prefix + (size_t)colour * (b.nrep + 1), b.block_rep + b.block_off[colour], b.cbegin,
                 b.ccount, b.ncol, b.total[colour], colour, b.ctr, e_off, nmetro, j);

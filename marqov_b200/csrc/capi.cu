@@ -1808,13 +1808,18 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         MQV_CK(upload_sync(b->stream, *dst, src, bytes));
         return MQV_OK;
     };
-    // measurement CTAs: about 1024 sites each (four per thread: enough CTAs
-    // to fill the SMs on farms of small members, few enough that the CTAs'
-    // atomic adds and reductions stay a small part), at least one per member
+    // measurement CTAs: 1024 sites each (four per thread: enough CTAs to fill
+    // the SMs on farms of small members), more where that would be more than
+    // 12 CTAs per SM (a thread's reductions cost what several sites cost), at
+    // least one per member
+    int64_t msites = 0;
+    for (int r = 0; r < n; ++r)
+        if (!b->resident[(size_t)r]) msites += b->sims[(size_t)r]->n;
+    const int64_t per_part = std::max<int64_t>(1024, msites / (148 * 12));
     std::vector<int32_t> mprefix((size_t)n + 1, 0), mrep;
     for (int r = 0; r < n; ++r) {
         const int64_t parts =
-            b->resident[(size_t)r] ? 0 : std::max<int64_t>(1, (b->sims[(size_t)r]->n + 1023) / 1024);
+            b->resident[(size_t)r] ? 0 : std::max<int64_t>(1, (b->sims[(size_t)r]->n + per_part - 1) / per_part);
         if (mprefix[(size_t)r] + parts >= (int64_t)1 << 31) return bail(fail(MQV_ERR_INVALID_ARG, "batch too large"));
         mprefix[(size_t)r + 1] = mprefix[(size_t)r] + (int32_t)parts;
         for (int64_t k = 0; k < parts; ++k) mrep.push_back(r);
@@ -1847,6 +1852,9 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     b->L.reps = b->d_reps;
     b->L.nrep = n;
     b->L.f32 = b->f32 ? 1 : 0;
+    b->L.stencil_symd = b->f32 ? b->sims[0]->symd : 0;
+    for (const Sim* s : b->sims)
+        if (s->lat_kind != MQV_LATTICE_HYPERCUBIC || s->symd != b->L.stencil_symd) b->L.stencil_symd = 0;
     b->L.ncol = ncol;
     b->L.prefix = b->d_prefix;
     b->L.block_rep = b->d_block_rep;

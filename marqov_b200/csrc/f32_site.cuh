@@ -44,8 +44,15 @@ __device__ __forceinline__ void smallcap3(SubStream& rng, const float o[3], doub
 #pragma unroll
     for (int c = 0; c < 3; ++c) nv[c] = dx * e1[c] + dy * e2[c] + dz * (double)o[c];
     const double nn = sqrt(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
+    // Three quotients by one divisor from its correctly rounded reciprocal
+    // (Markstein 1990: the quotient corrected once by its exact remainder is
+    // the correctly rounded one; nn lies near 1, the components within it).
+    const double rn = __drcp_rn(nn);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) v[c] = nv[c] / nn;
+    for (int c = 0; c < 3; ++c) {
+        const double q = __dmul_rn(nv[c], rn);
+        v[c] = __fma_rn(__fma_rn(-nn, q, nv[c]), rn, q);
+    }
 }
 
 // Component c of site i of a float state: structure of arrays, s[c n + i]
@@ -140,6 +147,23 @@ __device__ __forceinline__ void f32_site(const ModelDev& m, const Lat& lat, floa
     }
 }
 
+// Decision of a move from the top byte of the site's acceptance word: 1
+// accepted, 0 rejected, -1 the exact cut is needed.  The acceptance 2^(log2(e)
+// (-beta dE)) in FP32 is within 1e-5 of cut 2^-53 (the rule's polynomial within
+// 1e-8, FP32 rounding of the exponent below 1e-6 where the result matters), and
+// u lies in [top, top + 1) / 256; whatever comes within 1e-4 of the edges goes
+// to the exact cut, about 1 in 200 moves, most of which tie there as well.
+__device__ __forceinline__ int accept_screen(double dE, double beta, uint32_t top)
+{
+    if (dE <= 0) return 1;
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((float)MQV_DMUL(-beta, dE) * 1.4426950408889634f));
+    const float lo = (float)top * 0.00390625f;
+    if (lo + 0.00390625f <= y * 0.9999f) return 1;
+    if (top > 0 && lo >= y * 1.0001f) return 0;
+    return -1;
+}
+
 template <class ST>
 __device__ __forceinline__ int64_t parity_site_f(const ST& st, int64_t t, int colour)
 {
@@ -147,6 +171,90 @@ __device__ __forceinline__ int64_t parity_site_f(const ST& st, int64_t t, int co
     int par = 0;
     for (int j = 1; j < st.degree(0) / 2; ++j) par += st.coord(i0, j);
     return i0 + (((par & 1) != colour) ? 1 : 0);
+}
+
+// Sites per thread of the stencil sweeps of one colour of so many blocks: two of
+// scalar states where they fill the chip, one otherwise (us per
+// sweep with one / two: 16 phi^4 chains of 16^3 5.5 / 6.5, 8 of 40^3 11 / 10.5, 32 of
+// 64^3 125 / 83; 3-vectors L = 64 12.3 / 15.7, L = 128 49 / 49 -- twice the code
+// stalls on instruction fetch).
+constexpr int f32_sites(int symd, int64_t blocks) { return symd == 1 && blocks >= 148 * 8 ? 2 : 1; }
+
+// One aligned block of kAccSites positions of a colour of a stencil, by
+// kAccSites / NS threads of NS sites each (NS = 2: the draws, FP64 chains and
+// loads of two sites run side by side in a thread, and what a thread fetches
+// once -- the model, FP64 constants, the lattice -- serves both; nothing is
+// stored before both are decided).  The moves are f32_site's, the decision
+// taken by accept_screen where the top byte suffices.  The block's acceptance
+// planes are in `tab`.
+template <int SYMD, int NS, class Lat>
+__device__ __forceinline__ void f32_block(const ModelDev& m, const Lat& lat, float* __restrict__ s, int64_t t0,
+                                          int64_t cnt, int colour, Key key, uint32_t sweep, uint32_t replica,
+                                          const uint4* tab, uint32_t run0)
+{
+    const int64_t n = lat.n;
+    const double w0 = onsite_w0(m, colour), w1 = onsite_w1(m, colour);
+    int64_t site[NS];
+    bool live[NS];
+    float o[NS][SYMD], nb[NS][SYMD], nf[NS][SYMD];
+    double dE[NS];
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        const int64_t t = t0 + threadIdx.x + j * (kAccSites / NS);
+        live[j] = t < cnt;
+        site[j] = live[j] ? parity_site_f(lat, t, colour) : 0;
+#pragma unroll
+        for (int c = 0; c < SYMD; ++c) {
+            o[j][c] = f32_get(s, n, c, site[j]);
+            nb[j][c] = 0.f;
+        }
+        const int deg = lat.degree(site[j]);
+        for (int q = 0; q < deg; ++q) {
+            const int64_t i = lat.nbr(site[j], q);
+#pragma unroll
+            for (int c = 0; c < SYMD; ++c) nb[j][c] += f32_get(s, n, c, i);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        SubStream rng(key, (uint32_t)site[j], sweep, tag(kMetro, replica));
+        if (SYMD == 1) {
+            const double r = 1.0 + (-1.0 - 1.0) * real01(rng.next());
+            const float of = o[j][0];
+            const double old = of;
+            nf[j][0] = (float)(old + m.cap * r);
+            const double nw = nf[j][0];
+            const double o2 = old * old, n2 = nw * nw;
+            dE[j] = m.J * (double)((nf[j][0] - of) * nb[j][0]) + w0 * m.h * (n2 - o2) +
+                    w1 * m.h2 * ((n2 - 1.0) * (n2 - 1.0) - (o2 - 1.0) * (o2 - 1.0));
+        } else {
+            constexpr int X = 0, Y = SYMD > 1 ? 1 : 0, Z = SYMD > 2 ? 2 : 0;
+            const float old[3] = {o[j][X], o[j][Y], o[j][Z]};
+            double v[3];
+            if (m.proposal == MQV_PROPOSAL_SMALL_CAP) smallcap3(rng, old, m.cap, v);
+            else rnddir3(rng, v);
+            nf[j][X] = (float)v[0];
+            nf[j][Y] = (float)v[1];
+            nf[j][Z] = (float)v[2];
+            const double dxy = (double)((nf[j][X] - old[0]) * nb[j][X]) + (double)((nf[j][Y] - old[1]) * nb[j][Y]);
+            const double dz = (double)((nf[j][Z] - old[2]) * nb[j][Z]);
+            dE[j] = m.J * (m.kind == MQV_MODEL_XXZ ? m.delta * dxy + dz : dxy + dz);
+            if (m.kind == MQV_MODEL_XXZ) {
+                const double zn = nf[j][Z], zo = old[2];
+                dE[j] += w0 * m.h * (zn - zo) + w1 * m.h2 * (zn * zn - zo * zo);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        if (!live[j]) continue;
+        const uint32_t i = (uint32_t)site[j], top = accept_top8_tab(tab, run0, i);
+        const int quick = accept_screen(dE[j], m.beta, top);
+        if (quick > 0 || (quick < 0 && accept_top_or_fine(accept_cut_direct(1, dE[j], m.beta), top, key, i, sweep, replica))) {
+#pragma unroll
+            for (int c = 0; c < SYMD; ++c) s[(int64_t)c * n + site[j]] = nf[j][c];
+        }
+    }
 }
 
 // ---- measurement (FP64) ---------------------------------------------------------
@@ -158,61 +266,91 @@ __device__ __forceinline__ double warp_sum_d(double v)
     return v;
 }
 
-// Part `part` of `nparts` of the accumulation (grid-stride share of a CTA;
-// the CTA's totals go to acc with atomics).
-template <class Lat>
-__device__ __forceinline__ void measure_f32_part(const ModelDev& m, const Lat& lat, const float* __restrict__ s,
-                                                 double* __restrict__ acc, int64_t part, int64_t nparts)
+// The neighbours of an energy sum over bonds: on stencils every bond lies in
+// both ends' lists, so the forward neighbours (+x, +y, ...) counted twice give
+// the sum with half the loads and conversions.
+__device__ __forceinline__ int energy_step(const StencilDev&) { return 2; }
+__device__ __forceinline__ int energy_step(const CSRDev&) { return 1; }
+
+// One thread's share (sites first, first + stride, ...) of the sums (energy,
+// x, y, z, sum of squares, of (square - 1)^2; scalar models leave y and z).
+// Bound by the latency of its loads: unrolled, so that those of several sites
+// are under way together (32 phi^4 chains of 64^3 84 -> 43 us with the forward
+// neighbours and more sites per thread, 8 CTAs per SM at most; Heisenberg at L =
+// 128 24 -> 15 us).
+template <int SYMD, class Lat>
+__device__ __forceinline__ void measure_f32_sums(const ModelDev& m, const Lat& lat, const float* __restrict__ s,
+                                                 int64_t first, int64_t stride, double v[6])
 {
-    __shared__ double red[6][32];
-    double e = 0, mx = 0, my = 0, mz = 0, q2 = 0, q4 = 0;
+    constexpr int Y = SYMD > 1 ? 1 : 0, Z = SYMD > 2 ? 2 : 0;
+    const int64_t n = lat.n;
+    const int step = energy_step(lat);
     // InteractionEnergy applies the interaction's get() to both ends
     // (observables.h:186-217): XXZ weights x x' and y y' by delta^2
-    const double wxy = m.kind == MQV_MODEL_XXZ ? m.delta * m.delta : 1.0;
     const bool xxz = m.kind == MQV_MODEL_XXZ;
-    for (int64_t i = part * (int64_t)blockDim.x + threadIdx.x; i < lat.n; i += nparts * blockDim.x) {
+    const double wxy = xxz ? m.delta * m.delta : 1.0;
+    double e = 0, mx = 0, my = 0, mz = 0, q2 = 0, q4 = 0;
+#pragma unroll SYMD == 1 ? 4 : 2
+    for (int64_t i = first; i < n; i += stride) {
         const int deg = lat.degree(i);
-        if (m.symd == 1) {
-            const double si = s[i];
-            double nb = 0;
-            for (int t = 0; t < deg; ++t) nb += (double)s[lat.nbr(i, t)];
-            e += si * nb;
-            mx += si;
-            const double p2 = si * si;
+        double p[SYMD], nb[SYMD];
+#pragma unroll
+        for (int c = 0; c < SYMD; ++c) {
+            p[c] = f32_get(s, n, c, i);
+            nb[c] = 0;
+        }
+        for (int t = 0; t < deg; t += step) {
+            const int64_t j = lat.nbr(i, t);
+#pragma unroll
+            for (int c = 0; c < SYMD; ++c) nb[c] += (double)f32_get(s, n, c, j);
+        }
+        mx += p[0];
+        if (SYMD == 1) {
+            e += p[0] * nb[0];
+            const double p2 = p[0] * p[0];
             q2 += p2;
             q4 += (p2 - 1.0) * (p2 - 1.0);
         } else {
-            const int64_t n = lat.n;
-            const double a = f32_get(s, n, 0, i), b = f32_get(s, n, 1, i), c = f32_get(s, n, 2, i);
-            double na = 0, nb = 0, nc = 0;
-            for (int t = 0; t < deg; ++t) {
-                const int64_t j = lat.nbr(i, t);
-                na += (double)f32_get(s, n, 0, j);
-                nb += (double)f32_get(s, n, 1, j);
-                nc += (double)f32_get(s, n, 2, j);
-            }
-            e += wxy * (a * na + b * nb) + c * nc;
-            mx += a;
-            my += b;
-            mz += c;
+            e += wxy * (p[0] * nb[0] + p[Y] * nb[Y]) + p[Z] * nb[Z];
+            my += p[Y];
+            mz += p[Z];
             if (xxz) {
-                q2 += c * c;  // the single-ion term's sum of s_z^2
+                q2 += p[Z] * p[Z];  // the single-ion term's sum of s_z^2
             } else {
-                const double p2 = a * a + b * b + c * c;
+                const double p2 = p[0] * p[0] + p[Y] * p[Y] + p[Z] * p[Z];
                 q2 += p2;
                 q4 += (p2 - 1.0) * (p2 - 1.0);
             }
         }
     }
-    double v[6] = {e, mx, my, mz, q2, q4};
+    v[0] = e * (double)step;
+    v[1] = mx;
+    v[2] = my;
+    v[3] = mz;
+    v[4] = q2;
+    v[5] = q4;
+}
+
+// Part `part` of `nparts` of the accumulation (the CTA's totals go to acc with
+// atomics).
+template <class Lat>
+__device__ __forceinline__ void measure_f32_part(const ModelDev& m, const Lat& lat, const float* __restrict__ s,
+                                                 double* __restrict__ acc, int64_t part, int64_t nparts)
+{
+    __shared__ double red[6][32];
+    const int64_t first = part * (int64_t)blockDim.x + threadIdx.x, stride = nparts * blockDim.x;
+    double v[6];
+    if (m.symd == 1) measure_f32_sums<1>(m, lat, s, first, stride, v);
+    else measure_f32_sums<3>(m, lat, s, first, stride, v);
     const int wid = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
+        if (m.symd == 1 && (k == 2 || k == 3)) continue;
         v[k] = warp_sum_d(v[k]);
         if ((threadIdx.x & 31) == 0) red[k][wid] = v[k];
     }
     __syncthreads();
-    if (threadIdx.x < 6) {
+    if (threadIdx.x < 6 && !(m.symd == 1 && (threadIdx.x == 2 || threadIdx.x == 3))) {
         double a = 0;
         for (int k = 0; k < (int)(blockDim.x >> 5); ++k) a += red[threadIdx.x][k];
         const int idx[6] = {kAccEne, kAccMag, kAccMagY, kAccMagZ, kAccSq, kAccQ4};

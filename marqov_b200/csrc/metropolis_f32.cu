@@ -8,6 +8,8 @@
 // lattice-wide reductions accumulate in FP64.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "f32_site.cuh"
 
 namespace mqv {
@@ -15,28 +17,27 @@ namespace mqv {
 unsigned long long accept_cut(int pref, double dE, double beta);
 
 // One colour of a stencil sweep.  A CTA takes one aligned block of kAccSites
-// sites of the colour (kAccRuns runs of 64 lattice sites), one site per
-// thread: its first warp draws the block's acceptance bytes (accept_tab_fill,
-// one Philox block per lane), a CTA barrier publishes them, and every thread
-// updates its site.  One site per thread keeps enough warps in flight to
-// cover the FP64 latency of the proposal and the acceptance.
-constexpr int kMetroThreads = kAccSites;
-__global__ void __launch_bounds__(kMetroThreads) metro_f32_stencil(ModelDev m, StencilDev st, float* __restrict__ s,
+// sites of the colour (kAccRuns runs of 64 lattice sites), NS per thread:
+// its first warp draws the block's acceptance bytes (accept_tab_fill, one
+// Philox block per lane), a CTA barrier publishes them, and every thread
+// updates its sites (f32_block).
+// Bound by instruction issue (69 % busy, 528 instructions per 32 moves of a
+// small-cap proposal, a third of them FP64).  Heisenberg at L = 128: 58 -> 49 us a
+// sweep, since the decision no longer computes the exact cut (accept_screen), the
+// proposal's three quotients share a reciprocal, and the model's branches are
+// taken at compile time.
+template <int SYMD, int NS>
+__global__ void __launch_bounds__(kAccSites / NS) metro_f32_stencil(ModelDev m, StencilDev st, float* __restrict__ s,
                                                                    int colour, Key key, uint32_t sweep, uint32_t replica)
 {
     __shared__ uint4 tab[kAccTab];
-    const int64_t half = st.n / 2, nblk = (half + kAccSites - 1) / kAccSites;
-    for (int64_t b = blockIdx.x; b < nblk; b += gridDim.x) {
-        const uint32_t run0 = (uint32_t)(b * kAccRuns);
-        if (threadIdx.x < 32) accept_tab_fill(tab, run0, key, sweep, replica);
-        __syncthreads();
-        const int64_t t = b * kAccSites + threadIdx.x;
-        const bool live = t < half;
-        with_dim(st, [&](const auto& lt) {
-            f32_site(m, lt, s, live ? parity_site_f(lt, t, colour) : 0, key, sweep, replica, live, colour, tab, run0);
-        });
-        __syncthreads();  // every thread has read the table before the next block's draw
-    }
+    const uint32_t run0 = blockIdx.x * kAccRuns;
+    if (threadIdx.x < 32) accept_tab_fill(tab, run0, key, sweep, replica);
+    __syncthreads();
+    with_dim(st, [&](const auto& lt) {
+        f32_block<SYMD, NS>(m, lt, s, (int64_t)blockIdx.x * kAccSites, st.n / 2, colour, key, sweep, replica, tab,
+                            run0);
+    });
 }
 
 __global__ void metro_f32_csr(ModelDev m, CSRDev g, float* __restrict__ s, const int32_t* __restrict__ order,
@@ -121,7 +122,8 @@ cudaError_t launch_measure_f32(Sim* s, int slot)
 {
     double* acc = reinterpret_cast<double*>(s->d_acc + (size_t)slot * kAccStride);
     const float* st = (const float*)s->state[s->cur];
-    const int g = grid_for_f(s->n, 256);
+    // up to 8 CTAs per SM: more sites per thread before the reductions
+    const int g = std::min(grid_for_f(s->n, 256), 148 * 8);
     if (s->lat_kind == MQV_LATTICE_HYPERCUBIC) measure_f32<<<g, 256, 0, s->stream>>>(s->md, s->sten, st, acc);
     else measure_f32<<<g, 256, 0, s->stream>>>(s->md, s->csr, st, acc);
     s->launches++;
@@ -142,10 +144,11 @@ cudaError_t launch_metropolis_f32(Sim* s, int slot)
     float* st = (float*)s->state[s->cur];
     if (s->lat_kind == MQV_LATTICE_HYPERCUBIC) {
         // one CTA per block of kAccSites sites of a colour
-        const int g = grid_for_f((s->n / 2 + kAccSites - 1) / kAccSites * kMetroThreads, kMetroThreads);
+        const unsigned g = (unsigned)((s->n / 2 + kAccSites - 1) / kAccSites);
         for (int c = 0; c < 2; ++c) {
-            metro_f32_stencil<<<g, kMetroThreads, 0, s->stream>>>(s->md, s->sten, st, c, key, (uint32_t)s->sweep,
-                                                                  s->replica);
+            const int ns = f32_sites(s->symd, g);
+            auto* kernel = s->symd != 1 ? metro_f32_stencil<3, 1> : ns == 1 ? metro_f32_stencil<1, 1> : metro_f32_stencil<1, 2>;
+            kernel<<<g, kAccSites / ns, 0, s->stream>>>(s->md, s->sten, st, c, key, (uint32_t)s->sweep, s->replica);
             s->launches++;
         }
     } else {
