@@ -99,6 +99,19 @@ __global__ void __launch_bounds__(kAccSites / NS)
     });
 }
 
+// The same over members that are all Potts stencils in octets.
+__global__ void __launch_bounds__(kOctetThreads)
+    batch_metro_potts(const BatchRep* __restrict__ reps, const int64_t* __restrict__ prefix,
+                      const int32_t* __restrict__ block_rep, const int32_t* __restrict__ ccount, int ncol, int colour,
+                      const BatchCtr* __restrict__ ctr, uint32_t e_off, int nmetro, int j)
+{
+    const int r = block_rep[blockIdx.x];
+    const BatchRep& R = reps[r];
+    const uint32_t sweep = R.sweep0 + (ctr->e + e_off) * (uint32_t)nmetro + (uint32_t)j;
+    potts_block(R.md, R.st, (int8_t*)R.s, (int64_t)blockIdx.x * kAccSites - prefix[r],
+                ccount[(size_t)r * ncol + colour], colour, R.key, sweep, R.replica, R.cuts, R.D);
+}
+
 template <bool F32>
 __global__ void __launch_bounds__(1024) batch_wolff(const BatchRep* __restrict__ reps,
                                                     const BatchCtr* __restrict__ ctr, ClusterStep step,
@@ -146,7 +159,7 @@ __global__ void batch_measure(const BatchRep* __restrict__ reps, const BatchCtr*
             measure_f32_part(R.md, R.csr, (const float*)R.s, (double*)a, part, nparts);
     } else {
         if (R.lat_kind == MQV_LATTICE_HYPERCUBIC)
-            with_dim(R.st, [&](const auto& lt) { measure_int8_part(R.md, lt, (const int8_t*)R.s, a, part, nparts); });
+            measure_int8_stencil(R.md, R.st, (const int8_t*)R.s, a, part, nparts);
         else
             measure_int8_part(R.md, R.csr, (const int8_t*)R.s, a, part, nparts);
     }
@@ -336,6 +349,12 @@ static cudaError_t launch_emcs_t(const BatchLaunch& b, cudaStream_t st, int nclu
                 const int ns = f32_sites(b.stencil_symd, b.blocks[colour]);
                 auto* kernel = b.stencil_symd != 1 ? batch_metro_f32<3, 1> : ns == 1 ? batch_metro_f32<1, 1> : batch_metro_f32<1, 2>;
                 kernel<<<b.blocks[colour], kAccSites / ns, 0, st>>>(
+                    b.reps, b.prefix + (size_t)colour * (b.nrep + 1), b.block_rep + b.block_off[colour], b.ccount,
+                    b.ncol, colour, b.ctr, e_off, nmetro, j);
+                continue;
+            }
+            if (!F32 && b.potts_octets) {
+                batch_metro_potts<<<b.blocks[colour], kOctetThreads, 0, st>>>(
                     b.reps, b.prefix + (size_t)colour * (b.nrep + 1), b.block_rep + b.block_off[colour], b.ccount,
                     b.ncol, colour, b.ctr, e_off, nmetro, j);
                 continue;

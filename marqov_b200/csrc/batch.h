@@ -95,6 +95,7 @@ struct BatchLaunch {
     int nrep;
     int f32;                     // float members (else int8)
     int stencil_symd;            // float: the components of every member, all on hypercubic lattices (else 0)
+    int potts_octets;            // int8: every member not resident is a Potts stencil in octets
     int ncol;                    // colours of the member with the most
     const int64_t* prefix;       // [ncol][nrep + 1]
     const int32_t* block_rep;    // [sum of blocks]

@@ -1809,13 +1809,20 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         return MQV_OK;
     };
     // measurement CTAs: 1024 sites each (four per thread: enough CTAs to fill
-    // the SMs on farms of small members), more where that would be more than
+    // the SMs on farms of small members; two octets where sites are taken by
+    // octets), more where that would be more than
     // 12 CTAs per SM (a thread's reductions cost what several sites cost), at
     // least one per member
     int64_t msites = 0;
     for (int r = 0; r < n; ++r)
         if (!b->resident[(size_t)r]) msites += b->sims[(size_t)r]->n;
-    const int64_t per_part = std::max<int64_t>(1024, msites / (148 * 12));
+    b->L.potts_octets = b->f32 ? 0 : 1;
+    for (int r = 0; r < n; ++r) {
+        const Sim* s = b->sims[(size_t)r];
+        if (!b->resident[(size_t)r] && !(s->lat_kind == MQV_LATTICE_HYPERCUBIC && potts_octets(s->md, s->sten)))
+            b->L.potts_octets = 0;
+    }
+    const int64_t per_part = std::max<int64_t>(b->L.potts_octets ? 4096 : 1024, msites / (148 * 12));
     std::vector<int32_t> mprefix((size_t)n + 1, 0), mrep;
     for (int r = 0; r < n; ++r) {
         const int64_t parts =

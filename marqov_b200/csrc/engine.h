@@ -165,6 +165,13 @@ __device__ __forceinline__ void with_dim(const StencilDev& st, F&& f)
     }
 }
 
+// Potts stencils updated and measured by octets of an x-line (int8_site.cuh):
+// row-major int8 states with sides of a multiple of 8.
+MQV_HD bool potts_octets(const ModelDev& m, const StencilDev& st)
+{
+    return m.kind == MQV_MODEL_POTTS && (st.dim == 2 || st.dim == 3) && st.len % 8 == 0 && !st.split && !st.fb;
+}
+
 struct CSRDev {
     int64_t n;
     const int32_t* rp;

@@ -45,6 +45,14 @@ __global__ void __launch_bounds__(kMetroThreads) metro_int8_stencil(ModelDev m, 
     }
 }
 
+// The same of a Potts stencil in octets (potts_octet): a quarter of the threads.
+__global__ void __launch_bounds__(kOctetThreads) metro_potts(ModelDev m, StencilDev st, int8_t* __restrict__ s, int colour,
+                                                             Key key, uint32_t sweep, uint32_t replica,
+                                                             const unsigned long long* __restrict__ cuts, int D)
+{
+    potts_block(m, st, s, (int64_t)blockIdx.x * kAccSites, st.n / 2, colour, key, sweep, replica, cuts, D);
+}
+
 __global__ void metro_int8_csr(ModelDev m, CSRDev g, int8_t* __restrict__ s, const int32_t* __restrict__ order,
                                int64_t begin, int64_t count, Key key, uint32_t sweep, uint32_t replica,
                                const unsigned long long* __restrict__ cuts, int D)
@@ -120,7 +128,7 @@ __global__ void measure_int8(ModelDev m, Lat lat, const int8_t* __restrict__ s, 
 template <>
 __global__ void measure_int8(ModelDev m, StencilDev st, const int8_t* __restrict__ s, long long* __restrict__ acc)
 {
-    with_dim(st, [&](const auto& lt) { measure_int8_part(m, lt, s, acc, blockIdx.x, gridDim.x); });
+    measure_int8_stencil(m, st, s, acc, blockIdx.x, gridDim.x);
 }
 
 __global__ void finalize_int8(ModelDev m, int64_t n, const long long* __restrict__ acc, int nslots,
@@ -214,6 +222,12 @@ cudaError_t launch_metropolis_int8(Sim* s, int slot)
         // one CTA per block of kAccSites sites of a colour
         const int g = grid_for((s->n / 2 + kAccSites - 1) / kAccSites * kMetroThreads, kMetroThreads);
         for (int c = 0; c < 2; ++c) {
+            if (potts_octets(s->md, s->sten)) {
+                metro_potts<<<(unsigned)((s->n / 2 + kAccSites - 1) / kAccSites), kOctetThreads, 0, s->stream>>>(
+                    s->md, s->sten, st, c, key, (uint32_t)s->sweep, s->replica, s->d_cuts, s->max_degree);
+                s->launches++;
+                continue;
+            }
             metro_int8_stencil<<<g, kMetroThreads, 0, s->stream>>>(s->md, s->sten, st, c, key, (uint32_t)s->sweep,
                                                                    s->replica, s->d_cuts, s->max_degree);
             s->launches++;
