@@ -318,6 +318,8 @@ struct Sim {
     // clusters of this lattice: MQV_WOLFF_AUTO (by size), _BFS or _LABEL, and
     // the one-member tables of the labelling kernels (wolff.cu)
     int wolff_algo = 0;
+    double last_cluster = 0;  // mean size of the clusters last reported to the host
+    bool no_label = false;    // the labelling's tables did not fit the device
     struct BatchRep* d_rep1 = nullptr;
     struct BatchCtr* d_ctr1 = nullptr;
     void* d_seed1 = nullptr;
