@@ -171,29 +171,60 @@ __device__ void bits_run(const ResidentRun& R, unsigned char* smem)
     unsigned short* list = reinterpret_cast<unsigned short*>(edge) + warp * kBitsList;
     uint32_t* res = reinterpret_cast<uint32_t*>(P) + warp * kBitsRes;  // outcomes of the list (before there are runs)
 
-    // the state (and the bond signs) to planes, several words' loads in flight
-    constexpr int NLD = BOND ? 4 : 8;
-    for (int w0 = warp; w0 < NW; w0 += NLD * kBitsWarps) {
-        int8_t v[NLD][BOND ? 1 + D : 1];
-#pragma unroll
-        for (int k = 0; k < NLD; ++k) {
-            const int wi = w0 + k * kBitsWarps;
-            const auto o = g.word(wi < NW ? wi : 0);
-            const int x = 32 * o.w + lane;
-            const bool live = wi < NW && x < L;
-            const int64_t i = live ? (int64_t)o.row * L + x : 0;
-            v[k][0] = live ? R.state[R.st.addr(i)] : (int8_t)0;
-            if (BOND)
-#pragma unroll
-                for (int d = 0; d < D; ++d) v[k][1 + d] = live ? R.st.fb[(int64_t)d * n + i] : (int8_t)0;
+    // The state (and the bond signs) to planes: a thread takes 64 sites of split
+    // rows, or a word of a line of a multiple of 8 sites, in wide loads; else the
+    // warps take word by word, several words' loads in flight.
+    // (A call of one EMCS is mostly this: 32 members of L = 128, a sweep and an
+    // exchange per launch 29.6 -> 16.4 us, of L = 160 51 -> 20.)
+    const bool split = R.st.split, wide = split || L % 8 == 0;
+    if (!BOND && split) {
+        for (int k = tid; k < NW / 2; k += kBitsThreads) {
+            const int row = g.wr == 2 ? k : 2 * k / g.wr, h = k - row * (g.wr / 2);
+            const uint4* q = reinterpret_cast<const uint4*>(R.state + (int64_t)row * L + 32 * h);
+            const uint4* q1 = reinterpret_cast<const uint4*>(R.state + (int64_t)row * L + L / 2 + 32 * h);
+            const uint4 e0 = q[0], e1 = q[1], o0 = q1[0], o1 = q1[1];
+            const uint32_t E = pack_word(e0, e1), O = pack_word(o0, o1);
+            A[2 * k] = spread16(E & 0xFFFFu) | (spread16(O & 0xFFFFu) << 1);
+            A[2 * k + 1] = spread16(E >> 16) | (spread16(O >> 16) << 1);
         }
+    } else if (wide) {
+        // plane 0: the spins, plane 1 + d: the +d bonds
+        for (int k = tid; k < (BOND ? 1 + D : 1) * NW; k += kBitsThreads) {
+            const int d = BOND ? k / NW : 0, wi = k - d * NW;
+            const auto o = g.word(wi);
+            const int8_t* p = (d == 0 ? R.state : R.st.fb + (int64_t)(d - 1) * n) + (int64_t)o.row * L + 32 * o.w;
+            uint2 v[4];
 #pragma unroll
-        for (int k = 0; k < NLD; ++k) {
-            const int wi = w0 + k * kBitsWarps;
+            for (int j = 0; j < 4; ++j) v[j] = 8 * j < o.nb ? reinterpret_cast<const uint2*>(p)[j] : make_uint2(0u, 0u);
+            uint32_t m = 0u;
 #pragma unroll
-            for (int d = 0; d < (BOND ? 1 + D : 1); ++d) {
-                const uint32_t m = __ballot_sync(0xffffffffu, v[k][d] < 0);
-                if (lane == 0 && wi < NW) A[d * NW + wi] = m;  // the bonds' planes follow the spins'
+            for (int j = 0; j < 4; ++j) m |= (pack4(v[j].x) | (pack4(v[j].y) << 4)) << (8 * j);
+            A[k] = m;  // the bonds' planes follow the spins'
+        }
+    } else {
+        constexpr int NLD = BOND ? 4 : 8;
+        for (int w0 = warp; w0 < NW; w0 += NLD * kBitsWarps) {
+            int8_t v[NLD][BOND ? 1 + D : 1];
+#pragma unroll
+            for (int k = 0; k < NLD; ++k) {
+                const int wi = w0 + k * kBitsWarps;
+                const auto o = g.word(wi < NW ? wi : 0);
+                const int x = 32 * o.w + lane;
+                const bool live = wi < NW && x < L;
+                const int64_t i = live ? (int64_t)o.row * L + x : 0;
+                v[k][0] = live ? R.state[R.st.addr(i)] : (int8_t)0;
+                if (BOND)
+#pragma unroll
+                    for (int d = 0; d < D; ++d) v[k][1 + d] = live ? R.st.fb[(int64_t)d * n + i] : (int8_t)0;
+            }
+#pragma unroll
+            for (int k = 0; k < NLD; ++k) {
+                const int wi = w0 + k * kBitsWarps;
+#pragma unroll
+                for (int d = 0; d < (BOND ? 1 + D : 1); ++d) {
+                    const uint32_t m = __ballot_sync(0xffffffffu, v[k][d] < 0);
+                    if (lane == 0 && wi < NW) A[d * NW + wi] = m;  // the bonds' planes follow the spins'
+                }
             }
         }
     }
@@ -621,10 +652,35 @@ __device__ void bits_run(const ResidentRun& R, unsigned char* smem)
         }
     }
     __syncthreads();
-    for (int wi = warp; wi < NW; wi += kBitsWarps) {
-        const auto o = g.word(wi);
-        const int x = 32 * o.w + lane;
-        if (x < L) R.state[R.st.addr((int64_t)o.row * L + x)] = (A[wi] >> lane) & 1u ? -1 : 1;
+    if (!BOND && split) {
+        for (int k = tid; k < NW / 2; k += kBitsThreads) {
+            const int row = g.wr == 2 ? k : 2 * k / g.wr, h = k - row * (g.wr / 2);
+            const uint32_t a = A[2 * k], b = A[2 * k + 1];
+            uint4 lo, hi;
+            uint4* q = reinterpret_cast<uint4*>(R.state + (int64_t)row * L + 32 * h);
+            unpack_word(pack16(a) | (pack16(b) << 16), lo, hi);
+            q[0] = lo;
+            q[1] = hi;
+            q = reinterpret_cast<uint4*>(R.state + (int64_t)row * L + L / 2 + 32 * h);
+            unpack_word(pack16(a >> 1) | (pack16(b >> 1) << 16), lo, hi);
+            q[0] = lo;
+            q[1] = hi;
+        }
+    } else if (wide) {
+        for (int wi = tid; wi < NW; wi += kBitsThreads) {
+            const auto o = g.word(wi);
+            const uint32_t a = A[wi];
+            uint2* p = reinterpret_cast<uint2*>(R.state + (int64_t)o.row * L + 32 * o.w);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (8 * j < o.nb) p[j] = make_uint2(unpack4((a >> (8 * j)) & 15u), unpack4((a >> (8 * j + 4)) & 15u));
+        }
+    } else {
+        for (int wi = warp; wi < NW; wi += kBitsWarps) {
+            const auto o = g.word(wi);
+            const int x = 32 * o.w + lane;
+            if (x < L) R.state[R.st.addr((int64_t)o.row * L + x)] = (A[wi] >> lane) & 1u ? -1 : 1;
+        }
     }
 }
 

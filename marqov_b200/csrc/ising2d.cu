@@ -215,51 +215,6 @@ __device__ __forceinline__ int word_bonds(uint32_t An, uint32_t U, uint32_t D, u
     return 128 - 2 * sM - 8 * __popc(An) + 4 * sAM;
 }
 
-// Packing between the staged bytes (+1 -> 0x01, -1 -> 0xFF, one word of 32
-// sites stored transposed, see split_addr) and 32-bit words (bit s = site s,
-// 1 = spin -1): bit 1 of byte k of the word's 32-bit lane i is site 8k + i.
-//
-// lanes 0..3 of a word -> bits 8k + i, i < 4 (shift by 4 for lanes 4..7)
-__device__ __forceinline__ uint32_t pack_lanes4(uint4 v)
-{
-    const uint32_t M = 0x01010101u;
-    uint32_t t = (v.x >> 1) & M;
-    t |= v.y & (M << 1);
-    t |= (v.z << 1) & (M << 2);
-    t |= (v.w << 2) & (M << 3);
-    return t;
-}
-
-__device__ __forceinline__ uint32_t pack_word(uint4 lo, uint4 hi)
-{
-    // Horner's rule over lanes 6 .. 0 puts lane i's bit 1 of byte k at bit
-    // 8k + 1 + i (multiply-adds); lane 7 is placed separately so that nothing
-    // runs past bit 31
-    const uint32_t m = 0x02020202u;  // bit 1 of each byte: set for spin -1
-    uint32_t h = hi.z & m;
-    h = h * 2u + (hi.y & m);
-    h = h * 2u + (hi.x & m);
-    h = h * 2u + (lo.w & m);
-    h = h * 2u + (lo.z & m);
-    h = h * 2u + (lo.y & m);
-    h = h * 2u + (lo.x & m);
-    return (h >> 1) | ((hi.w & m) << 6);
-}
-
-// 32 bits -> the word's 32 bytes as two 16-byte vectors (lanes 0..3, 4..7)
-__device__ __forceinline__ void unpack_word(uint32_t t, uint4& lo, uint4& hi)
-{
-    const uint32_t M = 0x01010101u;
-    lo.x = (t & M) * 0xFEu + M;
-    lo.y = ((t >> 1) & M) * 0xFEu + M;
-    lo.z = ((t >> 2) & M) * 0xFEu + M;
-    lo.w = ((t >> 3) & M) * 0xFEu + M;
-    hi.x = ((t >> 4) & M) * 0xFEu + M;
-    hi.y = ((t >> 5) & M) * 0xFEu + M;
-    hi.z = ((t >> 6) & M) * 0xFEu + M;
-    hi.w = ((t >> 7) & M) * 0xFEu + M;
-}
-
 // 32 bits -> 32 bytes at p (16-byte aligned)
 __device__ __forceinline__ void unpack32(uint32_t bits, uint8_t* p)
 {
