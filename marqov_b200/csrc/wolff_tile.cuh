@@ -509,6 +509,7 @@ __global__ void __launch_bounds__(U * LPU)
     }
     __syncthreads();
     const int nrun = s_nrun;
+#pragma unroll 4
     for (int k = tid; k < nrun; k += NT) lab[k] = R.tl_lab[base + k];
     if (tid == 0) {
         // the seed's root
@@ -521,11 +522,33 @@ __global__ void __launch_bounds__(U * LPU)
     }
     __syncthreads();
     const int root = s_root;
-    // the forest above each local root
-    for (int k0 = tid - lane; k0 < nrun; k0 += NT) {
-        const int k = k0 + lane;
-        const uint32_t m = __ballot_sync(0xffffffffu, k < nrun && lab[k] == k && walk(base + k) == root);
-        if (lane == 0) in[k0 >> 5] = m;
+    // The forest above each local root.  A walk is a chain of dependent loads:
+    // a lane takes those of four runs side by side.
+    for (int k0 = tid - lane; k0 < nrun; k0 += 4 * NT) {
+        int x[4];  // -1: not a local root
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = k0 + j * NT + lane;
+            x[j] = k < nrun && lab[k] == k ? base + k : -1;
+        }
+        bool open;
+        do {
+            int p[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) p[j] = x[j] >= 0 ? __ldcg(forest + x[j]) : -1;
+            open = false;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                open = open || p[j] != x[j];
+                x[j] = p[j];
+            }
+        } while (open);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (k0 + j * NT >= nrun) break;
+            const uint32_t m = __ballot_sync(0xffffffffu, x[j] == root);
+            if (lane == 0) in[(k0 + j * NT) >> 5] = m;
+        }
     }
     __syncthreads();
     // every run follows its local root
