@@ -344,6 +344,12 @@ MQV_API mqv_status mqv_selftest_accept_cut(int32_t pref, int32_t n, const double
  * out_curand receive 4n words each (host). */
 MQV_API mqv_status mqv_selftest_philox(uint64_t seed, uint32_t c1, uint32_t c2, uint32_t c3,
                                        int32_t n, uint32_t* out_engine, uint32_t* out_curand);
+/* Self test (host only): the layout of the one-launch graph sweeps on `ctas`
+ * CTAs (1 .. 16).  words[c * ctas + r] receives the 32-site words of CTA r in
+ * the c-th colour that has sites, as far as `room` entries go, ncolours the
+ * number of those colours. */
+MQV_API mqv_status mqv_selftest_graph_words(int32_t n, const int32_t* colours, int32_t ctas, int32_t* words,
+                                            int32_t room, int32_t* ncolours);
 /* Self test of the bounded device waits: the next fused 2D Ising sweep of
  * the handle (band kernel, L = 8192 or 16384) has CTA 0 withhold its staged
  * row `row` (2 .. 64) and waits at most wait_ns for a row, so that the wait

@@ -45,6 +45,7 @@ cudaError_t ensure_label_tables(Sim* s, bool label);
 cudaError_t build_ell(Sim* s, int64_t n, const int32_t* rp, const int32_t* ci, const int8_t* bonds,
                       const std::vector<int32_t>& col);
 cudaError_t launch_ell_emcs(Sim* s, int n_emcs, int nmetro, long long* acc);
+int ell_words(int64_t n, const int32_t* col, int ctas, int32_t* words, int64_t room);
 bool resident_fits(const Sim* s);
 cudaError_t launch_emcs_cluster(Sim* s, int n_emcs, int ncluster, int nmetro, long long* acc, int32_t* csize);
 cudaError_t launch_emcs_resident(Sim* s, int n_emcs, int ncluster, int nmetro, bool measure, long long* acc,
@@ -1138,6 +1139,17 @@ MQV_API mqv_status mqv_selftest_accept_cut(int32_t pref, int32_t n, const double
     if (n < 0 || (n > 0 && (!dE || !beta || !cut)) || (pref != 1 && pref != 2))
         return fail(MQV_ERR_INVALID_ARG, "bad arguments");
     for (int32_t i = 0; i < n; ++i) cut[i] = accept_cut_direct(pref, dE[i], beta[i]);
+    return MQV_OK;
+}
+
+MQV_API mqv_status mqv_selftest_graph_words(int32_t n, const int32_t* colours, int32_t ctas, int32_t* words, int32_t room,
+                                            int32_t* ncolours)
+{
+    if (n < 1 || !colours || ctas < 1 || ctas > 16 || room < 0 || (room && !words) || !ncolours)
+        return fail(MQV_ERR_INVALID_ARG, "bad arguments");
+    for (int32_t i = 0; i < n; ++i)
+        if (colours[i] < 0 || colours[i] > 4096) return fail(MQV_ERR_INVALID_ARG, "colour out of range");
+    *ncolours = ell_words(n, colours, ctas, words, room);
     return MQV_OK;
 }
 

@@ -13,7 +13,20 @@
 // each from a lane of its own; its own CTA too).  A warp begins the next colour
 // when all words of this one have arrived, counted by an mbarrier -- which
 // also tells that every other warp has read what is about to change -- so a
-// colour needs no CTA or cluster barrier.  What does not depend on the spins,
+// colour needs no cluster barrier.
+// The initial state is step 0, the colours are steps 1, 2, ...; the words of
+// even steps count at one mbarrier, those of odd steps at the other.  Two rules
+// make that enough:
+//   * every CTA sends at least one word of every step (colours without a site
+//     are left out, a CTA without a site of a colour has a word of padding).
+//     So no word of step t + 2 is sent before step t has ended everywhere:
+//     its sender has the words of step t + 1 of every CTA, each sent after
+//     step t had ended there;
+//   * a CTA barrier comes before every wait.  Thread 0 arms step t + 1 behind
+//     it, so no barrier runs past a thread that still waits for step t - 1, and
+//     no thread waits for step t before thread 0 has armed it: the parity of
+//     the wait is unambiguous.
+// What does not depend on the spins,
 // a site and its neighbours' bits, is fetched ahead.  The neighbour lists lie
 // in slices of 32 positions, one row per neighbour, so that a warp reads them
 // in whole lines; a sweep's acceptance planes are drawn once per CTA for the
@@ -53,6 +66,18 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank)
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
+}
+
+// mbar_try_wait for words that came from other CTAs of the cluster
+__device__ __forceinline__ bool words_arrived(uint32_t bar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
 }
 
 // shared memory: the sweep's rounds, the graph's spins (a bit per position,
@@ -96,8 +121,8 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
     uint32_t* bits = reinterpret_cast<uint32_t*>(rounds + g.rounds);
     uint4* tab = reinterpret_cast<uint4*>(smem + (((size_t)g.rounds * 16 + (size_t)g.npos / 8 + 15) & ~(size_t)15));
     __shared__ int s_rounds;
-    // words of the colours: even ones count at the first barrier, odd ones at
-    // the second (a word of colour k + 1 may come before the last of colour k)
+    // words of even and of odd steps (one of step t + 1 may come before the last
+    // of step t)
     __shared__ __align__(8) uint64_t bars[2];
     const int lo = me * g.range;  // this CTA's sites [lo, lo + range)
     const int32_t* cptr = g.cptr + me * g.ncol;
@@ -106,11 +131,8 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
         int r = 0;
         for (int c = 0; c < g.ncol; ++c) {
             const int end = cptr[c + 1];
-            int p = cptr[c];
-            do {
+            for (int p = cptr[c]; p < end; p += kEllThreads)
                 rounds[r++] = make_int4(p, min(p + kEllThreads, end), p == cptr[c], g.cwords[c] * 4);
-                p += kEllThreads;
-            } while (p < end);
         }
         s_rounds = r;
         mbar_init(smem_addr(&bars[0]), 1);
@@ -123,7 +145,7 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
     const bool sends = lane < ctas;
     const uint32_t to = sends ? map_rank(smem_addr(bits), (uint32_t)lane) : 0u;
     const uint32_t to_bar = sends ? map_rank(smem_addr(&bars[0]), (uint32_t)lane) : 0u;
-    int step = 0;  // colours begun; the words of the initial state are colour 0
+    int step = 0;  // steps begun
     bool stop = false;
     auto arm = [&](int bytes) {
         if (tid == 0) mbar_expect_tx(smem_addr(&bars[step & 1]), (uint32_t)bytes);
@@ -132,14 +154,14 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
     auto send = [&](int word, uint32_t v) {
         if (sends) st_async(to + 4u * (uint32_t)word, v, to_bar + 8u * (uint32_t)((step - 1) & 1));
     };
-    // until every word of the last colour begun has arrived (bounded: a lost
-    // word sets the error status and ends the run)
+    // until every word of the last step begun has arrived, behind a CTA barrier
+    // (bounded: a lost word sets the error status and ends the run)
     auto receive = [&]() {
         if (stop) return;
         const uint32_t bar = smem_addr(&bars[(step - 1) & 1]), par = (uint32_t)((step - 1) >> 1) & 1u;
-        if (mbar_try_wait(bar, par)) return;
+        if (words_arrived(bar, par)) return;
         const uint64_t t0 = global_timer_ns();
-        for (uint32_t k = 1; !mbar_try_wait(bar, par); ++k)
+        for (uint32_t k = 1; !words_arrived(bar, par); ++k)
             if ((k & 255u) == 0 && global_timer_ns() - t0 > R.wait_ns) {
                 stop = true;
                 atomicExch(R.status, MQV_ERR_TIMEOUT);
@@ -215,7 +237,6 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
             for (int q = tid; q < g.range / 16; q += kEllThreads)
                 tab[q] = philox(((uint32_t)(lo >> 6) + ((uint32_t)q >> 2)) * 2u + (((uint32_t)q >> 1) & 1u), sweep,
                                 (uint32_t)q & 1u, c3a, R.key);
-            __syncthreads();
             for (int r = 0; r < nround; ++r) {
                 const EllPos q = cur;
                 const Pre e = pre;
@@ -225,6 +246,7 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
                 next = find_round(ahead);
                 const int4 rd = rounds[r];
                 if (rd.z) {  // a colour begins
+                    __syncthreads();  // also: the sweep's planes are there
                     receive();
                     arm(rd.w);
                 }
@@ -243,6 +265,7 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
         if (stop) break;
         if (!R.acc) continue;
         // measurement: the field of every site of this CTA, all colours
+        __syncthreads();
         receive();
         long long ene = 0;
         int down = 0, p = p0 + tid;
@@ -273,6 +296,7 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
         }
         cl.sync();  // the next sweep's words would arrive while others still read
     }
+    __syncthreads();
     receive();
     for (int p = p0 + tid; p < p1; p += kEllThreads) {
         const int i = g.site[p];
@@ -321,41 +345,69 @@ static int ell_max_ctas(int device)
     return best;
 }
 
+// Positions of a coloured graph on `ctas` CTAs of `range` sites: the site of
+// every position (-1: padding), the positions of every (CTA, colour), at least
+// one word each, and the words of every colour.  Colours without a site are
+// left out, the others keep their order.
+struct EllLayout {
+    int ncol = 0;
+    std::vector<int32_t> site, cptr, cwords;
+};
+static int64_t ell_range(int64_t n, int ctas) { return ((n + ctas - 1) / ctas + 63) / 64 * 64; }
+static EllLayout ell_layout(int64_t n, const int32_t* col, int ctas)
+{
+    EllLayout e;
+    const int64_t range = ell_range(n, ctas);
+    std::vector<int32_t> used;  // colour -> its place among those that have sites
+    for (int64_t i = 0; i < n; ++i) {
+        if ((size_t)col[i] >= used.size()) used.resize((size_t)col[i] + 1, 0);
+        used[(size_t)col[i]] = 1;
+    }
+    for (int32_t& u : used) u = u ? e.ncol++ : -1;
+    e.cptr.assign((size_t)ctas * e.ncol + 1, 0);
+    e.cwords.assign((size_t)e.ncol, 0);
+    e.site.reserve((size_t)n + (size_t)ctas * e.ncol * 32);
+    std::vector<std::vector<int32_t>> bins((size_t)e.ncol);
+    for (int r = 0; r < ctas; ++r) {
+        for (auto& b : bins) b.clear();
+        for (int64_t i = r * range; i < std::min(n, (r + 1) * range); ++i)
+            bins[(size_t)used[(size_t)col[i]]].push_back((int32_t)i);
+        for (int c = 0; c < e.ncol; ++c) {
+            const size_t first = e.site.size();
+            e.site.insert(e.site.end(), bins[(size_t)c].begin(), bins[(size_t)c].end());
+            while (e.site.size() == first || e.site.size() % 32) e.site.push_back(-1);  // a colour starts a slice
+            e.cptr[(size_t)r * e.ncol + c + 1] = (int32_t)e.site.size();
+            e.cwords[(size_t)c] += (int32_t)((e.site.size() - first) / 32);
+        }
+    }
+    return e;
+}
+
 // The sliced neighbour lists of a coloured graph (col: every site's colour),
 // built on the host and uploaded; nothing where the graph does not fit.
 cudaError_t build_ell(Sim* s, int64_t n, const int32_t* rp, const int32_t* ci, const int8_t* bonds,
                       const std::vector<int32_t>& col)
 {
-    const int ncol = (int)s->colour_ptr.size() - 1, most = ell_max_ctas(s->device);
+    const int most = ell_max_ctas(s->device);
+    int ncol = 0;  // colours that have sites
+    for (size_t c = 0; c + 1 < s->colour_ptr.size(); ++c) ncol += s->colour_ptr[c + 1] > s->colour_ptr[c];
     // a CTA per 1024 sites (us per sweep with one per 1024 / 4096 / 8192: 4096
     // sites 12 / 17 / 17, 16,384 sites 12 / 22 / 31)
     int ctas = 1;
     while (ctas < most && n > (int64_t)ctas * 1024) ctas *= 2;
-    const int64_t range64 = ((n + ctas - 1) / ctas + 63) / 64 * 64;
+    const int64_t range64 = ell_range(n, ctas);
     const int64_t most_rounds = ncol + (range64 + 32 * (int64_t)ncol) / kEllThreads + 1;  // colours are padded to 32
     const int64_t most_pos = n + 32 * (int64_t)ncol * ctas;
     if (most_pos >= (int64_t)1 << 31 || range64 * ctas >= (int64_t)1 << 31 || most_rounds > kEllRounds ||
         ell_smem((size_t)most_pos, (int)range64, (int)most_rounds) > kEllMaxSmem)
         return cudaSuccess;
     const int range = (int)range64;
-    std::vector<int32_t> cptr((size_t)ctas * ncol + 1, 0), site, deg;
-    site.reserve((size_t)n + (size_t)ctas * ncol * 32);
-    std::vector<std::vector<int32_t>> bins((size_t)ncol);
-    for (int r = 0; r < ctas; ++r) {
-        for (auto& b : bins) b.clear();
-        for (int64_t i = (int64_t)r * range; i < std::min(n, (int64_t)(r + 1) * range); ++i) bins[(size_t)col[(size_t)i]].push_back((int32_t)i);
-        for (int c = 0; c < ncol; ++c) {
-            site.insert(site.end(), bins[(size_t)c].begin(), bins[(size_t)c].end());
-            while (site.size() % 32) site.push_back(-1);  // a colour starts a slice
-            cptr[(size_t)r * ncol + c + 1] = (int32_t)site.size();
-        }
-    }
+    const EllLayout lay = ell_layout(n, col.data(), ctas);
+    const std::vector<int32_t>&site = lay.site, &cptr = lay.cptr, &cwords = lay.cwords;
+    std::vector<int32_t> deg;
     const size_t np = site.size();
-    // bytes of a colour's words count at one mbarrier: at most 2^20 - 1
-    std::vector<int32_t> cwords((size_t)ncol, 0), pos((size_t)n, 0);
-    for (int r = 0; r < ctas; ++r)
-        for (int c = 0; c < ncol; ++c)
-            cwords[(size_t)c] += (cptr[(size_t)r * ncol + c + 1] - cptr[(size_t)r * ncol + c]) / 32;
+    // bytes of a step's words count at one mbarrier: at most 2^20 - 1
+    std::vector<int32_t> pos((size_t)n, 0);
     if (np / 8 >= (size_t)1 << 20) return cudaSuccess;
     for (size_t p = 0; p < np; ++p)
         if (site[p] >= 0) pos[(size_t)site[p]] = (int32_t)p;
@@ -404,6 +456,19 @@ cudaError_t build_ell(Sim* s, int64_t n, const int32_t* rp, const int32_t* ci, c
     s->ell.rounds = (int)most_rounds;
     s->ell.npos = (int)np;
     return e;
+}
+
+// The words of every colour and CTA (colour by colour) of such a layout, as far
+// as `room` goes; returns the colours that have sites.
+int ell_words(int64_t n, const int32_t* col, int ctas, int32_t* words, int64_t room)
+{
+    const EllLayout e = ell_layout(n, col, ctas);
+    for (int c = 0; c < e.ncol; ++c)
+        for (int r = 0; r < ctas; ++r) {
+            const size_t k = (size_t)r * e.ncol + c;
+            if ((int64_t)c * ctas + r < room) words[(size_t)c * ctas + r] = (e.cptr[k + 1] - e.cptr[k]) / 32;
+        }
+    return e.ncol;
 }
 
 cudaError_t ensure_cuts(Sim* s);
