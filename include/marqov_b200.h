@@ -353,7 +353,9 @@ MQV_API mqv_status mqv_selftest_graph_words(int32_t n, const int32_t* colours, i
 /* Self test of the bounded device waits: the next fused 2D Ising sweep of
  * the handle (band kernel, L = 8192 or 16384) has CTA 0 withhold its staged
  * row `row` (2 .. 64) and waits at most wait_ns for a row, so that the wait
- * for the withheld row runs out.  The kernel then sets MQV_ERR_TIMEOUT,
+ * for the withheld row runs out.  On a graph whose sweeps take one launch
+ * (Ising-type CSR lattices), CTA 0 of that launch withholds a word of the
+ * row-th colour that it sweeps.  The kernel then sets MQV_ERR_TIMEOUT,
  * lets the copies it issued land and returns; the call that reads the
  * device status reports MQV_ERR_TIMEOUT, and the handle refuses compute
  * (MQV_ERR_STATE) until its state is set again.  Nothing faults or hangs:

@@ -1108,8 +1108,9 @@ MQV_API mqv_status mqv_selftest_inject_timeout(mqv_sim* h, int32_t row, uint64_t
 {
     Sim* s = reinterpret_cast<Sim*>(h);
     if (!s) return fail(MQV_ERR_INVALID_ARG, "null handle");
-    if (!s->fused_ising2d || ising2d_band_config(s) < 0)
-        return fail(MQV_ERR_UNSUPPORTED_TERM, "timeout injection needs the fused 2D Ising band path (L = 8192 or 16384)");
+    if (!s->d_ell && (!s->fused_ising2d || ising2d_band_config(s) < 0))
+        return fail(MQV_ERR_UNSUPPORTED_TERM,
+                    "timeout injection needs the fused 2D Ising band path (L = 8192 or 16384) or a graph swept in one launch");
     if (row < 2 || row > 64) return fail(MQV_ERR_INVALID_ARG, "withheld row must be in [2, 64]");
     s->inject_row = row;
     s->inject_wait_ns = wait_ns;

@@ -26,6 +26,13 @@
 //     it, so no barrier runs past a thread that still waits for step t - 1, and
 //     no thread waits for step t before thread 0 has armed it: the parity of
 //     the wait is unambiguous.
+// Waits are bounded.  A thread whose wait ran out sets the error status and
+// waits, sends and arms no more; its CTA learns of it before the next sweep or
+// measurement and skips the rest of the run, the other threads and CTAs run out in
+// turn for want of its words.  Every
+// CTA passes the same cluster barriers whether it runs or skips, and one that
+// gave up stays a while after the last of them, since words of others may still
+// be on their way to it.
 // What does not depend on the spins,
 // a site and its neighbours' bits, is fetched ahead.  The neighbour lists lie
 // in slices of 32 positions, one row per neighbour, so that a warp reads them
@@ -104,6 +111,7 @@ struct EllRun {
     long long* acc;  // measurement accumulators of the first EMCS, or NULL
     int* status;     // device error word
     unsigned long long wait_ns;
+    int hold;        // the colour of the run (from 1) of which CTA 0 withholds a word (tests); 0: none
 };
 
 template <bool BONDS>
@@ -145,14 +153,17 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
     const bool sends = lane < ctas;
     const uint32_t to = sends ? map_rank(smem_addr(bits), (uint32_t)lane) : 0u;
     const uint32_t to_bar = sends ? map_rank(smem_addr(&bars[0]), (uint32_t)lane) : 0u;
-    int step = 0;  // steps begun
-    bool stop = false;
+    int step = 0;       // steps begun
+    bool stop = false;  // a wait of this thread ran out
+    bool over = false;  // ... of this CTA, as of the last meet()
+    auto meet = [&]() { stop = over = __syncthreads_or(stop); };
     auto arm = [&](int bytes) {
-        if (tid == 0) mbar_expect_tx(smem_addr(&bars[step & 1]), (uint32_t)bytes);
+        if (tid == 0 && !stop) mbar_expect_tx(smem_addr(&bars[step & 1]), (uint32_t)bytes);
         ++step;
     };
+    const int hold = R.hold && me == 0 && warp == 0 ? R.hold + 1 : 0;  // the step of the withheld word
     auto send = [&](int word, uint32_t v) {
-        if (sends) st_async(to + 4u * (uint32_t)word, v, to_bar + 8u * (uint32_t)((step - 1) & 1));
+        if (sends && !stop) st_async(to + 4u * (uint32_t)word, v, to_bar + 8u * (uint32_t)((step - 1) & 1));
     };
     // until every word of the last step begun has arrived, behind a CTA barrier
     // (bounded: a lost word sets the error status and ends the run)
@@ -229,11 +240,11 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
     EllPos next = find_round(ahead);
     Pre pre = fetch(cur);
     for (int em = 0; em < R.n_emcs; ++em) {
-        for (int j = 0; j < R.nmetro; ++j) {
+        for (int j = 0; j < R.nmetro && !over; ++j) {
             const uint32_t sweep = R.sweep0 + (uint32_t)(em * R.nmetro + j);
             // the sweep's acceptance planes of this CTA's sites
-            stop = __syncthreads_or(stop);
-            if (stop) break;
+            meet();
+            if (over) break;
             for (int q = tid; q < g.range / 16; q += kEllThreads)
                 tab[q] = philox(((uint32_t)(lo >> 6) + ((uint32_t)q >> 2)) * 2u + (((uint32_t)q >> 1) & 1u), sweep,
                                 (uint32_t)q & 1u, c3a, R.key);
@@ -259,16 +270,15 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
                 }
                 const uint32_t m = __ballot_sync(0xffffffffu, flip);
                 const int word = (rd.x + warp * 32) >> 5;
-                if (rd.x + warp * 32 < rd.y) send(word, bits[word] ^ m);
+                if (rd.x + warp * 32 < rd.y && step != hold) send(word, bits[word] ^ m);
             }
         }
-        if (stop) break;
         if (!R.acc) continue;
         // measurement: the field of every site of this CTA, all colours
-        __syncthreads();
-        receive();
+        meet();
+        if (!over) receive();
         long long ene = 0;
-        int down = 0, p = p0 + tid;
+        int down = 0, p = over ? p1 : p0 + tid;
         EllPos q = find(p, p1), q2 = find(p + kEllThreads, p1);
         Pre e = fetch(q);
         for (; p < p1; p += kEllThreads) {
@@ -296,13 +306,20 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
         }
         cl.sync();  // the next sweep's words would arrive while others still read
     }
-    __syncthreads();
-    receive();
-    for (int p = p0 + tid; p < p1; p += kEllThreads) {
-        const int i = g.site[p];
-        if (i >= 0) R.s[i] = (int8_t)(1 - 2 * minus(p));
+    meet();
+    if (!over) {
+        receive();
+        for (int p = p0 + tid; p < p1; p += kEllThreads) {
+            const int i = g.site[p];
+            if (i >= 0) R.s[i] = (int8_t)(1 - 2 * minus(p));
+        }
     }
     cl.sync();  // no CTA leaves while words are on their way to it or from it
+    if (stop) {
+        // the last words sent are older than the barrier: 20 us are enough for them
+        const uint64_t t0 = global_timer_ns();
+        for (int k = 0; k < 1 << 16 && global_timer_ns() - t0 < 20000; ++k) __nanosleep(200);
+    }
 }
 
 typedef void (*EllKernel)(EllRun);
@@ -494,6 +511,11 @@ cudaError_t launch_ell_emcs(Sim* s, int n_emcs, int nmetro, long long* acc)
     R.acc = acc;
     R.status = s->d_status;
     R.wait_ns = 2000000000ull;  // 2 s
+    if (s->inject_row >= 0) {   // one launch only
+        R.hold = s->inject_row;
+        R.wait_ns = s->inject_wait_ns;
+        s->inject_row = -1;
+    }
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg;
     ell_config(cfg, at, s->ell.ctas, ell_smem((size_t)s->ell.npos, s->ell.range, s->ell.rounds), s->stream);

@@ -299,7 +299,7 @@ struct Sim {
     // a device wait gave up: compute is refused until the state is set again
     bool failed = false;
     int cluster_ok = -1;  // the device co-schedules this lattice's thread-block cluster (-1: not asked yet)
-    // one-shot injected timeout of the next fused band sweep (tests)
+    // one-shot injected timeout of the next fused band sweep or graph launch (tests)
     int inject_row = -1;
     unsigned long long inject_wait_ns = 0;
     // int8 models: u53 cut of every possible dE (int8_cut_table), on the device

@@ -1,6 +1,8 @@
 """One-launch sweeps of graphs whose colours are missing on some CTAs or have no
 site at all (csr_sweep.cu) against one launch per colour, bit for bit, also
-with several handles at work on their own streams."""
+with several handles at work on their own streams.  A wait that is made to run
+out (a word that nobody sends, a limit of 200 us) is reported, and the handle
+runs on from a state that is set again."""
 import threading
 
 import numpy as np
@@ -39,6 +41,36 @@ def test_missing_colours(name):
     lat = graph(name)
     for x, y in zip(chain(lat, False), chain(lat, True)):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("name", ["rgg", "gap"])
+@pytest.mark.parametrize("colour,nm,measure", [(2, 1, True), (2, 4, True), (7, 4, True), (3, 8, False)])
+def test_wait_that_runs_out(name, colour, nm, measure):
+    import marqov_b200 as M
+    from marqov_b200 import _lib
+    lat = graph(name)
+    with M.makeCore(lat, M.Config(seed=8), M.Ising(-1.0, "int8"), 0.4) as c:
+        c.init()
+        s0 = c.state
+        _lib.check(c._lib.mqv_selftest_inject_timeout(c.handle, colour, 200_000))
+        with pytest.raises(M.MarqovError) as ei:
+            if measure:
+                c.emcs(3, 0, nm)
+            else:
+                c.metropolis(nm)
+                c.synchronize()
+        assert ei.value.status == _lib.ERR_TIMEOUT
+        with pytest.raises(M.MarqovError) as ei:
+            c.metropolis(1)
+        assert ei.value.status == _lib.ERR_STATE
+        c.state = s0
+        before = c.counters
+        got = [*c.emcs(2, 0, 1), c.state]
+    with M.makeCore(lat, M.Config(seed=8, per_colour=True), M.Ising(-1.0, "int8"), 0.4) as c:
+        c.state = s0
+        c.counters = before
+        for x, y in zip(got, [*c.emcs(2, 0, 1), c.state]):
+            assert np.array_equal(x, y)
 
 
 def test_handles_side_by_side():
