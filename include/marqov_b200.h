@@ -118,7 +118,8 @@ typedef struct mqv_lattice_desc {
     const int32_t* col_idx;    /* CSR: neighbour ids in nbrs(0,i) order (host, copied) */
     const int8_t* bonds;       /* optional bond weights (bnds), symmetric: CSR, one per col_idx entry;
                                   hypercubic, 2 dim per site in the nbrs(0,i) order +x,-x,+y,-y,...
-                                  (RegularRandomBond), kept on the stencil path */
+                                  (RegularRandomBond), kept on the stencil path.  Weights beyond +-1:
+                                  the |weights| of a site sum to at most 2^24 */
     const int32_t* colours;    /* optional proper colouring; NULL = greedy colouring */
 } mqv_lattice_desc;
 

@@ -33,7 +33,7 @@ __device__ __forceinline__ void batch_site(const BatchRep& R, const Lat& lat, in
                                            int sub, const uint4* tab, uint32_t run0)
 {
     if (F32) f32_site(R.md, lat, (float*)R.s, i, R.key, sweep, R.replica, live, sub, tab, run0);
-    else int8_site(R.md, lat, (int8_t*)R.s, i, R.key, sweep, R.replica, R.cuts, R.D, live, sub, tab, run0);
+    else int8_site(R.md, lat, (int8_t*)R.s, i, R.key, sweep, R.replica, R.cuts, R.nbr_bound, live, sub, tab, run0);
 }
 
 // One colour of a sweep over every member.  Each CTA takes one block of

@@ -19,7 +19,8 @@ struct BatchRep {
     uint32_t* visited;          // Wolff scratch of the member handle
     int32_t* queue;
     const unsigned long long* cuts;  // int8: the member's Metropolis cut table
-    int D;                           // int8: its maximum degree
+    int D;                           // largest degree
+    int nbr_bound;                   // int8: bound of a neighbourhood sum, the middle of the cut table
     int resident;                    // runs in one CTA's shared memory (batch_resident), not in the graphs
     // labelling in bit tiles (wolff_tile.cuh): words per x-line, tiles in y and
     // z, their number (0: the lattice is labelled site by site), scratch

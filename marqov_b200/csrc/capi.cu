@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <limits>
 #include <new>
@@ -194,6 +195,18 @@ constexpr int64_t kEllMaxSites = 262144;
 
 // ---- lattice lowering -----------------------------------------------------------
 
+// The bound of the neighbourhood sums of a lattice whose sites' |bond weights|
+// sum to at most `sum`.  The cut table has two entries per unit of it, so
+// weights beyond +-1 are taken up to kMaxWeightSum.
+constexpr int64_t kMaxWeightSum = (int64_t)1 << 24;
+static mqv_status set_nbr_bound(Sim* s, int64_t sum)
+{
+    if (sum > std::max<int64_t>(kMaxWeightSum, s->max_degree))
+        return fail(MQV_ERR_BAD_DESCRIPTOR, "bond weights of a site sum to more than " + std::to_string(kMaxWeightSum));
+    s->nbr_bound = (int)sum;
+    return MQV_OK;
+}
+
 static mqv_status lower_csr(Sim* s, const mqv_lattice_desc* L)
 {
     const int64_t n = L->n;
@@ -286,11 +299,21 @@ static mqv_status lower_csr(Sim* s, const mqv_lattice_desc* L)
         MQV_CK(cudaMalloc(&s->d_bonds, (size_t)std::max<int64_t>(nnz, 1)));
         MQV_CK(upload_sync(s->stream, s->d_bonds, L->bonds, (size_t)nnz));
     }
+    s->max_degree = s->nbr_bound = maxdeg;
+    if (L->bonds) {
+        int64_t most = 0;
+        for (int64_t i = 0; i < n; ++i) {
+            int64_t sum = 0;
+            for (int32_t p = rp[i]; p < rp[i + 1]; ++p) sum += std::abs((int)L->bonds[p]);
+            most = std::max(most, sum);
+        }
+        const mqv_status st = set_nbr_bound(s, most);
+        if (st) return st;
+    }
     if (!(s->flags & MQV_FLAG_PER_COLOUR) && !s->is_f32 && s->md.kind != MQV_MODEL_POTTS &&
         s->md.kind != MQV_MODEL_BLUME_CAPEL && n <= kEllMaxSites)
         MQV_CK(build_ell(s, n, rp, ci, L->bonds, col));
     s->n = n;
-    s->max_degree = maxdeg;
     s->csr = CSRDev{n, s->d_rp, s->d_ci, s->d_bonds};
     uint64_t h = 1469598103934665603ull;
     auto mix = [&h](const void* p, size_t bytes) {
@@ -321,8 +344,10 @@ static mqv_status lower_stencil_bonds(Sim* s, const int8_t* bonds)
     const int64_t n = s->n;
     const int dim = s->dim, deg = 2 * dim;
     s->bonds_unit = true;
+    int most = 0;
     std::vector<int8_t> fb((size_t)dim * (size_t)n);
-    for (int64_t i = 0; i < n; ++i)
+    for (int64_t i = 0; i < n; ++i) {
+        int sum = 0;
         for (int d = 0; d < dim; ++d) {
             const int8_t w = bonds[(size_t)i * deg + 2 * d];
             const int64_t j = s->sten.nbr(i, 2 * d);
@@ -330,7 +355,12 @@ static mqv_status lower_stencil_bonds(Sim* s, const int8_t* bonds)
                 return fail(MQV_ERR_BAD_DESCRIPTOR, "hypercubic bonds are not symmetric at site " + std::to_string(i));
             fb[(size_t)d * n + i] = w;
             s->bonds_unit &= w == 1 || w == -1;
+            sum += std::abs((int)w) + std::abs((int)bonds[(size_t)i * deg + 2 * d + 1]);
         }
+        most = std::max(most, sum);
+    }
+    const mqv_status st = set_nbr_bound(s, most);
+    if (st) return st;
     MQV_CK(cudaMalloc(&s->d_bonds, fb.size()));
     MQV_CK(upload_sync(s->stream, s->d_bonds, fb.data(), fb.size()));
     s->sten.fb = s->d_bonds;
@@ -639,7 +669,7 @@ MQV_API mqv_status mqv_create(const mqv_model_desc* model, const mqv_lattice_des
         for (int b = 0; b < 31; ++b)
             if ((1 << b) == lattice->len) s->sten.lg = b;
         s->sten.mlen = s->sten.lg >= 0 ? 0 : UINT64_MAX / (uint64_t)lattice->len + 1;
-        s->max_degree = 2 * lattice->dim;
+        s->max_degree = s->nbr_bound = 2 * lattice->dim;
         s->colour_ptr = {0, (int32_t)(n / 2), (int32_t)n};
         if (lattice->bonds) {
             st = lower_stencil_bonds(s, lattice->bonds);
@@ -1398,6 +1428,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         r.queue = s->d_queue;
         r.cuts = s->d_cuts;
         r.D = s->max_degree;
+        r.nbr_bound = s->nbr_bound;
         r.resident = b->resident[(size_t)i] ? 1 : 0;
         if (b->d_tile && !b->resident[(size_t)i]) {
             const TileShape ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile.units);

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                         const int64_t t = t0 + k * 32 + lane;
                         const bool live = t < t_hi;
                         int8_site(B.md, lst, ds, live ? parity_site(lst, t, colour) : 0, B.key, sweep, B.replica,
-                                  B.cuts, B.D, live, colour, tab, run0);
+                                  B.cuts, B.nbr_bound, live, colour, tab, run0);
                     }
                 }
                 cl.sync();

@@ -106,7 +106,7 @@ struct EllRun {
     int8_t* s;
     Key key;
     uint32_t sweep0, replica;
-    int n_emcs, nmetro, D;
+    int n_emcs, nmetro, D;  // D: middle of the cut table
     const unsigned long long* cuts;
     long long* acc;  // measurement accumulators of the first EMCS, or NULL
     int* status;     // device error word
@@ -506,7 +506,7 @@ cudaError_t launch_ell_emcs(Sim* s, int n_emcs, int nmetro, long long* acc)
     R.replica = s->replica;
     R.n_emcs = n_emcs;
     R.nmetro = nmetro;
-    R.D = s->max_degree;
+    R.D = s->nbr_bound;
     R.cuts = s->d_cuts;
     R.acc = acc;
     R.status = s->d_status;

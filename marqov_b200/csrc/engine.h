@@ -221,8 +221,9 @@ constexpr int kWolffCapF = kWolffSmem / 24;
 MQV_HD int wolff_lanes(const StencilDev& st, int) { return 2 * st.dim; }
 MQV_HD int wolff_lanes(const CSRDev&, int max_degree) { return max_degree < 1 ? 1 : max_degree > 8 ? 8 : max_degree; }
 
-// u53 cuts of an int8 model's Metropolis moves for lattices of maximum degree
-// D, indexed as int8_site computes its dE index (host side).
+// u53 cuts of an int8 model's Metropolis moves, indexed as int8_site computes its
+// dE index (host side).  D bounds a neighbourhood sum: the largest degree, with
+// bonds the largest sum of a site's |weights|.
 std::vector<unsigned long long> int8_cut_table(const ModelDev& md, int D);
 // Activation rule of an int8 model (host side, wolff.cu).
 WolffDev wolff_int8_params(const ModelDev& md);
@@ -272,6 +273,7 @@ struct Sim {
     int8_t* d_bonds = nullptr;
     bool bonds_unit = false;  // stencil bonds are all +-1
     int max_degree = 0;
+    int nbr_bound = 0;  // largest |neighbourhood sum|: max_degree, with bonds the largest sum of a site's |weights|
     EllDev ell{};                     // CSR, Ising-type: for chunks of EMCS in one launch
     void* d_ell = nullptr;
     uint64_t lat_hash = 0;            // CSR: FNV-1a of row_ptr, col_idx and bonds

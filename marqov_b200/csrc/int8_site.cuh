@@ -10,8 +10,8 @@ namespace mqv {
 // ---------------------------------------------------------------------------
 // generic per-site update (Metropolis<H,L>::move, src/libmarqov/metropolis.h:88-126)
 
-// `cuts`: the u53 cut of every dE the model can produce, indexed as
-// int8_cut_index (host table int8_cut_table); the decision equals
+// `cuts`: the u53 cut of every dE the model can produce (host table
+// int8_cut_table), D the bound of a neighbourhood sum that it was made for; the decision equals
 // update_accepted<1>(dE, beta, word) on the site's acceptance word.  `sub`:
 // the site's sublattice (checkerboard colour) where the lattice has a
 // termselector.  Lanes with live == false touch no memory.

@@ -103,7 +103,7 @@ cudaError_t ensure_cuts(Sim* s)
 {
     const double key[7] = {s->md.J, s->md.h, s->md.k, s->md.beta, (double)s->md.kind, s->md.h2, (double)s->md.termsel};
     if (s->d_cuts && std::equal(key, key + 7, s->cuts_for)) return cudaSuccess;
-    const std::vector<unsigned long long> t = int8_cut_table(s->md, s->max_degree);
+    const std::vector<unsigned long long> t = int8_cut_table(s->md, s->nbr_bound);
     if ((int)t.size() > s->n_cuts) {
         if (s->d_cuts) cudaFree(s->d_cuts);
         s->d_cuts = nullptr;
@@ -229,7 +229,7 @@ cudaError_t launch_metropolis_int8(Sim* s, int slot)
                 continue;
             }
             metro_int8_stencil<<<g, kMetroThreads, 0, s->stream>>>(s->md, s->sten, st, c, key, (uint32_t)s->sweep,
-                                                                   s->replica, s->d_cuts, s->max_degree);
+                                                                   s->replica, s->d_cuts, s->nbr_bound);
             s->launches++;
         }
     } else {
@@ -238,7 +238,7 @@ cudaError_t launch_metropolis_int8(Sim* s, int slot)
             if (cnt == 0) continue;
             metro_int8_csr<<<grid_for(cnt, 256), 256, 0, s->stream>>>(s->md, s->csr, st, s->d_order, b, cnt, key,
                                                                        (uint32_t)s->sweep, s->replica, s->d_cuts,
-                                                                       s->max_degree);
+                                                                       s->nbr_bound);
             s->launches++;
         }
     }

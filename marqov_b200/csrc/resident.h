@@ -11,7 +11,7 @@ struct ResidentRun {
     WolffDev w;
     Key key;
     uint32_t replica, sweep0, cluster0;  // counters of the chunk's first EMCS
-    int n_emcs, ncluster, nmetro, D, runs;
+    int n_emcs, ncluster, nmetro, D, runs;  // D: middle of the cut table
     const unsigned long long* cuts;
     int8_t* state;      // global state, read at the start and written at the end
     long long* acc;     // measurement accumulators of the first EMCS (zeroed), or NULL
@@ -38,7 +38,7 @@ __device__ __forceinline__ void resident_member(ResidentRun& R, const BatchRep& 
     R.n_emcs = count;
     R.ncluster = ncluster;
     R.nmetro = nmetro;
-    R.D = B.D;
+    R.D = B.nbr_bound;
     R.cuts = B.cuts;
     R.state = (int8_t*)B.s;
     R.acc = acc + ((size_t)slot0 * nrep + r) * kAccStride;

@@ -693,7 +693,7 @@ cudaError_t launch_emcs_resident(Sim* s, int n_emcs, int ncluster, int nmetro, b
     R.n_emcs = n_emcs;
     R.ncluster = ncluster;
     R.nmetro = nmetro;
-    R.D = s->max_degree;
+    R.D = s->nbr_bound;
     R.runs = resident_runs(s->n);
     R.cuts = s->d_cuts;
     R.state = (int8_t*)s->state[s->cur];

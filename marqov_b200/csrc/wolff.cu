@@ -120,6 +120,7 @@ static BatchRep single_rep(const Sim* s)
     r.queue = s->d_queue;
     r.cuts = s->d_cuts;
     r.D = s->max_degree;
+    r.nbr_bound = s->nbr_bound;
     if (s->d_tile) tile_bind(r, tile_shape(s->lat_kind, s->dim, s->len, s->tile_units), s->tile_units, s->d_tile);
     return r;
 }
