@@ -132,7 +132,9 @@ enum {
                                  per cluster, colour and measurement instead (same results) */
     MQV_FLAG_RESIDENT = 4     /* take the resident path wherever the lattice fits it.  Default (neither
                                  flag): a single handle is resident up to 16384 sites, Ising-type 2D and
-                                 3D lattices (held as bit planes; bonds +-1) up to 32768 sites; these
+                                 3D lattices (held as bit planes; bonds +-1) up to 32768 sites (with
+                                 clusters as far as these fit one CTA's shared memory, which 2D
+                                 sides of 176 to 180 do not); these
                                  are resident in a batch too (spin glasses up to 65536 sites), the
                                  batch's other members run on its graph path */
 };

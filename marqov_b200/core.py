@@ -44,7 +44,8 @@ class Config:
     # int8 stencil lattices of <= 65536 sites (one CTA) or <= 262144 sites (a
     # thread-block cluster) can run whole chunks of EMCS in shared memory.
     # None: the engine decides (single handles up to 16384 sites, Ising-type
-    # lattices, which are held as bit planes, up to 32768 sites, also in a
+    # lattices, which are held as bit planes, up to 32768 sites -- 2D sides of
+    # 176 to 180 only without clusters -- also in a
     # batch, whose other members take its graph path); True: wherever the lattice fits;
     # False: never (launch per step).  The results are the same.
     resident: bool | None = None

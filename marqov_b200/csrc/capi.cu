@@ -1104,7 +1104,7 @@ MQV_API mqv_status mqv_describe(mqv_sim* h, char* buf, size_t len)
     // the sweep kernel's name, when there is one, ends the line
     std::snprintf(buf, len, "model=%d lattice=%s n=%lld clusters=%s path=%s%s%s", s->md.kind,
                   s->lat_kind == MQV_LATTICE_HYPERCUBIC ? (s->termsel ? "bipartite" : "hypercubic") : "csr", (long long)s->n,
-                  use_resident(s, 0) ? "label-smem" : use_cluster(s) ? "label-dsmem" : (cluster_by_label(s) ? "label" : "bfs"),
+                  use_resident(s, 1) ? "label-smem" : use_cluster(s) ? "label-dsmem" : (cluster_by_label(s) ? "label" : "bfs"),
                   use_resident(s, 0) ? "resident-smem"
                   : use_cluster(s) ? "resident-cluster"
                                    : (s->fused_ising2d ? "fused-2d-bitsliced" : (s->is_f32 ? "per-colour-f32" : "per-colour-int8")),
