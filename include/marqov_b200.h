@@ -134,9 +134,11 @@ enum {
                                  flag): a single handle is resident up to 16384 sites, Ising-type 2D and
                                  3D lattices (held as bit planes; bonds +-1) up to 32768 sites (with
                                  clusters as far as these fit one CTA's shared memory, which 2D
-                                 sides of 176 to 180 do not); these
-                                 are resident in a batch too (spin glasses up to 65536 sites), the
-                                 batch's other members run on its graph path */
+                                 sides of 176 to 180 do not, and as far as launches do not label
+                                 them faster: 3D side 32); these
+                                 are resident in a batch too (spin glasses up to 65536 sites), but
+                                 for few large members, and the batch's other members run on its
+                                 graph path */
 };
 
 typedef struct mqv_run_params {

@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(kBatchMetroThreads)
     if (g0 >= total) return;  // whole CTAs
     const int r = block_rep[blockIdx.x];
     const BatchRep& R = reps[r];
+    if (R.resident) return;  // on the graph path in other runs
     const int64_t t0 = g0 - prefix[r];
     const int64_t cnt = ccount[(size_t)r * ncol + colour];
     const uint32_t sweep = R.sweep0 + (ctr->e + e_off) * (uint32_t)nmetro + (uint32_t)j;
@@ -150,6 +151,7 @@ __global__ void batch_measure(const BatchRep* __restrict__ reps, const BatchCtr*
     const int r = meas_rep[blockIdx.x];
     const int part = (int)blockIdx.x - meas_prefix[r], nparts = meas_prefix[r + 1] - meas_prefix[r];
     const BatchRep& R = reps[r];
+    if (R.resident) return;  // on the graph path in other runs
     const uint32_t slot = ctr->e + e_off - ctr->ebase;
     long long* a = acc + ((size_t)slot * nrep + r) * kAccStride;
     if (F32) {

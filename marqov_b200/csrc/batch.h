@@ -21,7 +21,7 @@ struct BatchRep {
     const unsigned long long* cuts;  // int8: the member's Metropolis cut table
     int D;                           // largest degree
     int nbr_bound;                   // int8: bound of a neighbourhood sum, the middle of the cut table
-    int resident;                    // runs in one CTA's shared memory (batch_resident), not in the graphs
+    int resident;                    // this run's EMCS are done elsewhere (batch_resident, batch_bits, ...), not in the graphs
     // labelling in bit tiles (wolff_tile.cuh): words per x-line, tiles in y and
     // z, their number (0: the lattice is labelled site by site), scratch
     int tl_nw, tl_ny, tl_nz, tl_tiles;

@@ -524,18 +524,38 @@ static mqv_status check_wolff_supported(Sim* s)
 // spread a sweep over every SM, win (L = 256: 678 against 646 us).
 constexpr int64_t kResidentAutoSites = 16384;
 // Ising-type lattices are held as bit planes (bits_emcs.cu) up to this many
-// sites.  Per EMCS of one cluster and one sweep, beside the launches (us): 2D
-// L = 64 13 against 127 (the per-site resident kernel: 24.6), L = 128 31
-// against 310, L = 160 52 against 50 by labelling; 3D L = 32 62 against 45;
-// sweep and measurement alone at 3D L = 32: 6.8 against 12.5.  In a batch the
-// launches of members without clusters (spin glasses) lose up to the size that
-// fits (32 x L = 32: 9 against 42 us per EMCS).
+// sites, but for clusters of handles that the launches would label.  Per EMCS of
+// one cluster and one sweep, beside the launches (us): 2D L = 64 13 against 129
+// (the per-site resident kernel: 24.6), L = 128 30 against 291, L = 174 61
+// against 434, 3D L = 30 54 against 66 breadth first; 3D L = 32 61 against 43
+// labelled.  Sweep and measurement alone: 2D L = 128 4.1 against 4.2, L = 174 8.1
+// against 12.6, 3D L = 32 6.9 against 12.6.
 constexpr int64_t kBitsAutoSites = 32768;
+
+// A batch holds the same lattices as bit planes, one CTA per member however many
+// there are, where its launches spread few members over all SMs.  Launches are
+// taken (members that ask for residency apart) for the clusters of members of
+// more than kBitsFewWords words while these have at most kBitsWordsPer (words of
+// the largest - kBitsFewWords) words in all, and for spin glasses of more than
+// kGlassFewWords while these have at most kGlassWords in all.  Per EMCS, bit planes
+// and launches (us), a cluster and a sweep: 2D L = 128 (512 words) x 1 30 and 35;
+// 3D L = 24 (576) x 1 39.8 and 39.6, x 4 40 and 43; L = 28 (784) x 12 51.5 and 51.7,
+// x 16 52 and 54; 2D L = 160 (800) x 1 50 and 37, x 12 53 and 46, x 16 53 and 49,
+// x 24 53 and 60; 3D L = 32 (1024) x 1 62 and 41, x 16 65 and 59, x 20 65 and 66;
+// 2D L = 174 (1044) x 20 66 and 60, x 28 66 and 71.  Spin glasses, a sweep: 3D L =
+// 34 (2312) x 1 13.7 and 13.8; L = 40 (3200) x 1 17.6 and 13.7, x 4 17.6 and 15.0,
+// x 6 17.7 and 17.2, x 8 17.7 and 19.3.
+constexpr int64_t kBitsFewWords = 560, kBitsWordsPer = 46, kGlassFewWords = 2500, kGlassWords = 18000;
+static int64_t bit_words(const Sim* s) { return s->n / s->len * ((s->len + 31) / 32); }
+
 // EMCS of this handle run on the resident path (smem_emcs.cu, bits_emcs.cu)?
 static bool use_resident(const Sim* s, int ncluster)
 {
     if ((s->flags & MQV_FLAG_NO_RESIDENT) || s->n > kResidentMaxSites) return false;
-    if (s->n <= kBitsAutoSites && bits_fits(s, ncluster > 0)) return true;
+    if (s->n <= kBitsAutoSites && bits_fits(s, ncluster > 0)) {
+        const bool labelled = ncluster > 0 && s->n >= kLabelMinTiled && cluster_by_label(s);
+        if (!labelled || (s->flags & MQV_FLAG_RESIDENT)) return true;
+    }
     return resident_fits(s) && ((s->flags & MQV_FLAG_RESIDENT) || s->n <= kResidentAutoSites);
 }
 // ... or on a thread-block cluster (cluster_emcs.cu), for int8 stencils of
@@ -1226,17 +1246,20 @@ struct Batch {
     int32_t* d_block_rep = nullptr;
     int32_t* d_cbegin = nullptr;
     int32_t* d_ccount = nullptr;
-    // members run by batch_resident (one CTA each, state in shared memory):
-    // two classes by size (<= kResSmall sites: several CTAs per SM), each
-    // listed largest first; resident[r] marks them
-    std::vector<char> resident;
+    // Where every member runs, [0] in runs without clusters, [1] with: 0 the graph
+    // path, 1 batch_resident (one CTA each, state in shared memory), 2 a
+    // thread-block cluster, 3 as bit planes (batch_bits).  The tables of the graph
+    // path hold every member that runs there in either.
+    std::vector<char> path[2];
+    // batch_resident's members in two classes by size (<= kResSmall sites: several
+    // CTAs per SM), and the bit planes' members, each at a place of d_res_order,
+    // largest first, with the dynamic shared memory of its largest layout
+    struct Group {
+        int count = 0, off = 0;
+        size_t smem = 0;
+    };
+    Group res[2][2], bits[2];  // [with clusters]
     int32_t* d_res_order = nullptr;
-    int nres[2] = {0, 0};
-    size_t res_smem[2] = {0, 0};  // dynamic shared memory of each class (its largest layout)
-    // Ising-type members held as bit planes (batch_bits): nbits of them at
-    // d_res_order + bits_off, shared memory without and with clusters
-    int nbits = 0, bits_off = 0;
-    size_t bits_smem[2] = {0, 0};
     // members held by thread-block clusters of c CTAs (c = 2 .. 8): ncl[c]
     // of them at d_res_order + cl_off[c]
     int ncl[9] = {};
@@ -1389,6 +1412,8 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
                             double* d_samples, const TemperRun* pt = nullptr)
 {
     DeviceGuard guard_(b->device);
+    const std::vector<char>& path = b->path[ncluster > 0];
+    const Batch::Group *res = b->res[ncluster > 0], &bits = b->bits[ncluster > 0];
     if (n_emcs < 0 || ncluster < 0 || nmetro < 0) return fail(MQV_ERR_INVALID_ARG, "negative count");
     if (ncluster > 64 || nmetro > 64) return fail(MQV_ERR_INVALID_ARG, "at most 64 clusters and 64 sweeps per EMCS");
     for (Sim* s : b->sims) {
@@ -1402,7 +1427,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     }
     if (ncluster > 0)
         for (int i = 0; i < b->nrep; ++i) {
-            if (b->resident[(size_t)i]) continue;
+            if (path[(size_t)i]) continue;
             const mqv_status st = ensure_wolff(b->sims[(size_t)i]);
             if (st) return st;
         }
@@ -1429,8 +1454,8 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         r.cuts = s->d_cuts;
         r.D = s->max_degree;
         r.nbr_bound = s->nbr_bound;
-        r.resident = b->resident[(size_t)i] ? 1 : 0;
-        if (b->d_tile && !b->resident[(size_t)i]) {
+        r.resident = path[(size_t)i] ? 1 : 0;
+        if (b->d_tile && !b->path[1][(size_t)i]) {
             const TileShape ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile.units);
             if (ts.n) tile_bind(r, ts, b->L.tile.units, (char*)b->d_tile + b->tile_off[(size_t)i]);
         }
@@ -1456,7 +1481,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     // are short while the choice is by timing: a hot start's clusters, and with
     // them the cost of growing them, change within a few dozen EMCS.
     bool graph = false;  // members on the graph path
-    for (char r : b->resident) graph |= r == 0;
+    for (char p : path) graph |= p == 0;
     const bool adapt = b->wolff_mode == MQV_WOLFF_AUTO && ncluster > 0 && graph;
     const int fixed = b->wolff_mode == MQV_WOLFF_LABEL ? 1 : 0;
     const int max_chunk = adapt ? 64 : CH;
@@ -1494,9 +1519,9 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         per_emcs[w] = batch_launches_per_emcs(l, ncluster, nmetro);
     }
     // side streams of the resident classes and cluster sizes (created once)
-    int nside_needed = (b->nres[0] ? 1 : 0) + (b->nres[1] ? 1 : 0) + (b->nbits ? 1 : 0);
+    int nside_needed = (res[0].count ? 1 : 0) + (res[1].count ? 1 : 0) + (bits.count ? 1 : 0);
     for (int c = 2; c <= 8; ++c) nside_needed += b->ncl[c] ? 1 : 0;
-    const bool inline_bits = b->nbits == b->nrep;  // nothing to run beside them
+    const bool inline_bits = bits.count == b->nrep;  // nothing to run beside them
     if (nside_needed && !inline_bits && !b->fork_ev) {
         MQV_CK(cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming));
         for (int i = 0; i < Batch::kSide; ++i) {
@@ -1510,7 +1535,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     auto launch_emcs = [&](int w, int count, int k0) -> mqv_status {
         int nside = 0;
         if (inline_bits) {
-            MQV_CK(batch_launch_bits(b->L, b->stream, b->d_res_order + b->bits_off, b->nbits, b->bits_smem[ncluster > 0],
+            MQV_CK(batch_launch_bits(b->L, b->stream, b->d_res_order + bits.off, bits.count, bits.smem,
                                      (uint32_t)(done_run + k0), k0, count, ncluster, nmetro, b->device));
             b->launches++;
             return MQV_OK;
@@ -1527,19 +1552,19 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
             return e;
         };
         for (int cls = 0; cls < 2; ++cls) {
-            if (!b->nres[cls]) continue;
+            if (!res[cls].count) continue;
             cudaStream_t st2 = nullptr;
             MQV_CK(side_stream(st2));
-            MQV_CK(batch_launch_resident(b->L, st2, b->d_res_order + (cls ? b->nres[0] : 0), b->nres[cls],
-                                         b->res_smem[cls], (uint32_t)(done_run + k0), k0, count, ncluster, nmetro,
+            MQV_CK(batch_launch_resident(b->L, st2, b->d_res_order + res[cls].off, res[cls].count,
+                                         res[cls].smem, (uint32_t)(done_run + k0), k0, count, ncluster, nmetro,
                                          b->device));
             MQV_CK(side_done(st2));
             b->launches++;
         }
-        if (b->nbits) {
+        if (bits.count) {
             cudaStream_t st2 = nullptr;
             MQV_CK(side_stream(st2));
-            MQV_CK(batch_launch_bits(b->L, st2, b->d_res_order + b->bits_off, b->nbits, b->bits_smem[ncluster > 0],
+            MQV_CK(batch_launch_bits(b->L, st2, b->d_res_order + bits.off, bits.count, bits.smem,
                                      (uint32_t)(done_run + k0), k0, count, ncluster, nmetro, b->device));
             MQV_CK(side_done(st2));
             b->launches++;
@@ -1747,62 +1772,84 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         st = mqv_set_stream(h, b->stream);
         if (st) return bail(st);
     }
-    // resident members: int8 stencil lattices that fit one CTA's shared
-    // memory (or a thread-block cluster's) and whose spec asks for it
-    b->resident.assign((size_t)n, 0);
-    std::vector<int32_t> res_order[2], cl_order[9], bits_order;
+    // Ising-type members as bit planes: one SM then advances a lattice faster
+    // than its share of the launches of the graph path, unless they are few
+    // (kBitsFewWords)
+    auto flags = [&](int r) { return specs[r].params.flags; };
+    auto glass = [&](int r) { return b->sims[(size_t)r]->md.kind == MQV_MODEL_EA; };
+    for (int c = 0; c < 2; ++c) {
+        b->path[c].assign((size_t)n, 0);
+        int64_t words[2] = {0, 0}, largest = 0;  // few large members: of clusters, of spin glasses
+        auto few = [&](int r) {
+            return !(flags(r) & MQV_FLAG_RESIDENT) &&
+                   (glass(r) ? bit_words(b->sims[(size_t)r]) > kGlassFewWords
+                             : c == 1 && bit_words(b->sims[(size_t)r]) > kBitsFewWords);
+        };
+        for (int r = 0; r < n; ++r) {
+            const Sim* s = b->sims[(size_t)r];
+            if ((flags(r) & MQV_FLAG_NO_RESIDENT) || s->n > (glass(r) ? kResidentMaxSites : kBitsAutoSites) ||
+                !bits_fits(s, c == 1 && !glass(r)))
+                continue;
+            b->path[c][(size_t)r] = 3;
+            if (!few(r)) continue;
+            words[glass(r)] += bit_words(s);
+            if (!glass(r)) largest = std::max(largest, bit_words(s));
+        }
+        const bool launches[2] = {words[0] <= kBitsWordsPer * (largest - kBitsFewWords), words[1] <= kGlassWords};
+        for (int r = 0; r < n; ++r)
+            if (b->path[c][(size_t)r] == 3 && few(r) && launches[glass(r)]) b->path[c][(size_t)r] = 0;
+    }
+    // Other resident members: int8 stencil lattices that fit one CTA's shared
+    // memory or a thread-block cluster's.  Such a member runs on one CTA (or one
+    // cluster) for a whole chunk of EMCS, which leaves it at the speed of one SM (or
+    // a few): the graph path, whose launches spread every member over all SMs, is
+    // the default (the 256-replica Potts farm: 1.8 against 3.4 ms per EMCS); members
+    // that ask for it (MQV_FLAG_RESIDENT) stay resident.
+    std::vector<int32_t> res_order[2][2], bits_order[2], cl_order[9];
     bool cl_ok[9] = {}, cl_asked = false;
     for (int r = 0; r < n; ++r) {
         const Sim* s = b->sims[(size_t)r];
-        // Ising-type members as bit planes: one SM then advances a lattice
-        // faster than its share of the launches of the graph path
-        if (!(specs[r].params.flags & MQV_FLAG_NO_RESIDENT) &&
-            s->n <= (s->md.kind == MQV_MODEL_EA ? kResidentMaxSites : kBitsAutoSites) && bits_fits(s, s->md.kind != MQV_MODEL_EA)) {
-            b->resident[(size_t)r] = 3;
-            bits_order.push_back(r);
-            for (int c = 0; c < 2; ++c) b->bits_smem[c] = std::max(b->bits_smem[c], bits_smem(s, c && s->md.kind != MQV_MODEL_EA));
-            continue;
+        const bool asked = flags(r) & MQV_FLAG_RESIDENT;
+        for (int c = 0; c < 2; ++c) {
+            char& p = b->path[c][(size_t)r];
+            if (p == 3) bits_order[c].push_back(r);
+            else if (asked && resident_fits(s)) {
+                p = 1;
+                res_order[c][s->n > kResSmall ? 1 : 0].push_back(r);
+            }
         }
-        // A resident member runs on one CTA (or one cluster) for a whole chunk
-        // of EMCS, which leaves it at the speed of one SM (or a few): the
-        // graph path, whose launches spread every member over all SMs, is the
-        // default (the 256-replica Potts farm: 1.8 against 3.4 ms per EMCS);
-        // members that ask for it (MQV_FLAG_RESIDENT) stay resident.
-        if (!(specs[r].params.flags & MQV_FLAG_RESIDENT)) continue;
-        if (resident_fits(s)) {
-            b->resident[(size_t)r] = 1;
-            res_order[s->n > kResSmall ? 1 : 0].push_back(r);
-        } else if (!s->is_f32 && s->lat_kind == MQV_LATTICE_HYPERCUBIC) {
+        if (asked && !s->is_f32 && s->lat_kind == MQV_LATTICE_HYPERCUBIC && !b->path[0][(size_t)r] && !b->path[1][(size_t)r]) {
             const int c = cluster_ctas(s->n);
             if (!cl_asked)
                 for (int k = 2; k <= 8; ++k) cl_ok[k] = cluster_launchable(k);
             cl_asked = true;
             if (c >= 2 && cl_ok[c]) {
-                b->resident[(size_t)r] = 2;
+                b->path[0][(size_t)r] = b->path[1][(size_t)r] = 2;
                 cl_order[c].push_back(r);
             }
         }
     }
-
-    for (int k = 0; k < 2; ++k) {
-        std::stable_sort(res_order[k].begin(), res_order[k].end(),
+    std::vector<int32_t> res_all;
+    auto place = [&](std::vector<int32_t>& order, Batch::Group& g, auto&& smem) {
+        std::stable_sort(order.begin(), order.end(),
                          [&](int32_t x, int32_t y) { return b->sims[(size_t)x]->n > b->sims[(size_t)y]->n; });
-        b->nres[k] = (int)res_order[k].size();
-        b->res_smem[k] = 0;
-        for (int32_t r : res_order[k]) b->res_smem[k] = std::max(b->res_smem[k], resident_smem_for(b->sims[(size_t)r]->sten));
+        g.count = (int)order.size();
+        g.off = (int)res_all.size();
+        for (int32_t r : order) g.smem = std::max(g.smem, smem(b->sims[(size_t)r]));
+        res_all.insert(res_all.end(), order.begin(), order.end());
+    };
+    for (int c = 0; c < 2; ++c) {
+        for (int k = 0; k < 2; ++k)
+            place(res_order[c][k], b->res[c][k], [](const Sim* s) { return resident_smem_for(s->sten); });
+        place(bits_order[c], b->bits[c],
+              [c](const Sim* s) { return bits_smem(s, c == 1 && s->md.kind != MQV_MODEL_EA); });
     }
-    std::vector<int32_t> res_all(res_order[0]);
-    res_all.insert(res_all.end(), res_order[1].begin(), res_order[1].end());
     for (int c = 2; c <= 8; ++c) {
         b->cl_off[c] = (int)res_all.size();
         b->ncl[c] = (int)cl_order[c].size();
         res_all.insert(res_all.end(), cl_order[c].begin(), cl_order[c].end());
     }
-    std::stable_sort(bits_order.begin(), bits_order.end(),
-                     [&](int32_t x, int32_t y) { return b->sims[(size_t)x]->n > b->sims[(size_t)y]->n; });
-    b->nbits = (int)bits_order.size();
-    b->bits_off = (int)res_all.size();
-    res_all.insert(res_all.end(), bits_order.begin(), bits_order.end());
+    auto on_graph = [&](int r) { return !b->path[0][(size_t)r] || !b->path[1][(size_t)r]; };
     // per-colour work: colour c concatenates every graph member's colour-c
     // sites (resident members contribute none), each member's count padded
     // to whole blocks of kAccSites, so that a CTA's block lies in one member
@@ -1824,7 +1871,7 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
                 cnt = s->colour_ptr[(size_t)c + 1] - s->colour_ptr[(size_t)c];
                 cbegin[(size_t)r * ncol + c] = s->colour_ptr[(size_t)c];
             }
-            if (b->resident[(size_t)r]) cnt = 0;
+            if (!on_graph(r)) cnt = 0;
             ccount[(size_t)r * ncol + c] = (int32_t)cnt;
             pf[r + 1] = pf[r] + (cnt + kAccSites - 1) / kAccSites * kAccSites;
         }
@@ -1845,7 +1892,7 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     int64_t units = 0;
     for (int r = 0; r < n; ++r) {
         const Sim* s = b->sims[(size_t)r];
-        if (!b->resident[(size_t)r] && tile_shape(s->lat_kind, s->dim, s->len, 64).n) units += tile_lattice_units(s->dim, s->len);
+        if (!b->path[1][(size_t)r] && tile_shape(s->lat_kind, s->dim, s->len, 64).n) units += tile_lattice_units(s->dim, s->len);
     }
     b->L.tile = tile_config(units);
     std::vector<int32_t> tprefix((size_t)n + 1, 0), trep;
@@ -1854,13 +1901,13 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     for (int r = 0; r < n; ++r) {
         const Sim* s = b->sims[(size_t)r];
         TileShape ts;
-        if (!b->resident[(size_t)r]) ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile.units);
+        if (!b->path[1][(size_t)r]) ts = tile_shape(s->lat_kind, s->dim, s->len, b->L.tile.units);
         if ((int64_t)tprefix[(size_t)r] + ts.n >= (int64_t)1 << 31) return bail(fail(MQV_ERR_INVALID_ARG, "batch too large"));
         tprefix[(size_t)r + 1] = tprefix[(size_t)r] + ts.n;
         trep.insert(trep.end(), (size_t)ts.n, (int32_t)r);
         b->tile_off[(size_t)r] = b->tile_bytes;
         b->tile_bytes += (ts.bytes(b->L.tile.units) + 255) / 256 * 256;
-        sprefix[r + 1] = sprefix[r] + (b->resident[(size_t)r] || ts.n ? 0 : s->n);
+        sprefix[r + 1] = sprefix[r] + (b->path[1][(size_t)r] || ts.n ? 0 : s->n);
     }
     b->L.tiles = (int)trep.size();
     if (trep.empty()) trep.push_back(0);
@@ -1883,18 +1930,18 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     // least one per member
     int64_t msites = 0;
     for (int r = 0; r < n; ++r)
-        if (!b->resident[(size_t)r]) msites += b->sims[(size_t)r]->n;
+        if (on_graph(r)) msites += b->sims[(size_t)r]->n;
     b->L.potts_octets = b->f32 ? 0 : 1;
     for (int r = 0; r < n; ++r) {
         const Sim* s = b->sims[(size_t)r];
-        if (!b->resident[(size_t)r] && !(s->lat_kind == MQV_LATTICE_HYPERCUBIC && potts_octets(s->md, s->sten)))
+        if (on_graph(r) && !(s->lat_kind == MQV_LATTICE_HYPERCUBIC && potts_octets(s->md, s->sten)))
             b->L.potts_octets = 0;
     }
     const int64_t per_part = std::max<int64_t>(b->L.potts_octets ? 4096 : 1024, msites / (148 * 12));
     std::vector<int32_t> mprefix((size_t)n + 1, 0), mrep;
     for (int r = 0; r < n; ++r) {
         const int64_t parts =
-            b->resident[(size_t)r] ? 0 : std::max<int64_t>(1, (b->sims[(size_t)r]->n + per_part - 1) / per_part);
+            !on_graph(r) ? 0 : std::max<int64_t>(1, (b->sims[(size_t)r]->n + per_part - 1) / per_part);
         if (mprefix[(size_t)r] + parts >= (int64_t)1 << 31) return bail(fail(MQV_ERR_INVALID_ARG, "batch too large"));
         mprefix[(size_t)r + 1] = mprefix[(size_t)r] + (int32_t)parts;
         for (int64_t k = 0; k < parts; ++k) mrep.push_back(r);
