@@ -328,6 +328,7 @@ struct Sim {
     int64_t* d_sprefix1 = nullptr;
     int32_t* d_sbrep1 = nullptr;
     std::vector<unsigned char> rep1_host;  // what d_rep1 holds
+    bool rep1_captured = false;            // a captured graph writes d_rep1 too
     // labelling in bit tiles (wolff_tile.cuh): its tables, scratch, units per tile
     int32_t* d_ttab1 = nullptr;
     void* d_tile = nullptr;

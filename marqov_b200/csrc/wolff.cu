@@ -125,11 +125,18 @@ static BatchRep single_rep(const Sim* s)
     return r;
 }
 
-// The one-member table holds `r` (written only when something changed).
+// The one-member table holds `r` (written only when something changed).  Under
+// stream capture the write belongs to the graph: it is not done now, and every
+// replay does it again, so from then on the table is written each time.
 static void set_single_rep(Sim* s, const BatchRep& r)
 {
-    if (s->rep1_host.size() == sizeof r && std::memcmp(s->rep1_host.data(), &r, sizeof r) == 0) return;
-    s->rep1_host.assign((const unsigned char*)&r, (const unsigned char*)&r + sizeof r);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess) cudaGetLastError();
+    if (cap != cudaStreamCaptureStatusNone) s->rep1_captured = true;
+    if (!s->rep1_captured) {
+        if (s->rep1_host.size() == sizeof r && std::memcmp(s->rep1_host.data(), &r, sizeof r) == 0) return;
+        s->rep1_host.assign((const unsigned char*)&r, (const unsigned char*)&r + sizeof r);
+    }
     single_rep_set<<<1, 1, 0, s->stream>>>(s->d_rep1, r, s->d_ctr1);
     s->launches++;
 }
