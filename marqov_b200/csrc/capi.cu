@@ -473,9 +473,9 @@ static mqv_status launch_sweeps(Sim* s, int count, int slot)
 constexpr int64_t kLabelMinSites = (int64_t)1 << 18, kLabelMinTiled = 32768;
 static bool cluster_by_label(const Sim* s)
 {
+    if (s->wolff_algo == MQV_WOLFF_BFS || s->no_label) return false;
     if (s->wolff_algo == MQV_WOLFF_LABEL) return true;
-    if (s->wolff_algo == MQV_WOLFF_BFS) return false;
-    if (s->is_f32) return s->last_cluster > 200.0 + (double)s->n / 800.0 && !s->no_label && label_in_tiles(s);
+    if (s->is_f32) return s->last_cluster > 200.0 + (double)s->n / 800.0 && label_in_tiles(s);
     return s->n >= (label_in_tiles(s) ? kLabelMinTiled : kLabelMinSites);
 }
 
@@ -490,11 +490,16 @@ static void note_clusters(Sim* s, const int32_t* sizes, size_t count)
 static mqv_status launch_cluster(Sim* s, int slot)
 {
     bool label = cluster_by_label(s);
-    if (label && s->is_f32 && s->wolff_algo == MQV_WOLFF_AUTO && ensure_label_tables(s, true) != cudaSuccess) {
-        // no memory for the labelling's tables: breadth first needs none of them
-        cudaGetLastError();
-        s->no_label = true;
-        label = false;
+    if (label && label_in_tiles(s)) {
+        const cudaError_t e = ensure_label_tables(s, true);
+        if (e == cudaErrorMemoryAllocation) {
+            // no memory for the tiles: breadth first takes two thirds of it (floats less)
+            cudaGetLastError();
+            s->no_label = true;
+            label = false;
+        } else {
+            MQV_CK(e);
+        }
     }
     if (!label || !label_in_tiles(s)) {
         const mqv_status st = ensure_wolff(s);
@@ -1173,6 +1178,7 @@ MQV_API mqv_status mqv_set_wolff(mqv_sim* h, int32_t algorithm)
     if (!s) return fail(MQV_ERR_INVALID_ARG, "null handle");
     if (algorithm < MQV_WOLFF_AUTO || algorithm > MQV_WOLFF_LABEL) return fail(MQV_ERR_INVALID_ARG, "unknown algorithm");
     s->wolff_algo = algorithm;
+    s->no_label = false;
     return MQV_OK;
 }
 
@@ -1277,6 +1283,7 @@ struct Batch {
     size_t tile_bytes = 0;
     std::vector<size_t> tile_off;
     int wolff_mode = MQV_WOLFF_AUTO;
+    bool no_label = false;  // the tiles did not fit the device
     // MQV_WOLFF_AUTO: ms per EMCS of breadth first [0] and labelling [1] when
     // last timed (-1: never), the one in use, EMCS since the other was tried
     double wolff_est[2] = {-1.0, -1.0};
@@ -1431,8 +1438,16 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
             const mqv_status st = ensure_wolff(b->sims[(size_t)i]);
             if (st) return st;
         }
-    if (ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile)  // graph members
-        MQV_CK(cudaMalloc(&b->d_tile, b->tile_bytes));
+    if (ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile && !b->no_label) {  // graph members
+        const cudaError_t e = cudaMalloc(&b->d_tile, b->tile_bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            b->no_label = true;  // no memory for the tiles: breadth first needs none of them
+        } else {
+            MQV_CK(e);
+        }
+    }
+    const int wolff_mode = b->no_label ? MQV_WOLFF_BFS : b->wolff_mode;
     // member table at the start of the run
     b->reps.assign((size_t)b->nrep, BatchRep{});
     for (int i = 0; i < b->nrep; ++i) {
@@ -1482,8 +1497,8 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     // them the cost of growing them, change within a few dozen EMCS.
     bool graph = false;  // members on the graph path
     for (char p : path) graph |= p == 0;
-    const bool adapt = b->wolff_mode == MQV_WOLFF_AUTO && ncluster > 0 && graph;
-    const int fixed = b->wolff_mode == MQV_WOLFF_LABEL ? 1 : 0;
+    const bool adapt = wolff_mode == MQV_WOLFF_AUTO && ncluster > 0 && graph;
+    const int fixed = wolff_mode == MQV_WOLFF_LABEL ? 1 : 0;
     const int max_chunk = adapt ? 64 : CH;
     if (b->g_ncluster != ncluster || b->g_nmetro != nmetro || b->g_steps != K) {
         free_graphs(b);
@@ -2043,6 +2058,7 @@ MQV_API mqv_status mqv_batch_set_wolff(mqv_batch* h, int32_t algorithm)
     if (algorithm != MQV_WOLFF_AUTO && algorithm != MQV_WOLFF_BFS && algorithm != MQV_WOLFF_LABEL)
         return fail(MQV_ERR_INVALID_ARG, "unknown cluster algorithm");
     b->wolff_mode = algorithm;
+    b->no_label = false;
     if (algorithm == MQV_WOLFF_AUTO) {
         b->wolff_est[0] = b->wolff_est[1] = -1.0;
         b->wolff_best = 0;
@@ -2056,7 +2072,8 @@ MQV_API mqv_status mqv_batch_get_wolff(mqv_batch* h, int32_t* algorithm)
     Batch* b = reinterpret_cast<Batch*>(h);
     if (!b || !algorithm) return fail(MQV_ERR_INVALID_ARG, "null argument");
     const bool timed = b->wolff_est[0] > 0 && b->wolff_est[1] > 0;
-    *algorithm = b->wolff_mode != MQV_WOLFF_AUTO ? b->wolff_mode
+    *algorithm = b->no_label ? MQV_WOLFF_BFS
+                 : b->wolff_mode != MQV_WOLFF_AUTO ? b->wolff_mode
                  : !timed                       ? MQV_WOLFF_AUTO
                  : b->wolff_best == 1           ? MQV_WOLFF_LABEL
                                                 : MQV_WOLFF_BFS;
