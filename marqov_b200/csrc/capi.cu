@@ -190,7 +190,8 @@ static mqv_status check_runnable(const Sim* s)
 }
 
 // Graphs swept by one cluster (csr_sweep.cu) up to here: above, the launches,
-// which spread a colour over every SM, win (400,000 sites: 112 against 123 us).
+// which spread a colour over every SM, win (262,144 sites: 101 against 85 us a
+// sweep; 400,000 sites, before the limit was set: 112 against 123).
 constexpr int64_t kEllMaxSites = 262144;
 
 // ---- lattice lowering -----------------------------------------------------------

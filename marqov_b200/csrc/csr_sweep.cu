@@ -40,8 +40,8 @@
 // range of sites that it owns.  Same words, decisions and order of colours as
 // metro_int8_csr, same sums as measure_int8.  Bound by the latency of a
 // colour (gather, decision, words on their way).  Per sweep, launches and
-// this kernel (us): 1000 sites 50 and 9, 16,384 sites 74 and 12, 131,072 sites
-// 93 and 47, 400,000 sites 112 and 123.
+// this kernel (us): 1000 sites 45 and 9.4, 16,384 sites 72 and 12.2, 131,072 sites
+// 92 and 47, 262,144 sites 101 and 85.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -73,18 +73,6 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank)
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
-}
-
-// mbar_try_wait for words that came from other CTAs of the cluster
-__device__ __forceinline__ bool words_arrived(uint32_t bar, uint32_t parity)
-{
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return done != 0;
 }
 
 // shared memory: the sweep's rounds, the graph's spins (a bit per position,
@@ -166,13 +154,17 @@ __global__ void __launch_bounds__(kEllThreads, 1) ell_emcs(EllRun R)
         if (sends && !stop) st_async(to + 4u * (uint32_t)word, v, to_bar + 8u * (uint32_t)((step - 1) & 1));
     };
     // until every word of the last step begun has arrived, behind a CTA barrier
-    // (bounded: a lost word sets the error status and ends the run)
+    // (bounded: a lost word sets the error status and ends the run).  The wait
+    // acquires at CTA scope: what it guards lies in this CTA's shared memory, where
+    // a word lands before it is counted.  At cluster scope it drops the L1, and
+    // with it the neighbour lists, at every colour (16,384 sites 12.2 -> 15.6 us a
+    // sweep).
     auto receive = [&]() {
         if (stop) return;
         const uint32_t bar = smem_addr(&bars[(step - 1) & 1]), par = (uint32_t)((step - 1) >> 1) & 1u;
-        if (words_arrived(bar, par)) return;
+        if (mbar_try_wait(bar, par)) return;
         const uint64_t t0 = global_timer_ns();
-        for (uint32_t k = 1; !words_arrived(bar, par); ++k)
+        for (uint32_t k = 1; !mbar_try_wait(bar, par); ++k)
             if ((k & 255u) == 0 && global_timer_ns() - t0 > R.wait_ns) {
                 stop = true;
                 atomicExch(R.status, MQV_ERR_TIMEOUT);
