@@ -1,6 +1,8 @@
 """Clusters on a device whose free memory holds the breadth-first queues but not
 the scratch of labelling in bit tiles: the calls run, on the same clusters."""
 import contextlib
+import ctypes as C
+import gc
 
 import numpy as np
 import pytest
@@ -22,34 +24,51 @@ def kernels_loaded():
 
 @contextlib.contextmanager
 def free_memory(nbytes):
+    """All device memory but `nbytes` taken, down to the allocator's 2 MB."""
     import torch
+    gc.collect()  # handles of other tests that still wait for it
     torch.cuda.empty_cache()
-    free, _ = torch.cuda.mem_get_info()
-    hog = torch.empty(free - nbytes, dtype=torch.uint8, device="cuda")
+    rt = C.CDLL("libcudart.so.12")  # torch's, already loaded
+    taken = []
+
+    def take(size):
+        p = C.c_void_p()
+        if rt.cudaMalloc(C.byref(p), C.c_size_t(size)):
+            rt.cudaGetLastError()
+            return False
+        taken.append(p)
+        return True
+
+    assert take(nbytes)
+    size = torch.cuda.mem_get_info()[0]
+    while size >= 2 << 20:
+        if not take(size):
+            size //= 2
+    rt.cudaFree(taken.pop(0))
     try:
         yield
     finally:
-        del hog
-        torch.cuda.empty_cache()
+        for p in taken:
+            rt.cudaFree(p)
 
 
-def members(n):
+def members(n, L):
     import marqov_b200 as M
-    return [(M.RegularHypercubic(2048, 2), M.Config(seed=5, repid=i), M.Ising(-1.0), 0.2) for i in range(n)]
+    return [(M.RegularHypercubic(L, 2), M.Config(seed=5, repid=i), M.Ising(-1.0), 0.2) for i in range(n)]
 
 
 @pytest.mark.parametrize("algo", ["auto", "label"])
 def test_handle(algo):
     import marqov_b200 as M
-    (lat, cfg, ham, beta), = members(1)
+    (lat, cfg, ham, beta), = members(1, 4096)
     got = []
     for limit in (True, False):
         with M.makeCore(lat, cfg, ham, beta) as c:
             c.set_wolff(algo)
             c.init()
             c.emcs(1, 0, 1)
-            # queue and bitmap 17.3 MB, tiles 26.7 MB
-            with free_memory(23 << 20) if limit else contextlib.nullcontext():
+            # queue and bitmap 66 MiB, tiles 102 MiB
+            with free_memory(80 << 20) if limit else contextlib.nullcontext():
                 got.append([c.wolff(4), *c.emcs(2, 2, 1), c.state])
                 assert ("clusters=bfs" in c.describe()) == limit
             if limit:
@@ -65,12 +84,12 @@ def test_batch(algo):
     import marqov_b200 as M
     got = []
     for limit in (True, False):
-        with M.Batch(members(4)) as b:
+        with M.Batch(members(4, 2048)) as b:
             b.set_wolff(algo)
             b.init()
             b.emcs(2, 0, 1)
-            # queues and bitmaps 69 MB, tiles 107 MB
-            with free_memory(96 << 20) if limit else contextlib.nullcontext():
+            # queues and bitmaps 66 MiB, tiles 102 MiB
+            with free_memory(84 << 20) if limit else contextlib.nullcontext():
                 got.append([*b.emcs(6, 2, 1)] + [b.member(i).state for i in range(4)])
                 if limit:
                     assert b.wolff == "bfs"
