@@ -550,7 +550,11 @@ constexpr int64_t kBitsAutoSites = 32768;
 // x 24 53 and 60; 3D L = 32 (1024) x 1 62 and 41, x 16 65 and 59, x 20 65 and 66;
 // 2D L = 174 (1044) x 20 66 and 60, x 28 66 and 71.  Spin glasses, a sweep: 3D L =
 // 34 (2312) x 1 13.7 and 13.8; L = 40 (3200) x 1 17.6 and 13.7, x 4 17.6 and 15.0,
-// x 6 17.7 and 17.2, x 8 17.7 and 19.3.
+// x 6 17.7 and 17.2, x 8 17.7 and 19.3.  The launches have to be captured and
+// their cluster algorithm to be chosen (9 members of L = 160: 2.4 ms more up to the
+// end of the first call, then 61 us per EMCS against 85 with an exchange each), so
+// a batch takes the bit planes until it goes beyond kFewAfter EMCS.
+constexpr int64_t kFewAfter = 256;
 constexpr int64_t kBitsFewWords = 560, kBitsWordsPer = 46, kGlassFewWords = 2500, kGlassWords = 18000;
 static int64_t bit_words(const Sim* s) { return s->n / s->len * ((s->len + 31) / 32); }
 
@@ -1253,11 +1257,13 @@ struct Batch {
     int32_t* d_block_rep = nullptr;
     int32_t* d_cbegin = nullptr;
     int32_t* d_ccount = nullptr;
-    // Where every member runs, [0] in runs without clusters, [1] with: 0 the graph
-    // path, 1 batch_resident (one CTA each, state in shared memory), 2 a
-    // thread-block cluster, 3 as bit planes (batch_bits).  The tables of the graph
-    // path hold every member that runs there in either.
-    std::vector<char> path[2];
+    // Where every member runs, [1] in runs with clusters, [0] without, [2 +] those of
+    // the first kFewAfter EMCS: 0 the graph path, 1 batch_resident (one CTA each,
+    // state in shared memory), 2 a thread-block cluster, 3 as bit planes
+    // (batch_bits).  The tables of the graph path hold every member that runs
+    // there in any.
+    std::vector<char> path[4];
+    int64_t emcs_done = 0;
     // batch_resident's members in two classes by size (<= kResSmall sites: several
     // CTAs per SM), and the bit planes' members, each at a place of d_res_order,
     // largest first, with the dynamic shared memory of its largest layout
@@ -1265,7 +1271,7 @@ struct Batch {
         int count = 0, off = 0;
         size_t smem = 0;
     };
-    Group res[2][2], bits[2];  // [with clusters]
+    Group res[4][2], bits[4];  // as path
     int32_t* d_res_order = nullptr;
     // members held by thread-block clusters of c CTAs (c = 2 .. 8): ncl[c]
     // of them at d_res_order + cl_off[c]
@@ -1420,8 +1426,9 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
                             double* d_samples, const TemperRun* pt = nullptr)
 {
     DeviceGuard guard_(b->device);
-    const std::vector<char>& path = b->path[ncluster > 0];
-    const Batch::Group *res = b->res[ncluster > 0], &bits = b->bits[ncluster > 0];
+    const int kind = (ncluster > 0 ? 1 : 0) + (b->emcs_done + n_emcs <= kFewAfter ? 2 : 0);
+    const std::vector<char>& path = b->path[kind];
+    const Batch::Group *res = b->res[kind], &bits = b->bits[kind];
     if (n_emcs < 0 || ncluster < 0 || nmetro < 0) return fail(MQV_ERR_INVALID_ARG, "negative count");
     if (ncluster > 64 || nmetro > 64) return fail(MQV_ERR_INVALID_ARG, "at most 64 clusters and 64 sweeps per EMCS");
     for (Sim* s : b->sims) {
@@ -1699,6 +1706,7 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         s->sweep += (uint64_t)n_emcs * (uint64_t)nmetro;
         s->cluster += (uint64_t)n_emcs * (uint64_t)ncluster;
     }
+    b->emcs_done += n_emcs;
     return MQV_OK;
 }
 
@@ -1793,11 +1801,12 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     // (kBitsFewWords)
     auto flags = [&](int r) { return specs[r].params.flags; };
     auto glass = [&](int r) { return b->sims[(size_t)r]->md.kind == MQV_MODEL_EA; };
-    for (int c = 0; c < 2; ++c) {
-        b->path[c].assign((size_t)n, 0);
+    for (int k = 0; k < 4; ++k) {
+        const int c = k & 1;
+        b->path[k].assign((size_t)n, 0);
         int64_t words[2] = {0, 0}, largest = 0;  // few large members: of clusters, of spin glasses
         auto few = [&](int r) {
-            return !(flags(r) & MQV_FLAG_RESIDENT) &&
+            return k < 2 && !(flags(r) & MQV_FLAG_RESIDENT) &&
                    (glass(r) ? bit_words(b->sims[(size_t)r]) > kGlassFewWords
                              : c == 1 && bit_words(b->sims[(size_t)r]) > kBitsFewWords);
         };
@@ -1806,14 +1815,14 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
             if ((flags(r) & MQV_FLAG_NO_RESIDENT) || s->n > (glass(r) ? kResidentMaxSites : kBitsAutoSites) ||
                 !bits_fits(s, c == 1 && !glass(r)))
                 continue;
-            b->path[c][(size_t)r] = 3;
+            b->path[k][(size_t)r] = 3;
             if (!few(r)) continue;
             words[glass(r)] += bit_words(s);
             if (!glass(r)) largest = std::max(largest, bit_words(s));
         }
         const bool launches[2] = {words[0] <= kBitsWordsPer * (largest - kBitsFewWords), words[1] <= kGlassWords};
         for (int r = 0; r < n; ++r)
-            if (b->path[c][(size_t)r] == 3 && few(r) && launches[glass(r)]) b->path[c][(size_t)r] = 0;
+            if (b->path[k][(size_t)r] == 3 && few(r) && launches[glass(r)]) b->path[k][(size_t)r] = 0;
     }
     // Other resident members: int8 stencil lattices that fit one CTA's shared
     // memory or a thread-block cluster's.  Such a member runs on one CTA (or one
@@ -1821,26 +1830,28 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
     // a few): the graph path, whose launches spread every member over all SMs, is
     // the default (the 256-replica Potts farm: 1.8 against 3.4 ms per EMCS); members
     // that ask for it (MQV_FLAG_RESIDENT) stay resident.
-    std::vector<int32_t> res_order[2][2], bits_order[2], cl_order[9];
+    std::vector<int32_t> res_order[4][2], bits_order[4], cl_order[9];
     bool cl_ok[9] = {}, cl_asked = false;
     for (int r = 0; r < n; ++r) {
         const Sim* s = b->sims[(size_t)r];
         const bool asked = flags(r) & MQV_FLAG_RESIDENT;
-        for (int c = 0; c < 2; ++c) {
-            char& p = b->path[c][(size_t)r];
-            if (p == 3) bits_order[c].push_back(r);
+        bool graph = true;
+        for (int k = 0; k < 4; ++k) {
+            char& p = b->path[k][(size_t)r];
+            if (p == 3) bits_order[k].push_back(r);
             else if (asked && resident_fits(s)) {
                 p = 1;
-                res_order[c][s->n > kResSmall ? 1 : 0].push_back(r);
+                res_order[k][s->n > kResSmall ? 1 : 0].push_back(r);
             }
+            graph = graph && p == 0;
         }
-        if (asked && !s->is_f32 && s->lat_kind == MQV_LATTICE_HYPERCUBIC && !b->path[0][(size_t)r] && !b->path[1][(size_t)r]) {
+        if (asked && !s->is_f32 && s->lat_kind == MQV_LATTICE_HYPERCUBIC && graph) {
             const int c = cluster_ctas(s->n);
             if (!cl_asked)
                 for (int k = 2; k <= 8; ++k) cl_ok[k] = cluster_launchable(k);
             cl_asked = true;
             if (c >= 2 && cl_ok[c]) {
-                b->path[0][(size_t)r] = b->path[1][(size_t)r] = 2;
+                for (auto& p : b->path) p[(size_t)r] = 2;
                 cl_order[c].push_back(r);
             }
         }
@@ -1854,18 +1865,22 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         for (int32_t r : order) g.smem = std::max(g.smem, smem(b->sims[(size_t)r]));
         res_all.insert(res_all.end(), order.begin(), order.end());
     };
-    for (int c = 0; c < 2; ++c) {
-        for (int k = 0; k < 2; ++k)
-            place(res_order[c][k], b->res[c][k], [](const Sim* s) { return resident_smem_for(s->sten); });
-        place(bits_order[c], b->bits[c],
-              [c](const Sim* s) { return bits_smem(s, c == 1 && s->md.kind != MQV_MODEL_EA); });
+    for (int k = 0; k < 4; ++k) {
+        for (int cls = 0; cls < 2; ++cls)
+            place(res_order[k][cls], b->res[k][cls], [](const Sim* s) { return resident_smem_for(s->sten); });
+        place(bits_order[k], b->bits[k],
+              [k](const Sim* s) { return bits_smem(s, (k & 1) && s->md.kind != MQV_MODEL_EA); });
     }
     for (int c = 2; c <= 8; ++c) {
         b->cl_off[c] = (int)res_all.size();
         b->ncl[c] = (int)cl_order[c].size();
         res_all.insert(res_all.end(), cl_order[c].begin(), cl_order[c].end());
     }
-    auto on_graph = [&](int r) { return !b->path[0][(size_t)r] || !b->path[1][(size_t)r]; };
+    auto on_graph = [&](int r) {
+        for (const auto& p : b->path)
+            if (!p[(size_t)r]) return true;
+        return false;
+    };
     // per-colour work: colour c concatenates every graph member's colour-c
     // sites (resident members contribute none), each member's count padded
     // to whole blocks of kAccSites, so that a CTA's block lies in one member

@@ -1,6 +1,6 @@
 """Where a batch's Ising-type members run: as bit planes, one CTA each, or by
-launches where few large ones would leave the chip idle.  The same chain either
-way, also in batches that change between runs with and without clusters, in
+launches where few large ones would leave the chip idle and the batch has run a
+while (256 EMCS).  The same chain either way, also in batches that change between runs with and without clusters, in
 mixed batches and between exchanges; and single handles whose clusters are
 labelled by launches."""
 import numpy as np
@@ -32,7 +32,7 @@ def run(members, clusters):
     with M.Batch(members, graph_steps=3) as b:
         b.init()
         out, took = [], []
-        for nc, nm, n in ((0, 2, 5), (1, 1, 7), (0, 1, 4), (2, 1, 5)):
+        for nc, nm, n in ((0, 2, 5), (1, 1, 245), (0, 1, 4), (2, 1, 5), (0, 1, 3)):
             before = b.launches
             out += [*b.emcs(n, nc if clusters else 0, nm)]
             took.append((b.launches - before) / n)
@@ -50,10 +50,12 @@ def test_same_chain_on_either_path(make, clusters):
 
 
 @pytest.mark.parametrize("make,clusters,on_launches", [
-    (lambda **c: ising(2, (128, 128), **c), True, [False] * 4), (lambda **c: ising(2, (160, 160), **c), True, [False, True] * 2),
-    (lambda **c: ising(2, (160,) * 24, **c), True, [False] * 4), (lambda **c: ising(2, (178, 178), **c), True, [False, True] * 2),
-    (lambda **c: ising(2, (160, 160), resident=True, **c), True, [False] * 4),
-    (lambda **c: glasses(40, 3, **c), False, [True] * 4), (lambda **c: glasses(40, 12, **c), False, [False] * 4)])
+    (lambda **c: ising(2, (128, 128), **c), True, [False] * 5),
+    (lambda **c: ising(2, (160, 160), **c), True, [False, False, False, True, False]),
+    (lambda **c: ising(2, (160,) * 24, **c), True, [False] * 5),
+    (lambda **c: ising(2, (178, 178), **c), True, [False, True, False, True, False]),
+    (lambda **c: ising(2, (160, 160), resident=True, **c), True, [False] * 5),
+    (lambda **c: glasses(40, 3, **c), False, [False] * 3 + [True] * 2), (lambda **c: glasses(40, 12, **c), False, [False] * 5)])
 def test_path_taken(make, clusters, on_launches):
     _, took = run(make(), clusters)
     # bit planes: a launch or two per call; launches: several per EMCS
@@ -68,7 +70,7 @@ def test_exchanges():
                   for i, ((lat, _, h, _), b) in enumerate(zip(ising(2, (160,) * 6), np.linspace(0.43, 0.45, 6)))]
         with M.Batch(ladder) as b:
             b.init()
-            got.append([*b.tempering(6, 2, 1, 1, seed=3), *b.tempering(6, 1, 0, 2, seed=4), *b.tempering(4, 1, 1, 1, seed=5)]
+            got.append([*b.tempering(125, 2, 1, 1, seed=3), *b.tempering(6, 2, 1, 1, seed=8), *b.tempering(6, 1, 0, 2, seed=4), *b.tempering(4, 1, 1, 1, seed=5)]
                        + [b.member(i).state for i in range(6)])
     for x, y in zip(*got):
         assert np.array_equal(x, y)
