@@ -428,6 +428,9 @@ cudaError_t build_ell(Sim* s, int64_t n, const int32_t* rp, const int32_t* ci, c
         slice.push_back(total);
         total += 32 * (int64_t)*std::max_element(deg.begin() + (int64_t)p, deg.begin() + (int64_t)p + 32);
     }
+    // few large degrees among small ones of their colour: the slices would take
+    // many times the graph's memory, the launches take none
+    if (total > std::min<int64_t>(8 * (int64_t)rp[n] + (1 << 20), (int64_t)1 << 29)) return cudaSuccess;
     std::vector<int32_t> nb((size_t)std::max<int64_t>(total, 1), 0);
     std::vector<int8_t> bd(bonds ? nb.size() : 0, 0);
     for (size_t p = 0; p < np; ++p)

@@ -43,6 +43,22 @@ def test_missing_colours(name):
         assert np.array_equal(x, y)
 
 
+def test_slices_beyond_the_graphs_size():
+    import marqov_b200 as M
+    hubs, leaves = 32 * np.arange(1000), 32000 + np.arange(1100)  # a hub per slice of its colour
+    deg = np.zeros(33100, int)
+    deg[hubs], deg[leaves] = 1100, 1000
+    ci = np.r_[np.tile(leaves, 1000), np.tile(hubs, 1100)]
+    lat = M.CSRLattice(np.r_[0, np.cumsum(deg)], ci)
+    for x, y in zip(chain(lat, False), chain(lat, True)):
+        assert np.array_equal(x, y)
+    with M.makeCore(lat, M.Config(seed=8), M.Ising(-1.0, "int8"), 0.4) as c:
+        c.init()
+        before = c.launches
+        c.metropolis(5)
+        assert c.launches - before == 10  # a launch per colour
+
+
 @pytest.mark.parametrize("name", ["rgg", "gap"])
 @pytest.mark.parametrize("colour,nm,measure", [(2, 1, True), (2, 4, True), (7, 4, True), (3, 8, False)])
 def test_wait_that_runs_out(name, colour, nm, measure):
