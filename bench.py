@@ -816,17 +816,28 @@ def run_engine(args, ws, rank, local):
     core.close()
     peak, peak_kind = measured_peaks()
     per_launch_s = ms * 1e-3 / (args.steps * args.nmetro)
-    # one int8 read + one int8 write per site update; on bit planes once per
-    # run of nmetro sweeps (the planes stay in the L2: bound by the ALU pipe)
     kernel = kernel_desc.split("kernel=")[-1]
-    on_bits = kernel.startswith("ising2d_bits")
-    alg_bytes = 2 * n / args.nmetro if on_bits else 2 * n
-    achieved = alg_bytes / per_launch_s / 1e9
-    tr = profiled_traffic(kernel)
-    roof = {"bound": "alu" if on_bits else "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": None if tr is None else tr.get("bytes_per_launch"),
-            "kernel": kernel, "peak_source": f"{peak_kind} hbm_gbs",
-            "algorithmic_bytes_per_launch": alg_bytes}
+    tr = profiled_traffic(kernel) or {}
+    clocks = clk.summary()
+    if kernel.startswith("ising2d_bits"):
+        # bit planes stay in the L2 and are bound by the ALU pipe: its warp
+        # instructions of a sweep (ncu) against one per two cycles and scheduler;
+        # one int8 read + one int8 write per run of nmetro sweeps
+        alg_bytes = 2 * n / args.nmetro
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        peak = sms * 4 * 0.5 * clocks["sm_mhz"] * 1e-3 if clocks["sm_mhz"] else None
+        achieved = tr["alu_inst_per_sweep"] / per_launch_s / 1e9 if "alu_inst_per_sweep" in tr and L == 16384 else None
+        roof = {"bound": "alu", "achieved": achieved, "peak": peak, "unit": "G warp instructions/s",
+                "frac": achieved / peak if achieved and peak else None,
+                "peak_source": "SMs x 4 schedulers x 1/2 ALU instruction per cycle x median SM clock",
+                "hbm_frac": alg_bytes / per_launch_s / 1e9 / measured_peaks()[0]}
+    else:
+        # one int8 read + one int8 write per site update
+        alg_bytes = 2 * n
+        achieved = alg_bytes / per_launch_s / 1e9
+        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                "peak_source": f"{peak_kind} hbm_gbs"}
+    roof.update({"kernel": kernel, "traffic": tr.get("bytes_per_launch"), "algorithmic_bytes_per_launch": alg_bytes})
 
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
@@ -836,7 +847,7 @@ def run_engine(args, ws, rank, local):
                    "sweeps_per_step": args.nmetro, "parallelism": f"replicas ({ws} x 1 per GPU)",
                    "l2": "inputs larger than L2: the 268 MB int8 state is read and written every step"},
         "e2e": e2e, "e2e_host_state": e2e_host, "roofline": roof, "gpu_launches": launches,
-        "clocks": clk.summary(),
+        "clocks": clocks,
     }
     if rank == 0 and ws == 1 and not args.no_secondary:
         line["secondary"] = secondary(M, torch)

@@ -211,7 +211,10 @@ MQV_API mqv_status mqv_metropolis(mqv_sim* sim, int32_t nsweeps);
 enum { MQV_WOLFF_AUTO = 0, MQV_WOLFF_BFS = 1, MQV_WOLFF_LABEL = 2 };
 /* No counterpart in the reference.  The cluster algorithm of a handle:
  * MQV_WOLFF_AUTO (default) labels int8 lattices of at least 2^18 sites (2D and
- * 3D hypercubic ones from 2^15) and grows the others breadth first; lattices on the resident path
+ * 3D hypercubic ones from 2^15), and 2D and 3D float lattices once the clusters
+ * reported to the host exceed 200 + n / 800 sites, and grows the others breadth
+ * first.  Where the labelling's scratch does not fit the device, breadth first is
+ * taken instead, until this is called again.  Lattices on the resident path
  * (MQV_FLAG_NO_RESIDENT unset, int8 stencils of <= 262144 sites) label in
  * (distributed) shared memory. */
 MQV_API mqv_status mqv_set_wolff(mqv_sim* sim, int32_t algorithm);
@@ -298,7 +301,7 @@ MQV_API mqv_status mqv_batch_init_state(mqv_batch* batch);
  * whole-lattice passes (cost independent of cluster depth; pays for
  * percolating clusters on large lattices).  The default, MQV_WOLFF_AUTO,
  * times every chunk of EMCS (up
- * to 256 between host synchronisations), tries the algorithm not in use on a
+ * to 64 between host synchronisations), tries the algorithm not in use on a
  * few EMCS at the start of a chunk when it has no estimate or an old one, and
  * uses the faster estimate: the chain is the same whichever runs. */
 MQV_API mqv_status mqv_batch_set_wolff(mqv_batch* batch, int32_t algorithm);

@@ -240,7 +240,8 @@ class Core:
 
     def set_wolff(self, algorithm: str):
         """Cluster algorithm of this lattice: "auto" (labelling for int8 lattices
-        of >= 2^18 sites, 2D and 3D ones from 2^15), "bfs" or "label"; the
+        of >= 2^18 sites, 2D and 3D ones from 2^15, and for 2D and 3D float
+        lattices whose reported clusters have grown), "bfs" or "label"; the
         clusters are the same."""
         code = {"auto": L.WOLFF_AUTO, "bfs": L.WOLFF_BFS, "label": L.WOLFF_LABEL}[algorithm]
         L.check(self._lib.mqv_set_wolff(self._h, code))
