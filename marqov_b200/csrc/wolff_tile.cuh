@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(U * LPU, 1280 / (U * LPU))
     grid_dep_wait();
     const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
+    if (R.resident) return;  // on the graph path in other runs: grown by batch_bits in this one
     const uint32_t serial = cluster_serial(R, ctr, step);
     const TileAt<U> at(R, t);
     const int dim = R.st.dim, L = at.L;
@@ -409,6 +410,7 @@ __global__ void __launch_bounds__(U * LPU)
     grid_dep_wait();
     const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
+    if (R.resident) return;
     const uint32_t serial = cluster_serial(R, ctr, step);
     const TileAt<U> at(R, t);
     const int L = at.L, TY = at.TY, TZ = at.TZ;
@@ -492,6 +494,7 @@ __global__ void __launch_bounds__(U * LPU)
     grid_dep_wait();
     const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
+    if (R.resident) return;
     const CclSeed sd = seeds[r];
     const TileAt<U> at(R, t);
     const int L = at.L, base = t * (U * 32);

@@ -91,3 +91,18 @@ def test_handle_whose_clusters_are_labelled():
     for other in got[1:]:
         for x, y in zip(got[0], other):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("algo", ["bfs", "label"])
+def test_mixed_batch_by_either_algorithm(algo):
+    # the lattices of 160 and 174 run as bit planes here, beside launches that
+    # grow the clusters of the others and later theirs
+    import marqov_b200 as M
+    got = []
+    for resident in (None, False):
+        with M.Batch(mixed(resident=resident), graph_steps=2) as b:
+            b.set_wolff(algo)
+            b.init()
+            got.append([*b.emcs(7, 2, 1), *b.emcs(40, 3, 1), *b.emcs(250, 1, 1)] + [b.member(i).state for i in range(6)])
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)
