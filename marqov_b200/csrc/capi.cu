@@ -1286,6 +1286,8 @@ struct Batch {
     // tile_off[r] bytes), allocated by the first run with clusters
     int32_t* d_tile_prefix = nullptr;
     int32_t* d_tile_rep = nullptr;
+    std::vector<int32_t> tile_rep;  // the member of every tile
+    bool tiles_masked = false;      // d_tile_rep leaves members out
     void* d_tile = nullptr;
     size_t tile_bytes = 0;
     std::vector<size_t> tile_off;
@@ -1485,6 +1487,16 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     }
     MQV_CK(cudaMemcpyAsync(b->d_reps, b->reps.data(), sizeof(BatchRep) * b->reps.size(), cudaMemcpyHostToDevice,
                            b->stream));
+    // tiles of members that run elsewhere now and by launches later
+    bool mask = false;
+    for (int i = 0; i < b->nrep; ++i) mask |= path[(size_t)i] && !b->path[1][(size_t)i];
+    if (ncluster > 0 && mask != b->tiles_masked) {
+        std::vector<int32_t> rep(b->tile_rep);
+        for (int32_t& r : rep)
+            if (path[(size_t)r]) r = -1;
+        MQV_CK(upload_sync(b->stream, b->d_tile_rep, rep.data(), sizeof(int32_t) * rep.size()));
+        b->tiles_masked = mask;
+    }
     const int CH = 256;  // EMCS per chunk of measurements
     const int slots = std::min(CH, std::max(n_emcs, 1));
     const long long* acc0 = b->d_acc;
@@ -1926,7 +1938,8 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         if (!b->path[1][(size_t)r] && tile_shape(s->lat_kind, s->dim, s->len, 64).n) units += tile_lattice_units(s->dim, s->len);
     }
     b->L.tile = tile_config(units);
-    std::vector<int32_t> tprefix((size_t)n + 1, 0), trep;
+    std::vector<int32_t> tprefix((size_t)n + 1, 0);
+    std::vector<int32_t>& trep = b->tile_rep;
     std::vector<int64_t> sprefix((size_t)n + 1, 0);
     b->tile_off.assign((size_t)n, 0);
     for (int r = 0; r < n; ++r) {

@@ -198,9 +198,10 @@ __global__ void __launch_bounds__(U * LPU, 1280 / (U * LPU))
     const uint32_t part = (LPU == 1 ? 0xFFFFFFFFu : (1u << (BITS & 31)) - 1u) << (BITS * (tid % LPU));
     grid_dep_launch();
     grid_dep_wait();
-    const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
+    const int r = tile_rep[blockIdx.x];
+    if (r < 0) return;  // its member is held elsewhere in this run
+    const int t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
-    if (R.resident) return;  // on the graph path in other runs: grown by batch_bits in this one
     const uint32_t serial = cluster_serial(R, ctr, step);
     const TileAt<U> at(R, t);
     const int dim = R.st.dim, L = at.L;
@@ -408,9 +409,10 @@ __global__ void __launch_bounds__(U * LPU)
 {
     grid_dep_launch();
     grid_dep_wait();
-    const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
+    const int r = tile_rep[blockIdx.x];
+    if (r < 0) return;  // its member is held elsewhere in this run
+    const int t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
-    if (R.resident) return;
     const uint32_t serial = cluster_serial(R, ctr, step);
     const TileAt<U> at(R, t);
     const int L = at.L, TY = at.TY, TZ = at.TZ;
@@ -492,9 +494,10 @@ __global__ void __launch_bounds__(U * LPU)
     const uint32_t part = (LPU == 1 ? 0xFFFFFFFFu : (1u << (BITS & 31)) - 1u) << (BITS * (tid % LPU));
     grid_dep_launch();
     grid_dep_wait();
-    const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
+    const int r = tile_rep[blockIdx.x];
+    if (r < 0) return;  // its member is held elsewhere in this run
+    const int t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
-    if (R.resident) return;
     const CclSeed sd = seeds[r];
     const TileAt<U> at(R, t);
     const int L = at.L, base = t * (U * 32);
