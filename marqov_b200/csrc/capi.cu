@@ -1448,7 +1448,9 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
             const mqv_status st = ensure_wolff(b->sims[(size_t)i]);
             if (st) return st;
         }
-    if (ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile && !b->no_label) {  // graph members
+    bool graph = false;  // members on the graph path
+    for (char p : path) graph |= p == 0;
+    if (graph && ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile && !b->no_label) {
         const cudaError_t e = cudaMalloc(&b->d_tile, b->tile_bytes);
         if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
@@ -1515,8 +1517,6 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     // much slower it was), and the faster estimate is used after that.  Chunks
     // are short while the choice is by timing: a hot start's clusters, and with
     // them the cost of growing them, change within a few dozen EMCS.
-    bool graph = false;  // members on the graph path
-    for (char p : path) graph |= p == 0;
     const bool adapt = wolff_mode == MQV_WOLFF_AUTO && ncluster > 0 && graph;
     const int fixed = wolff_mode == MQV_WOLFF_LABEL ? 1 : 0;
     const int max_chunk = adapt ? 64 : CH;
