@@ -103,6 +103,7 @@ struct DeviceGuard {
         cudaError_t e_ = (expr);                                                             \
         if (e_ != cudaSuccess) {                                                             \
             set_error(std::string("CUDA error: ") + cudaGetErrorString(e_) + " at " #expr); \
+            cudaGetLastError(); /* not reported again by the next launch */                 \
             return e_ == cudaErrorMemoryAllocation ? MQV_ERR_OUT_OF_MEMORY : MQV_ERR_CUDA;   \
         }                                                                                    \
     } while (0)
@@ -155,8 +156,8 @@ static mqv_status ensure_cslots(Sim* s, int n)
 
 static mqv_status ensure_wolff(Sim* s)
 {
-    if (s->d_queue) return MQV_OK;
-    MQV_CK(cudaMalloc(&s->d_queue, sizeof(int32_t) * (size_t)s->n));
+    if (!s->d_queue) MQV_CK(cudaMalloc(&s->d_queue, sizeof(int32_t) * (size_t)s->n));
+    if (s->d_visited) return MQV_OK;  // else: never allocated, or it failed then
     const size_t words = (size_t)((s->n + 31) / 32);
     MQV_CK(cudaMalloc(&s->d_visited, sizeof(uint32_t) * words));
     MQV_CK(cudaMemsetAsync(s->d_visited, 0, sizeof(uint32_t) * words, s->stream));

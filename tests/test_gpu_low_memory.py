@@ -95,3 +95,24 @@ def test_batch(algo):
                     assert b.wolff == "bfs"
     for x, y in zip(*got):
         assert np.array_equal(x, y)
+
+
+def test_queue_without_bitmap():
+    """Room for the breadth-first queue and none for its bitmap: refused as often
+    as it is asked for, then run when there is room."""
+    import marqov_b200 as M
+    (lat, cfg, ham, beta), = members(1, 4096)
+    got = []
+    for limit in (True, False):
+        with M.makeCore(lat, cfg, ham, beta) as c:
+            c.set_wolff("bfs")
+            c.init()
+            c.emcs(1, 0, 1)
+            if limit:
+                with free_memory(64 << 20):
+                    for _ in range(2):
+                        with pytest.raises(M.MarqovError, match="memory"):
+                            c.wolff(1)
+            got.append([c.wolff(3), c.state])
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)
