@@ -554,7 +554,8 @@ constexpr int64_t kBitsAutoSites = 32768;
 // x 6 17.7 and 17.2, x 8 17.7 and 19.3.  The launches have to be captured and
 // their cluster algorithm to be chosen (9 members of L = 160: 2.4 ms more up to the
 // end of the first call, then 61 us per EMCS against 85 with an exchange each), so
-// a batch takes the bit planes until it goes beyond kFewAfter EMCS.
+// a batch takes the bit planes until it goes beyond kFewAfter EMCS (and
+// after that where clusters are to grow breadth first).
 constexpr int64_t kFewAfter = 256;
 constexpr int64_t kBitsFewWords = 560, kBitsWordsPer = 46, kGlassFewWords = 2500, kGlassWords = 18000;
 static int64_t bit_words(const Sim* s) { return s->n / s->len * ((s->len + 31) / 32); }
@@ -1294,6 +1295,7 @@ struct Batch {
     std::vector<size_t> tile_off;
     int wolff_mode = MQV_WOLFF_AUTO;
     bool no_label = false;  // the tiles did not fit the device
+    bool few_stay = false;  // the scratch of few large members' clusters did not: they stay on the bit planes
     // MQV_WOLFF_AUTO: ms per EMCS of breadth first [0] and labelling [1] when
     // last timed (-1: never), the one in use, EMCS since the other was tried
     double wolff_est[2] = {-1.0, -1.0};
@@ -1423,15 +1425,19 @@ struct TemperRun {
     int32_t* d_flags = nullptr;
 };
 
+// The scratch of tile labelling, allocated on first use.
+static mqv_status batch_tiles(Batch* b)
+{
+    if (b->tile_bytes && !b->d_tile) MQV_CK(cudaMalloc(&b->d_tile, b->tile_bytes));
+    return MQV_OK;
+}
+
 // n_emcs EMCS of every member; observables / cluster means to the host, raw
 // sums to the device samples buffer ([member][n_emcs][4]), each when given.
 static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_obs* obs, double* mean_cluster,
                             double* d_samples, const TemperRun* pt = nullptr)
 {
     DeviceGuard guard_(b->device);
-    const int kind = (ncluster > 0 ? 1 : 0) + (b->emcs_done + n_emcs <= kFewAfter ? 2 : 0);
-    const std::vector<char>& path = b->path[kind];
-    const Batch::Group *res = b->res[kind], &bits = b->bits[kind];
     if (n_emcs < 0 || ncluster < 0 || nmetro < 0) return fail(MQV_ERR_INVALID_ARG, "negative count");
     if (ncluster > 64 || nmetro > 64) return fail(MQV_ERR_INVALID_ARG, "at most 64 clusters and 64 sweeps per EMCS");
     for (Sim* s : b->sims) {
@@ -1443,6 +1449,24 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
             if (st) return st;
         }
     }
+    int kind = (ncluster > 0 ? 1 : 0) + (b->emcs_done + n_emcs <= kFewAfter ? 2 : 0);
+    if (kind == 1 && b->path[1] != b->path[3]) {
+        // Members that could stay on the bit planes do where their clusters are set
+        // to grow breadth first (us per EMCS, bit planes and launches: 2D L = 160 x 9
+        // 53 and 765, L = 174 x 20 67 and 982) or the launches' scratch does not fit
+        // the device.
+        mqv_status st = b->few_stay || b->no_label ? MQV_ERR_OUT_OF_MEMORY : MQV_OK;
+        if (b->wolff_mode != MQV_WOLFF_BFS) {
+            for (int i = 0; i < b->nrep && !st; ++i)
+                if (!b->path[1][(size_t)i] && b->path[3][(size_t)i]) st = ensure_wolff(b->sims[(size_t)i]);
+            if (!st) st = batch_tiles(b);
+            if (st && st != MQV_ERR_OUT_OF_MEMORY) return st;
+            b->few_stay = st != MQV_OK;
+        }
+        if (b->few_stay || b->wolff_mode == MQV_WOLFF_BFS) kind = 3;
+    }
+    const std::vector<char>& path = b->path[kind];
+    const Batch::Group *res = b->res[kind], &bits = b->bits[kind];
     if (ncluster > 0)
         for (int i = 0; i < b->nrep; ++i) {
             if (path[(size_t)i]) continue;
@@ -1451,14 +1475,10 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         }
     bool graph = false;  // members on the graph path
     for (char p : path) graph |= p == 0;
-    if (graph && ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && b->tile_bytes && !b->d_tile && !b->no_label) {
-        const cudaError_t e = cudaMalloc(&b->d_tile, b->tile_bytes);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            b->no_label = true;  // no memory for the tiles: breadth first needs none of them
-        } else {
-            MQV_CK(e);
-        }
+    if (graph && ncluster > 0 && b->wolff_mode != MQV_WOLFF_BFS && !b->no_label) {
+        const mqv_status st = batch_tiles(b);
+        if (st && st != MQV_ERR_OUT_OF_MEMORY) return st;
+        b->no_label = st != MQV_OK;  // no memory for the tiles: breadth first needs none of them
     }
     const int wolff_mode = b->no_label ? MQV_WOLFF_BFS : b->wolff_mode;
     // member table at the start of the run
@@ -2088,7 +2108,7 @@ MQV_API mqv_status mqv_batch_set_wolff(mqv_batch* h, int32_t algorithm)
     if (algorithm != MQV_WOLFF_AUTO && algorithm != MQV_WOLFF_BFS && algorithm != MQV_WOLFF_LABEL)
         return fail(MQV_ERR_INVALID_ARG, "unknown cluster algorithm");
     b->wolff_mode = algorithm;
-    b->no_label = false;
+    b->no_label = b->few_stay = false;
     if (algorithm == MQV_WOLFF_AUTO) {
         b->wolff_est[0] = b->wolff_est[1] = -1.0;
         b->wolff_best = 0;

@@ -116,3 +116,25 @@ def test_queue_without_bitmap():
             got.append([c.wolff(3), c.state])
     for x, y in zip(*got):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("algo", ["auto", "label", "bfs"])
+def test_few_large_members_stay_on_bit_planes(algo):
+    import marqov_b200 as M
+    got = []
+    for limit in (True, False):
+        with M.Batch(members(20, 174)) as b:
+            b.set_wolff(algo)
+            b.init()
+            b.emcs(250, 1, 1)
+            # queues and bitmaps 2.4 MiB, tiles 4 MiB
+            before = b.launches
+            with free_memory(1 << 20) if limit else contextlib.nullcontext():
+                out = [*b.emcs(10, 1, 1), *b.emcs(5, 2, 1)]
+            assert (b.launches - before < 15) == (limit or algo == "bfs")
+            b.set_wolff(algo)  # asked again, there is room
+            before = b.launches
+            got.append(out + [*b.emcs(4, 1, 0)] + [b.member(i).state for i in range(20)])
+            assert (b.launches - before < 4) == (algo == "bfs")
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)
