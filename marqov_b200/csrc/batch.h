@@ -111,7 +111,7 @@ struct BatchLaunch {
     const int32_t* meas_rep;     // [meas_blocks]
     int meas_blocks;
     // labelling in bit tiles: tiles of member r from tile_prefix[r], tile_rep[t]
-    // the member of tile t (negative: held elsewhere in this run)
+    // the member of tile t
     const int32_t* tile_prefix;  // [nrep + 1]
     const int32_t* tile_rep;     // [tiles]
     int tiles;

@@ -551,11 +551,14 @@ constexpr int64_t kBitsAutoSites = 32768;
 // x 24 53 and 60; 3D L = 32 (1024) x 1 62 and 41, x 16 65 and 59, x 20 65 and 66;
 // 2D L = 174 (1044) x 20 66 and 60, x 28 66 and 71.  Spin glasses, a sweep: 3D L =
 // 34 (2312) x 1 13.7 and 13.8; L = 40 (3200) x 1 17.6 and 13.7, x 4 17.6 and 15.0,
-// x 6 17.7 and 17.2, x 8 17.7 and 19.3.  The launches have to be captured and
-// their cluster algorithm to be chosen (9 members of L = 160: 2.4 ms more up to the
-// end of the first call, then 61 us per EMCS against 85 with an exchange each), so
-// a batch takes the bit planes until it goes beyond kFewAfter EMCS (and
-// after that where clusters are to grow breadth first).
+// x 6 17.7 and 17.2, x 8 17.7 and 19.3.  The launches have to be captured, and
+// their scratch allocated (0.5 to 2 ms in the first call), so a batch takes the bit
+// planes until it goes beyond kFewAfter EMCS.  From then on such clusters are
+// labelled, which holds at any temperature (us per EMCS, bit planes, labelled and
+// by breadth first or labelling timed: L = 160 x 12 at beta = 0.2 35, 36 and 26, at 0.5
+// 66, 47 and 47; 3D L = 28 x 6 at 0.4 182, 47 and 47), while timing lets breadth first
+// run for up to 64 EMCS (20 to 45 ms in the first call).  Members beside others that
+// always take the launches stay on the bit planes, which run beside these.
 constexpr int64_t kFewAfter = 256;
 constexpr int64_t kBitsFewWords = 560, kBitsWordsPer = 46, kGlassFewWords = 2500, kGlassWords = 18000;
 static int64_t bit_words(const Sim* s) { return s->n / s->len * ((s->len + 31) / 32); }
@@ -1288,14 +1291,13 @@ struct Batch {
     // tile_off[r] bytes), allocated by the first run with clusters
     int32_t* d_tile_prefix = nullptr;
     int32_t* d_tile_rep = nullptr;
-    std::vector<int32_t> tile_rep;  // the member of every tile
-    bool tiles_masked = false;      // d_tile_rep leaves members out
     void* d_tile = nullptr;
     size_t tile_bytes = 0;
     std::vector<size_t> tile_off;
     int wolff_mode = MQV_WOLFF_AUTO;
     bool no_label = false;  // the tiles did not fit the device
-    bool few_stay = false;  // the scratch of few large members' clusters did not: they stay on the bit planes
+    bool few = false;       // few large members, whose clusters go to the launches after a while
+    bool few_stay = false;  // the scratch of these did not fit: they stay on the bit planes
     // MQV_WOLFF_AUTO: ms per EMCS of breadth first [0] and labelling [1] when
     // last timed (-1: never), the one in use, EMCS since the other was tried
     double wolff_est[2] = {-1.0, -1.0};
@@ -1450,15 +1452,14 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         }
     }
     int kind = (ncluster > 0 ? 1 : 0) + (b->emcs_done + n_emcs <= kFewAfter ? 2 : 0);
-    if (kind == 1 && b->path[1] != b->path[3]) {
-        // Members that could stay on the bit planes do where their clusters are set
-        // to grow breadth first (us per EMCS, bit planes and launches: 2D L = 160 x 9
-        // 53 and 765, L = 174 x 20 67 and 982) or the launches' scratch does not fit
-        // the device.
-        mqv_status st = b->few_stay || b->no_label ? MQV_ERR_OUT_OF_MEMORY : MQV_OK;
+    if (kind == 1 && b->few) {
+        // They stay on the bit planes where their clusters are set to grow breadth
+        // first (us per EMCS, bit planes and launches: 2D L = 160 x 9 53 and 765,
+        // L = 174 x 20 67 and 982) or the launches' scratch does not fit the device.
+        mqv_status st = b->few_stay ? MQV_ERR_OUT_OF_MEMORY : MQV_OK;
         if (b->wolff_mode != MQV_WOLFF_BFS) {
             for (int i = 0; i < b->nrep && !st; ++i)
-                if (!b->path[1][(size_t)i] && b->path[3][(size_t)i]) st = ensure_wolff(b->sims[(size_t)i]);
+                if (!b->path[1][(size_t)i]) st = ensure_wolff(b->sims[(size_t)i]);
             if (!st) st = batch_tiles(b);
             if (st && st != MQV_ERR_OUT_OF_MEMORY) return st;
             b->few_stay = st != MQV_OK;
@@ -1480,7 +1481,8 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
         if (st && st != MQV_ERR_OUT_OF_MEMORY) return st;
         b->no_label = st != MQV_OK;  // no memory for the tiles: breadth first needs none of them
     }
-    const int wolff_mode = b->no_label ? MQV_WOLFF_BFS : b->wolff_mode;
+    // few large members are labelled: breadth first is hardly ever the faster one
+    const int wolff_mode = b->no_label ? MQV_WOLFF_BFS : kind == 1 && b->few ? MQV_WOLFF_LABEL : b->wolff_mode;
     // member table at the start of the run
     b->reps.assign((size_t)b->nrep, BatchRep{});
     for (int i = 0; i < b->nrep; ++i) {
@@ -1510,16 +1512,6 @@ static mqv_status batch_run(Batch* b, int n_emcs, int ncluster, int nmetro, mqv_
     }
     MQV_CK(cudaMemcpyAsync(b->d_reps, b->reps.data(), sizeof(BatchRep) * b->reps.size(), cudaMemcpyHostToDevice,
                            b->stream));
-    // tiles of members that run elsewhere now and by launches later
-    bool mask = false;
-    for (int i = 0; i < b->nrep; ++i) mask |= path[(size_t)i] && !b->path[1][(size_t)i];
-    if (ncluster > 0 && mask != b->tiles_masked) {
-        std::vector<int32_t> rep(b->tile_rep);
-        for (int32_t& r : rep)
-            if (path[(size_t)r]) r = -1;
-        MQV_CK(upload_sync(b->stream, b->d_tile_rep, rep.data(), sizeof(int32_t) * rep.size()));
-        b->tiles_masked = mask;
-    }
     const int CH = 256;  // EMCS per chunk of measurements
     const int slots = std::min(CH, std::max(n_emcs, 1));
     const long long* acc0 = b->d_acc;
@@ -1853,7 +1845,11 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
             words[glass(r)] += bit_words(s);
             if (!glass(r)) largest = std::max(largest, bit_words(s));
         }
-        const bool launches[2] = {words[0] <= kBitsWordsPer * (largest - kBitsFewWords), words[1] <= kGlassWords};
+        bool launches[2] = {words[0] > 0 && words[0] <= kBitsWordsPer * (largest - kBitsFewWords), words[1] <= kGlassWords};
+        for (int r = 0; r < n; ++r)  // beside members that always take the launches they stay
+            if (b->path[k][(size_t)r] != 3 && !((flags(r) & MQV_FLAG_RESIDENT) && resident_fits(b->sims[(size_t)r])))
+                launches[0] = false;
+        if (c == 1) b->few |= launches[0];
         for (int r = 0; r < n; ++r)
             if (b->path[k][(size_t)r] == 3 && few(r) && launches[glass(r)]) b->path[k][(size_t)r] = 0;
     }
@@ -1959,8 +1955,7 @@ MQV_API mqv_status mqv_batch_create(const mqv_sim_spec* specs, int32_t n, mqv_ba
         if (!b->path[1][(size_t)r] && tile_shape(s->lat_kind, s->dim, s->len, 64).n) units += tile_lattice_units(s->dim, s->len);
     }
     b->L.tile = tile_config(units);
-    std::vector<int32_t> tprefix((size_t)n + 1, 0);
-    std::vector<int32_t>& trep = b->tile_rep;
+    std::vector<int32_t> tprefix((size_t)n + 1, 0), trep;
     std::vector<int64_t> sprefix((size_t)n + 1, 0);
     b->tile_off.assign((size_t)n, 0);
     for (int r = 0; r < n; ++r) {

@@ -198,9 +198,7 @@ __global__ void __launch_bounds__(U * LPU, 1280 / (U * LPU))
     const uint32_t part = (LPU == 1 ? 0xFFFFFFFFu : (1u << (BITS & 31)) - 1u) << (BITS * (tid % LPU));
     grid_dep_launch();
     grid_dep_wait();
-    const int r = tile_rep[blockIdx.x];
-    if (r < 0) return;  // its member is held elsewhere in this run
-    const int t = (int)blockIdx.x - tile_prefix[r];
+    const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
     const uint32_t serial = cluster_serial(R, ctr, step);
     const TileAt<U> at(R, t);
@@ -409,9 +407,7 @@ __global__ void __launch_bounds__(U * LPU)
 {
     grid_dep_launch();
     grid_dep_wait();
-    const int r = tile_rep[blockIdx.x];
-    if (r < 0) return;  // its member is held elsewhere in this run
-    const int t = (int)blockIdx.x - tile_prefix[r];
+    const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
     const uint32_t serial = cluster_serial(R, ctr, step);
     const TileAt<U> at(R, t);
@@ -494,9 +490,7 @@ __global__ void __launch_bounds__(U * LPU)
     const uint32_t part = (LPU == 1 ? 0xFFFFFFFFu : (1u << (BITS & 31)) - 1u) << (BITS * (tid % LPU));
     grid_dep_launch();
     grid_dep_wait();
-    const int r = tile_rep[blockIdx.x];
-    if (r < 0) return;  // its member is held elsewhere in this run
-    const int t = (int)blockIdx.x - tile_prefix[r];
+    const int r = tile_rep[blockIdx.x], t = (int)blockIdx.x - tile_prefix[r];
     const BatchRep& R = reps[r];
     const CclSeed sd = seeds[r];
     const TileAt<U> at(R, t);

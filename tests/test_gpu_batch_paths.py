@@ -55,6 +55,7 @@ def test_same_chain_on_either_path(make, clusters):
     (lambda **c: ising(2, (160,) * 24, **c), True, [False] * 5),
     (lambda **c: ising(2, (178, 178), **c), True, [False, True, False, True, False]),
     (lambda **c: ising(2, (160, 160), resident=True, **c), True, [False] * 5),
+    (lambda **c: ising(2, (160, 160, 32), **c), True, [False, False, False, True, False]),
     (lambda **c: glasses(40, 3, **c), False, [False] * 3 + [True] * 2), (lambda **c: glasses(40, 12, **c), False, [False] * 5)])
 def test_path_taken(make, clusters, on_launches):
     _, took = run(make(), clusters)
@@ -95,8 +96,8 @@ def test_handle_whose_clusters_are_labelled():
 
 @pytest.mark.parametrize("algo", ["bfs", "label"])
 def test_mixed_batch_by_either_algorithm(algo):
-    # the lattices of 160 and 174 run as bit planes here, beside launches that
-    # grow the clusters of the others and later theirs
+    # the lattices of 160 and 174 stay on the bit planes, beside launches that
+    # grow the clusters of the others
     import marqov_b200 as M
     got = []
     for resident in (None, False):
