@@ -563,13 +563,27 @@ constexpr int64_t kFewAfter = 256;
 constexpr int64_t kBitsFewWords = 560, kBitsWordsPer = 46, kGlassFewWords = 2500, kGlassWords = 18000;
 static int64_t bit_words(const Sim* s) { return s->n / s->len * ((s->len + 31) / 32); }
 
+// The scratch of tile labelling is there or can be had: not under stream capture,
+// which allows no allocation, nor where it does not fit the device.
+static bool label_ready(Sim* s)
+{
+    if (s->d_tile) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s->stream, &cap);
+    if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) return false;
+    if (e == cudaSuccess) e = ensure_label_tables(s, true);
+    if (e == cudaSuccess) return true;
+    cudaGetLastError();
+    s->no_label = e == cudaErrorMemoryAllocation;
+    return false;
+}
 // EMCS of this handle run on the resident path (smem_emcs.cu, bits_emcs.cu)?
-static bool use_resident(const Sim* s, int ncluster)
+static bool use_resident(Sim* s, int ncluster)
 {
     if ((s->flags & MQV_FLAG_NO_RESIDENT) || s->n > kResidentMaxSites) return false;
     if (s->n <= kBitsAutoSites && bits_fits(s, ncluster > 0)) {
-        const bool labelled = ncluster > 0 && s->n >= kLabelMinTiled && cluster_by_label(s);
-        if (!labelled || (s->flags & MQV_FLAG_RESIDENT)) return true;
+        const bool may_label = ncluster > 0 && s->n >= kLabelMinTiled && !(s->flags & MQV_FLAG_RESIDENT);
+        if (!may_label || !cluster_by_label(s) || !label_ready(s)) return true;
     }
     return resident_fits(s) && ((s->flags & MQV_FLAG_RESIDENT) || s->n <= kResidentAutoSites);
 }

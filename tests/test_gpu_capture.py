@@ -50,3 +50,34 @@ def test_clusters_beside_a_captured_call(replays):
         del graph
         torch.cuda.synchronize()
         c.set_stream(0)
+
+
+def test_first_clusters_in_a_captured_call():
+    """3D L = 32 is labelled, with scratch that a captured call cannot allocate: it
+    stays on the bit planes there."""
+    import marqov_b200 as M
+    import torch
+    from marqov_b200 import _lib
+    lib = _lib.load()
+
+    def make(resident):
+        c = M.makeCore(M.RegularHypercubic(32, 3), M.Config(seed=4, resident=resident), M.Ising(-1.0), 0.2216546)
+        c.init()
+        c.emcs(2, 0, 1)
+        return c
+
+    with make(None) as c, make(True) as want:
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        c.set_stream(stream.cuda_stream)
+        with torch.cuda.graph(graph, stream=stream):
+            _lib.check(lib.mqv_wolff(c.handle, 1, None))
+        graph.replay()
+        torch.cuda.synchronize()
+        want.wolff(1)
+        assert np.array_equal(c.state, want.state)
+        assert np.array_equal(c.wolff(3), want.wolff(3))
+        assert np.array_equal(c.state, want.state)
+        assert "clusters=label " in c.describe()
+        del graph
+        torch.cuda.synchronize()
+        c.set_stream(0)

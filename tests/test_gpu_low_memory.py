@@ -138,3 +138,28 @@ def test_few_large_members_stay_on_bit_planes(algo):
             assert (b.launches - before < 4) == (algo == "bfs")
     for x, y in zip(*got):
         assert np.array_equal(x, y)
+
+
+def test_small_handle_stays_on_bit_planes():
+    import marqov_b200 as M
+    rt = C.CDLL("libcudart.so.12")
+    got = []
+    for limit in (True, False):
+        with M.makeCore(M.RegularHypercubic(32, 3), M.Config(seed=5), M.Ising(-1.0), 0.2216546) as c:
+            c.init()
+            c.emcs(2, 0, 1)
+            with free_memory(64 << 10) if limit else contextlib.nullcontext():
+                small, size = [], 1 << 20
+                while limit and size >= 64 << 10:  # what is left of the allocator's blocks; queue 131 KB, tiles 213
+                    p = C.c_void_p()
+                    if rt.cudaMalloc(C.byref(p), C.c_size_t(size)):
+                        rt.cudaGetLastError()
+                        size //= 2
+                    else:
+                        small.append(p)
+                got.append([c.wolff(3), *c.emcs(2, 1, 1), c.state])
+                for p in small:
+                    rt.cudaFree(p)
+            assert ("clusters=label-smem" in c.describe()) == limit
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)
