@@ -137,8 +137,8 @@ enum {
                                  sides of 176 to 180 do not, and as far as launches do not label
                                  them faster: 3D side 32); these
                                  are resident in a batch too (spin glasses up to 65536 sites), but
-                                 for few large members, and the batch's other members run on its
-                                 graph path */
+                                 where few large ones are all its members and it has run 256 EMCS,
+                                 and the batch's other members run on its graph path */
 };
 
 typedef struct mqv_run_params {
@@ -303,7 +303,9 @@ MQV_API mqv_status mqv_batch_init_state(mqv_batch* batch);
  * times every chunk of EMCS (up
  * to 64 between host synchronisations), tries the algorithm not in use on a
  * few EMCS at the start of a chunk when it has no estimate or an old one, and
- * uses the faster estimate: the chain is the same whichever runs. */
+ * uses the faster estimate: the chain is the same whichever runs.  Few large
+ * Ising members that left the bit planes are labelled without timing, and stay on
+ * the bit planes under MQV_WOLFF_BFS. */
 MQV_API mqv_status mqv_batch_set_wolff(mqv_batch* batch, int32_t algorithm);
 /* The algorithm in use: MQV_WOLFF_BFS or MQV_WOLFF_LABEL, or MQV_WOLFF_AUTO
  * while the automatic choice has not been timed yet. */

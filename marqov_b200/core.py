@@ -46,7 +46,8 @@ class Config:
     # None: the engine decides (single handles up to 16384 sites, Ising-type
     # lattices, which are held as bit planes, up to 32768 sites -- 2D sides of
     # 176 to 180 and the 3D side 32 only without clusters -- also in a
-    # batch, whose other members, and few large ones, take its graph path); True: wherever the lattice fits;
+    # batch, whose other members take its graph path, and these too where few
+    # large ones are all its members and it has run 256 EMCS); True: wherever the lattice fits;
     # False: never (launch per step).  The results are the same.
     resident: bool | None = None
 
